@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(64) beam_kernel(const __grid_constant__ BeamPa
     const double omega_img = sqrt(cimg[0] * cimg[0] + cimg[1] * cimg[1] + cimg[2] * cimg[2]);
     const double sgn_img = cimg[0] * d0[1] + cimg[1] * d0[2] + cimg[2] * d0[3] >= 0.0 ? 1.0 : -1.0;
 
-    const DPTable<double>& D = dp_table<double>();
+    const DPTable& D = kDPd;
     double h = c.h0;
     double K[7][24];
     beam_rhs(m, Y, K[0]);

@@ -39,7 +39,7 @@ __device__ __forceinline__ float rsqrt_(float x) { return rsqrtf(x); }
 // sequence with a special-case branch); FP64: sqrt.
 __device__ __forceinline__ float sqrtp_(float x) { return x * rsqrtf(x); }
 __device__ __forceinline__ double sqrtp_(double x) { return sqrt(x); }
-__device__ __forceinline__ double rsqrt_(double x) { return 1.0 / sqrt(x); }
+__device__ __forceinline__ double rsqrt_(double x) { return rsqrt(x); }
 __device__ __forceinline__ float exp_(float x) { return __expf(x); }
 __device__ __forceinline__ double exp_(double x) { return exp(x); }
 __device__ __forceinline__ float tanh_(float x) { return tanhf(x); }

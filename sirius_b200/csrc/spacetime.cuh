@@ -15,6 +15,8 @@
 // (PHMT100A.h:362-369) is folded in exactly by a Sherman-Morrison update.
 #pragma once
 
+#include <type_traits>
+
 #include "dual.cuh"
 #include "../../include/sirius_cuda.h"
 
@@ -135,7 +137,7 @@ SIRIUS_HD __forceinline__ void ks_rhs(const MetricDev& m, const T x[4], const T 
 //   d H  = ((2 M r^2 + 2 r (2 M r - Q^2) - H 4 r^3) dr - H (0, 0, 2 a^2 z)) / fden
 // with num = (2 M r - Q^2) r^2, fden = r^4 + a^2 z^2, H = num / fden.
 template <class T>
-SIRIUS_HD __forceinline__ void ks_rhs_fast(const MetricDev& m, const T x[4], const T p[4], T k[4], T f[4]) {
+SIRIUS_HD __forceinline__ void ks_rhs_terms(const MetricDev& m, const T x[4], const T p[4], T k[4], T f[4]) {
     const T a = cst<T>(m.a, m.fa), a2 = cst<T>(m.a2, m.fa2);
     const T X = x[1], Y = x[2], Z = x[3];
     const T zz = Z * Z;
@@ -193,6 +195,79 @@ SIRIUS_HD __forceinline__ void ks_rhs_fast(const MetricDev& m, const T x[4], con
         const T qq = cst<T>(m.lam3, m.flam3) * k[0] * k[0];
         f[1] -= qq * X; f[2] -= qq * Y; f[3] -= qq * Z;
     }
+}
+
+// The same right-hand side in closed form, the one the FP64 arithmetic runs. With
+// sd = sqrt((R^2 - a^2)^2 + 4 a^2 z^2) the implicit equation of r gives
+// r^4 + a^2 z^2 = r^2 sd, so H = (2 M r - Q^2) / sd, and with dr = (r x, r y,
+// z (r^2 + a^2) / r) / sd every gradient is a multiple of dr plus an explicit term.
+// The sum over l's components is formed before the gradient's, so that
+//   d_i l_j k^j = S dr_i + E_i,
+//     S = (k^x x + k^y y - 2 r (l_x k^x + l_y k^y)) / (r^2 + a^2) - k^z z / r^2,
+//     E = ((r k^x - a k^y) / (r^2 + a^2), (a k^x + r k^y) / (r^2 + a^2), k^z / r),
+//   d_i H = w dr_i - 2 H a^2 z / (r^2 sd) delta_iz,  w = (2 M + 2 (2 M r - Q^2) / r - 4 H r) / sd,
+//   dp_i = (l.k) ((w (l.k) / 2 + H S) dr_i + H E_i - H a^2 z (l.k) / (r^2 sd) delta_iz).
+// l is null for eta, so l.k = l#.p where k = g^{-1} p carries no Lambda term.
+// The FP64 kernels are bound by the issue and latency of their FP64 instructions,
+// and an FP64 root or reciprocal is a sequence of about ten: this form takes two
+// reciprocal square roots and one reciprocal where the terms take two square
+// roots and four reciprocals, and 94 operations instead of 143 (717 x 405 FP64
+// frame 8.73 -> 7.45 ms from this alone). The FP32 arithmetic keeps the terms: the two forms round
+// differently, and near the critical curve FP32 roundings reach the image.
+template <class T>
+SIRIUS_HD __forceinline__ void ks_rhs_closed(const MetricDev& m, const T x[4], const T p[4], T k[4], T f[4]) {
+    const T a = cst<T>(m.a, m.fa), a2 = cst<T>(m.a2, m.fa2), M2 = cst<T>(2.0 * m.M, m.fM2);
+    const T X = x[1], Y = x[2], Z = x[3];
+    const T zz = Z * Z;
+    const T R2 = X * X + Y * Y + zz;
+    const T Rm2 = R2 - a2;
+    const T disc = tmax(Rm2 * Rm2 + T(4) * a2 * zz, T(1e-20));
+    const T isd = rsqrt_(disc);
+    const T r2 = tmax((Rm2 + disc * isd) * T(0.5), T(1e-10));
+    const T ir = rsqrt_(r2);
+    const T r = r2 * ir;
+    const T den = r2 + a2;
+    const T iden = rcp_(den);
+    const T l1 = (r * X + a * Y) * iden, l2 = (r * Y - a * X) * iden, l3 = Z * ir;
+    const T q = M2 * r - cst<T>(m.Q2, m.fQ2);
+    const T H = q * isd;
+    // k = g^{-1} p = eta p - H l# (l# . p), l# = (-1, l1, l2, l3)
+    const T lp = -p[0] + l1 * p[1] + l2 * p[2] + l3 * p[3];
+    const T Hlp = H * lp;
+    k[0] = -p[0] + Hlp;
+    k[1] = p[1] - l1 * Hlp;
+    k[2] = p[2] - l2 * Hlp;
+    k[3] = p[3] - l3 * Hlp;
+    T lk = lp;
+    if (m.has_lambda) {
+        const T c = cst<T>(m.lam3, m.flam3) * R2;
+        const T w0 = -T(1) - H, w1 = H * l1, w2 = H * l2, w3 = H * l3;
+        const T s = c * (w0 * p[0] + w1 * p[1] + w2 * p[2] + w3 * p[3]) * rcp_(T(1) + c * (T(1) + H));
+        k[0] += s * w0; k[1] += s * w1; k[2] += s * w2; k[3] += s * w3;
+        lk = k[0] + l1 * k[1] + l2 * k[2] + l3 * k[3];
+    }
+    const T S = (X * k[1] + Y * k[2] - T(2) * r * (l1 * k[1] + l2 * k[2])) * iden - k[3] * l3 * ir;
+    const T w = (M2 + T(2) * q * ir - T(4) * H * r) * isd;
+    const T Hlk = H * lk, e = Hlk * iden;
+    const T g = lk * (T(0.5) * w * lk + H * S) * isd;
+    const T gr = g * r;
+    f[0] = T(0);
+    f[1] = gr * X + e * (r * k[1] - a * k[2]);
+    f[2] = gr * Y + e * (a * k[1] + r * k[2]);
+    f[3] = ir * (g * den * Z + Hlk * (k[3] - a2 * l3 * isd * lk));
+    // the Lambda term of dp: - Lambda x_i (k^0)^2 / 3
+    if (m.has_lambda) {
+        const T qq = cst<T>(m.lam3, m.flam3) * k[0] * k[0];
+        f[1] -= qq * X; f[2] -= qq * Y; f[3] -= qq * Z;
+    }
+}
+
+// The Kerr-Schild right-hand side of precision T: the closed form in FP64, the
+// terms otherwise (and for the operation count, which is the FP32 kernel's).
+template <class T>
+SIRIUS_HD __forceinline__ void ks_rhs_fast(const MetricDev& m, const T x[4], const T p[4], T k[4], T f[4]) {
+    if constexpr (std::is_same<T, double>::value) ks_rhs_closed(m, x, p, k, f);
+    else ks_rhs_terms(m, x, p, k, f);
 }
 
 // ---------------------------------------------------------------------------
@@ -314,26 +389,27 @@ __device__ __forceinline__ void inv_form(const MetricDev& m, const double x[4], 
         F.vf = m.vs * f.v;
         return;
     }
+    // (roots and reciprocals as in ks_rhs_closed: H = (2 M r - Q^2) / sd)
     const double a2 = m.a2, Rm2 = R2 - a2;
-    const double sd = sqrt(fmax(Rm2 * Rm2 + 4.0 * a2 * Z * Z, 1e-20));
-    const double r2 = fmax(0.5 * (Rm2 + sd), 1e-10);
-    const double r = sqrt(r2);
+    const double disc = fmax(Rm2 * Rm2 + 4.0 * a2 * Z * Z, 1e-20);
+    const double isd = rsqrt_(disc);
+    const double r2 = fmax(0.5 * (Rm2 + disc * isd), 1e-10);
+    const double ir = rsqrt_(r2), r = r2 * ir;
+    const double den = r2 + a2, iden = 1.0 / den;
     F.r = r;
-    if (m.a == 0.0) {
-        const double Rr = sqrt(R2);
-        F.d[1] = X / Rr; F.d[2] = Y / Rr; F.d[3] = Z / Rr;
-    } else {
-        F.d[1] = r * X / sd; F.d[2] = r * Y / sd; F.d[3] = Z * (r2 + a2) / (r * sd);
-    }
-    const double den = r2 + a2;
+    F.d[1] = r * X * isd; F.d[2] = r * Y * isd; F.d[3] = Z * den * ir * isd;
     F.l[0] = -1.0;  // l# = eta l
-    F.l[1] = (r * X + m.a * Y) / den;
-    F.l[2] = (r * Y - m.a * X) / den;
-    F.l[3] = Z / r;
-    F.H = (2.0 * m.M * r - m.Q2) * r2 / (r2 * r2 + a2 * Z * Z);
-    F.c = m.has_lambda ? m.lam3 * R2 : 0.0;
+    F.l[1] = (r * X + m.a * Y) * iden;
+    F.l[2] = (r * Y - m.a * X) * iden;
+    F.l[3] = Z * ir;
+    F.H = (2.0 * m.M * r - m.Q2) * isd;
     F.w[0] = -1.0 - F.H; F.w[1] = F.H * F.l[1]; F.w[2] = F.H * F.l[2]; F.w[3] = F.H * F.l[3];
-    F.sm = F.c / (1.0 + F.c * (1.0 + F.H));
+    F.c = 0.0;
+    F.sm = 0.0;
+    if (m.has_lambda) {
+        F.c = m.lam3 * R2;
+        F.sm = F.c / (1.0 + F.c * (1.0 + F.H));
+    }
 }
 
 __device__ __forceinline__ double inv_apply(const MetricDev& m, const InvForm& F, const double u[4], const double v[4]) {
@@ -375,42 +451,47 @@ __device__ __forceinline__ double project_null(const MetricDev& m, const InvForm
 // The same re-projection for the mixed-precision path, Kerr-Schild family
 // without Lambda. Only the null value C = g^{-1}(p, p) needs FP64: it is a
 // difference of O(p^2) terms that must survive to ~1e-16 of them, so r, H and
-// l are FP64 (their three reciprocals from one division). The direction dr and
-// the coefficients A = g^{-1}(dr, dr), B = 2 g^{-1}(p, dr) only set alpha =
+// l are FP64 (two reciprocal square roots and one reciprocal). The direction dr
+// and the coefficients A = g^{-1}(dr, dr), B = 2 g^{-1}(p, dr) only set alpha =
 // C / q, which needs single-precision relative accuracy; they are FP32, and
-// the constraint left after the update is ~1e-7 C. Returns C; r_out = r.
+// the constraint left after the update is ~1e-7 C. Returns C; r_out = r;
+// moved: the update is beyond what an f(x, p) stored in FP32 resolves (1e-6 of p).
 __device__ __forceinline__ double project_null_ks_mixed(const MetricDev& m, const double x[4], double p[4],
-                                                        double& r_out) {
+                                                        double& r_out, bool& moved) {
+    moved = false;
     const double X = x[1], Y = x[2], Z = x[3];
     const double a = m.a, a2 = m.a2;
     const double R2 = X * X + Y * Y + Z * Z, Rm2 = R2 - a2;
-    const double sd = sqrt(fmax(Rm2 * Rm2 + 4.0 * a2 * Z * Z, 1e-20));
-    const double r2 = fmax(0.5 * (Rm2 + sd), 1e-10);
-    const double r = sqrt(r2);
+    const double disc2 = fmax(Rm2 * Rm2 + 4.0 * a2 * Z * Z, 1e-20);
+    const double isd = rsqrt_(disc2);
+    const double r2 = fmax(0.5 * (Rm2 + disc2 * isd), 1e-10);
+    const double ir = rsqrt_(r2), r = r2 * ir;
     r_out = r;
-    const double den = r2 + a2, hden = r2 * r2 + a2 * Z * Z;
-    const double t = 1.0 / (den * r * hden);
-    const double iden = t * r * hden, ir = t * den * hden, ihden = t * den * r;
+    const double den = r2 + a2, iden = 1.0 / den;
     const double l1 = (r * X + a * Y) * iden, l2 = (r * Y - a * X) * iden, l3 = Z * ir;
-    const double H = (2.0 * m.M * r - m.Q2) * r2 * ihden;
+    const double H = (2.0 * m.M * r - m.Q2) * isd;
     const double lp = -p[0] + l1 * p[1] + l2 * p[2] + l3 * p[3];
     const double C = -p[0] * p[0] + p[1] * p[1] + p[2] * p[2] + p[3] * p[3] - H * lp * lp;
-    const float rf = float(r), isd = 1.f / float(sd);
-    const float d1 = rf * float(X) * isd, d2 = rf * float(Y) * isd, d3 = float(Z) * float(den) * isd / rf;
+    const float isdf = float(isd), rs = float(r) * isdf;
+    const float d1 = rs * float(X), d2 = rs * float(Y), d3 = float(Z) * float(den) * isdf * float(ir);
+    const float p1 = float(p[1]), p2 = float(p[2]), p3 = float(p[3]);
     const float Hf = float(H);
     const float ld = float(l1) * d1 + float(l2) * d2 + float(l3) * d3;
     const float A = d1 * d1 + d2 * d2 + d3 * d3 - Hf * ld * ld;
-    const float pd = float(p[1]) * d1 + float(p[2]) * d2 + float(p[3]) * d3;
+    const float pd = p1 * d1 + p2 * d2 + p3 * d3;
     const float B = 2.f * (pd - Hf * float(lp) * ld);
     const float Cf = float(C);
     const float disc = B * B - 4.f * A * Cf;
     if (!(disc >= 0.f) || fabsf(A) < 1e-15f) return C;
     const float q = -0.5f * (B + copysignf(sqrtf(disc), B));
     if (q == 0.f) return C;
-    const double alpha = double(Cf / q);
+    const float al = Cf * rcp_(q);
+    const double alpha = double(al);
     p[1] += alpha * double(d1);
     p[2] += alpha * double(d2);
     p[3] += alpha * double(d3);
+    const float pm = fmaxf(fmaxf(fabsf(float(p[0])), fabsf(p1)), fmaxf(fabsf(p2), fabsf(p3)));
+    moved = fabsf(al) * fmaxf(fmaxf(fabsf(d1), fabsf(d2)), fabsf(d3)) > 1e-6f * pm;
     return C;
 }
 

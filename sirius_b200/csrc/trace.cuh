@@ -259,36 +259,26 @@ __device__ __forceinline__ void init_state_ks(const FrameDev& F, const double di
 // last); DP_E[j] = b_{j+1} - b*_{j+1}. Rows are read with a warp-uniform index
 // (constant-cache broadcast).
 // ---------------------------------------------------------------------------
-template <class T>
 struct DPTable {
-    T A[6][6];
-    T E[7];
+    double A[6][6];
+    double E[7];
 };
-#define SIRIUS_DP45_TABLE(T)                                                                                      \
-    {{{T(1.0 / 5.0), T(3.0 / 40.0), T(44.0 / 45.0), T(19372.0 / 6561.0), T(9017.0 / 3168.0), T(35.0 / 384.0)},      \
-      {T(9.0 / 40.0), T(-56.0 / 15.0), T(-25360.0 / 2187.0), T(-355.0 / 33.0), T(0), T(0)},                        \
-      {T(32.0 / 9.0), T(64448.0 / 6561.0), T(46732.0 / 5247.0), T(500.0 / 1113.0), T(0), T(0)},                    \
-      {T(-212.0 / 729.0), T(49.0 / 176.0), T(125.0 / 192.0), T(0), T(0), T(0)},                                     \
-      {T(-5103.0 / 18656.0), T(-2187.0 / 6784.0), T(0), T(0), T(0), T(0)},                                          \
-      {T(11.0 / 84.0), T(0), T(0), T(0), T(0), T(0)}},                                                              \
-     {T(35.0 / 384.0 - 5179.0 / 57600.0), T(0), T(500.0 / 1113.0 - 7571.0 / 16695.0),                              \
-      T(125.0 / 192.0 - 393.0 / 640.0), T(-2187.0 / 6784.0 + 92097.0 / 339200.0), T(11.0 / 84.0 - 187.0 / 2100.0),  \
-      T(-1.0 / 40.0)}}
-static __constant__ DPTable<float> kDPf = SIRIUS_DP45_TABLE(float);
-static __constant__ DPTable<double> kDPd = SIRIUS_DP45_TABLE(double);
-
-template <class T>
-__device__ __forceinline__ const DPTable<T>& dp_table();
-template <>
-__device__ __forceinline__ const DPTable<float>& dp_table<float>() { return kDPf; }
-template <>
-__device__ __forceinline__ const DPTable<double>& dp_table<double>() { return kDPd; }
+static __constant__ DPTable kDPd = {
+    {{1.0 / 5.0, 3.0 / 40.0, 44.0 / 45.0, 19372.0 / 6561.0, 9017.0 / 3168.0, 35.0 / 384.0},
+     {9.0 / 40.0, -56.0 / 15.0, -25360.0 / 2187.0, -355.0 / 33.0, 0, 0},
+     {32.0 / 9.0, 64448.0 / 6561.0, 46732.0 / 5247.0, 500.0 / 1113.0, 0, 0},
+     {-212.0 / 729.0, 49.0 / 176.0, 125.0 / 192.0, 0, 0, 0},
+     {-5103.0 / 18656.0, -2187.0 / 6784.0, 0, 0, 0, 0},
+     {11.0 / 84.0, 0, 0, 0, 0, 0}},
+    {35.0 / 384.0 - 5179.0 / 57600.0, 0, 500.0 / 1113.0 - 7571.0 / 16695.0, 125.0 / 192.0 - 393.0 / 640.0,
+     -2187.0 / 6784.0 + 92097.0 / 339200.0, 11.0 / 84.0 - 187.0 / 2100.0, -1.0 / 40.0}};
 
 // One DP45 attempt on y = (x^mu, p_mu) with the stage arithmetic in T (float:
 // the FP32 bulk; double: FP64). The state stays in FP64; stage inputs are
-// x + h acc where acc = sum_j a_sj k_j accumulates in T in a sliding window, so
-// the six right-hand sides share one call site (a compact loop body keeps the
-// instruction stream in cache). The p_0 component is not accumulated: every
+// x + h acc where acc = sum_j a_sj k_j accumulates in T. In FP32 the sums sit in
+// a sliding window, so the six right-hand sides share one call site (a compact
+// loop body keeps the instruction stream in cache); the FP64 form is
+// dp45_attempt_f64. The p_0 component is not accumulated: every
 // family's metric is static, so dp_0/dl = 0 and p_0 (the conserved -E) carries
 // through the attempt unchanged. On entry k1 = f(x, p); on exit (xn, pn) is the
 // fifth-order solution and k7 = f(xn, pn) (first same as last). Returns the
@@ -392,158 +382,100 @@ __device__ __forceinline__ double dp45_attempt_x2(const MetricDev& m, const CfgD
     return double(sqrtp_(tmax(0.25f * en, 1e-30f)));
 }
 
-template <class T, int FAM = kAnyFamily>
-__device__ __forceinline__ double dp45_attempt(const MetricDev& m, const CfgDev& c, const double x[4], const double p[4],
-                                               double h, const T k1[8], double xn[4], double pn[4], T k7[8]) {
-    if constexpr (std::is_same<T, float>::value) return dp45_attempt_x2<FAM>(m, c, x, p, h, k1, xn, pn, k7);
-    const DPTable<T>& D = dp_table<T>();
-    const T ht = T(h);
-    T X[8];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { X[i] = T(x[i]); X[4 + i] = T(p[i]); }
-    T acc[6][8];
-    T eacc[4];
-    T kc[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        kc[i] = k1[i];
-#pragma unroll
-        for (int s = 0; s < 6; ++s) acc[s][i] = T(0);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) eacc[i] = T(0);
-#pragma unroll 1
-    for (int j = 0; j < 6; ++j) {
-        // fold k_{j+1} into the inputs of every later stage, and into the error
-#pragma unroll
-        for (int s = 0; s < 6; ++s) {
-            const T a = D.A[j][s];
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (i != 4) acc[s][i] += a * kc[i];
-        }
-        const T e = D.E[j];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) eacc[i] += e * kc[i];
-        T xs[4], ps[4];
-        if (j == 5) {  // stage 7 is the solution point
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                xn[i] = x[i] + h * double(acc[0][i]);
-                pn[i] = i == 0 ? p[0] : p[i] + h * double(acc[0][4 + i]);
-                xs[i] = T(xn[i]);
-                ps[i] = T(pn[i]);
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                xs[i] = X[i] + ht * acc[0][i];
-                ps[i] = i == 0 ? X[4] : X[4 + i] + ht * acc[0][4 + i];
-            }
-        }
-        rhs<T, FAM>(m, xs, ps, kc, kc + 4);
-        // slide the window: the next stage's input moves to slot 0
-#pragma unroll
-        for (int s = 0; s < 5; ++s)
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (i != 4) acc[s][i] = acc[s + 1][i];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) acc[5][i] = T(0);
-    }
-    T en = T(0);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        k7[i] = kc[i];
-        k7[4 + i] = kc[4 + i];
-        const T ex = eacc[i] + D.E[6] * kc[i];
-        if constexpr (sizeof(T) == sizeof(double)) {
-            const double e = h * double(ex) / (c.atol + c.rtol * fabs(xn[i]));
-            en += e * e;
-        } else {  // the estimate needs a few digits only
-            const float e = ht * ex * rcp_(c.fatol + c.frtol * fabsf(float(xn[i])));
-            en += e * e;
-        }
-    }
-    if constexpr (sizeof(T) == sizeof(double)) return sqrt(0.25 * en);
-    else return double(sqrtp_(tmax(T(0.25) * en, T(1e-30))));  // 1e-15 when the estimate vanishes
-}
-
-// The same DP45 attempt in FP64 with the stage derivatives in a thread-local
-// array indexed at run time (L1-resident local memory instead of registers): the
-// rare FP64 island steps of the mixed path then do not set its register budget.
-// Butcher form: stage s input = x + h sum_{j<s} a_sj k_j, with the tableau rows
-// of DP_A read back as a_{s, j+1} = A[j][s-1-j].
-template <int FAM = kAnyFamily>
-__device__ __forceinline__ double dp45_attempt_lowreg(const MetricDev& m, const CfgDev& c, const double x[4],
-                                                      const double p[4], double h, const double k1[8], double xn[4],
-                                                      double pn[4], double k7[8]) {
-    const DPTable<double>& D = kDPd;
-    double K[7][8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) K[0][i] = k1[i];
-#pragma unroll 1
-    for (int s = 1; s < 7; ++s) {
-        double sx[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) sx[i] = 0.0;
-#pragma unroll 1
-        for (int j = 0; j < s; ++j) {
-            const double a = D.A[j][s - 1 - j];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) sx[i] += a * K[j][i];
-        }
+// The FP64 attempt, stage by stage in straight-line code: no window to slide
+// (40 register moves a stage in a rolled loop) and only the tableau's non-zero
+// entries folded (147 + 32 multiply-adds, against 252 + 24 with the zeros). k_1..k_3 are kept until
+// stage 5, where they fold into the sums of stages 5, 6, the solution and the error
+// estimate, which the later k then join: at most 25 sums are live, where a sum
+// per later stage from the start keeps 35. The sums run in the order of the k.
+// With the FP64 projection, step control and crossing location of the same step:
+// 717 x 405 FP64 frame 7.45 -> 5.78 ms, 160 x 90 mixed frame (its near-critical rays
+// take FP64 steps, and the longest sets its time) 2.01 -> 1.55 ms.
+template <int FAM>
+__device__ __forceinline__ double dp45_attempt_f64(const MetricDev& m, const CfgDev& c, const double x[4],
+                                                   const double p[4], double h, const double k1[8], double xn[4],
+                                                   double pn[4], double k7[8]) {
+    const DPTable& D = kDPd;
+    constexpr int C[7] = {0, 1, 2, 3, 5, 6, 7};  // the components that change (p_0 is constant)
+    double k2[8], k3[8], k4[8], sx[8], a6[7], b[7], e[4];
+    auto stage = [&](double kk[8]) {  // kk = f(x + h sx)
         double xs[4], ps[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             xs[i] = x[i] + h * sx[i];
-            ps[i] = p[i] + h * sx[4 + i];
+            ps[i] = i == 0 ? p[0] : p[i] + h * sx[4 + i];
         }
-        if (s == 6) {
+        rhs<double, FAM>(m, xs, ps, kk, kk + 4);
+    };
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { xn[i] = xs[i]; pn[i] = ps[i]; }
-        }
-        rhs<double, FAM>(m, xs, ps, K[s], K[s] + 4);
+    for (int q = 0; q < 7; ++q) sx[C[q]] = D.A[0][0] * k1[C[q]];
+    stage(k2);
+#pragma unroll
+    for (int q = 0; q < 7; ++q) sx[C[q]] = D.A[0][1] * k1[C[q]] + D.A[1][0] * k2[C[q]];
+    stage(k3);
+#pragma unroll
+    for (int q = 0; q < 7; ++q)
+        sx[C[q]] = D.A[0][2] * k1[C[q]] + D.A[1][1] * k2[C[q]] + D.A[2][0] * k3[C[q]];
+    stage(k4);
+#pragma unroll
+    for (int q = 0; q < 7; ++q) {
+        const int i = C[q];
+        sx[i] = D.A[0][3] * k1[i] + D.A[1][2] * k2[i] + D.A[2][1] * k3[i] + D.A[3][0] * k4[i];
+        a6[q] = D.A[0][4] * k1[i] + D.A[1][3] * k2[i] + D.A[2][2] * k3[i] + D.A[3][1] * k4[i];
+        b[q] = D.A[0][5] * k1[i] + D.A[2][3] * k3[i] + D.A[3][2] * k4[i];
+        if (i < 4) e[i] = D.E[0] * k1[i] + D.E[2] * k3[i] + D.E[3] * k4[i];
     }
+    stage(k2);  // k_5
+#pragma unroll
+    for (int q = 0; q < 7; ++q) {
+        const int i = C[q];
+        sx[i] = a6[q] + D.A[4][0] * k2[i];
+        b[q] += D.A[4][1] * k2[i];
+        if (i < 4) e[i] += D.E[4] * k2[i];
+    }
+    stage(k3);  // k_6
+#pragma unroll
+    for (int q = 0; q < 7; ++q) {
+        const int i = C[q];
+        b[q] += D.A[5][0] * k3[i];
+        if (i < 4) e[i] += D.E[5] * k3[i];
+        (i < 4 ? xn[i] : pn[i - 4]) = (i < 4 ? x[i] : p[i - 4]) + h * b[q];
+    }
+    pn[0] = p[0];
+    rhs<double, FAM>(m, xn, pn, k7, k7 + 4);
     double en = 0.0;
-#pragma unroll 1
-    for (int i = 0; i < 4; ++i) {
-        double ex = 0.0;
-#pragma unroll 1
-        for (int j = 0; j < 7; ++j) ex += D.E[j] * K[j][i];
-        const double e = h * ex / (c.atol + c.rtol * fabs(xn[i]));
-        en += e * e;
-    }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) k7[i] = K[6][i];
+    for (int i = 0; i < 4; ++i) {
+        const double s = h * (e[i] + D.E[6] * k7[i]) * rcp_(c.atol + c.rtol * fabs(xn[i]));
+        en += s * s;
+    }
     return sqrt(0.25 * en);
 }
 
+template <class T, int FAM = kAnyFamily>
+__device__ __forceinline__ double dp45_attempt(const MetricDev& m, const CfgDev& c, const double x[4], const double p[4],
+                                               double h, const T k1[8], double xn[4], double pn[4], T k7[8]) {
+    if constexpr (std::is_same<T, float>::value) return dp45_attempt_x2<FAM>(m, c, x, p, h, k1, xn, pn, k7);
+    else return dp45_attempt_f64<FAM>(m, c, x, p, h, k1, xn, pn, k7);
+}
+
 // Event location of the equatorial crossing inside an accepted step: DP45
-// sub-steps from the step's start state (x0, p0) with f(x0, p0) recomputed in
-// T, the sub-step length corrected by Newton on z(l) (dz/dl = k^z), seeded by
-// the cubic Hermite root; two sub-steps and a final first-order correction.
-// LOWREG (FP64 only) takes the sub-steps with the local-array attempt, for the
-// mixed path's rare FP64 steps: with the register-resident attempt, the 48 FP64
-// stage accumulators of this rare path set the mixed kernel's register count.
-template <class T, int FAM = kAnyFamily, bool LOWREG = false>
+// sub-steps from the step's start state (x0, p0) with f(x0, p0) recomputed, the
+// sub-step length corrected by Newton on z(l) (dz/dl = k^z), seeded by the cubic
+// Hermite root; two sub-steps and a final first-order correction, in FP64.
+template <int FAM = kAnyFamily>
 __device__ __forceinline__ void locate_equator(const MetricDev& m, const CfgDev& c, const double x0[4],
                                             const double p0[4], double hs, double& xc1, double& xc2) {
-    static_assert(!LOWREG || sizeof(T) == sizeof(double), "the low-register attempt is FP64");
-    T xk[4], pk[4], k0[8], k7[8];
-    for (int i = 0; i < 4; ++i) { xk[i] = T(x0[i]); pk[i] = T(p0[i]); }
-    rhs<T, FAM>(m, xk, pk, k0, k0 + 4);
-    double xn[4], pn[4];
-    auto attempt = [&](double hh) {
-        if constexpr (LOWREG) dp45_attempt_lowreg<FAM>(m, c, x0, p0, hh, k0, xn, pn, k7);
-        else dp45_attempt<T, FAM>(m, c, x0, p0, hh, k0, xn, pn, k7);
-    };
-    attempt(hs);
-    hs -= xn[3] / double(k7[3]);
-    attempt(hs);
-    const double dl = -xn[3] / double(k7[3]);
-    xc1 = xn[1] + dl * double(k7[1]);
-    xc2 = xn[2] + dl * double(k7[2]);
+    double k0[8], k7[8], xn[4], pn[4];
+    rhs<double, FAM>(m, x0, p0, k0, k0 + 4);
+#pragma unroll 1
+    for (int it = 0; it < 2; ++it) {
+        if (it) hs -= xn[3] / k7[3];
+        dp45_attempt_f64<FAM>(m, c, x0, p0, hs, k0, xn, pn, k7);
+    }
+    const double dl = -xn[3] / k7[3];
+    xc1 = xn[1] + dl * k7[1];
+    xc2 = xn[2] + dl * k7[2];
 }
 
 // The mixed path's event location: one FP32 DP45 sub-step of length hs from
@@ -562,10 +494,25 @@ __device__ __forceinline__ void locate_equator_f32(const MetricDev& m, const Cfg
     xc2 = xn[2] + dl * double(k7[2]);
 }
 
+// e^(-1/5) of e > 0: an FP32 estimate from the hardware logarithm and exponential
+// (1e-5 relative at worst), and two Newton steps of y -> y + y (1 - e y^5) / 5, whose
+// error goes from d to 3 d^2: FP64 rounding after the second (twelve FP64
+// operations, where pow takes more than a right-hand side). An estimate that under-
+// or overflowed stays as it is (the caller clamps the factor).
+__device__ __forceinline__ double inv_root5(double e) {
+    double y = double(exp2f(-0.2f * __log2f(float(e))));
+#pragma unroll
+    for (int it = 0; it < 2; ++it) {
+        const double y2 = y * y;
+        y += 0.2 * y * (1.0 - e * y * (y2 * y2));
+    }
+    return y;
+}
+
 // Geodesic::computeOptimalStep (PHGD001A.cpp:471-483).
 __device__ __forceinline__ double optimal_step(double h, double err, const CfgDev& c) {
     if (err < 1e-15) return fmin(h * c.grow, c.hmax);
-    double fac = c.safety * pow(1.0 / err, 0.2);
+    double fac = c.safety * inv_root5(err);
     fac = fmax(c.shrink, fmin(c.grow, fac));
     return fmax(c.hmin, fmin(c.hmax, h * fac));
 }
@@ -662,16 +609,27 @@ __device__ __forceinline__ float volume_step_cap_f(float r, float z, float vx, f
     return fmaxf(0.5f * H, dist) * rsqrtf(fmaxf(vx * vx + vy * vy + vz * vz, 1e-6f));
 }
 
-// Cubic Hermite interpolation of z over the accepted step; bisection for z = 0.
+// The zero in [0, 1] of the cubic Hermite interpolant of z over the accepted step
+// (z0 and z1 have opposite signs): Newton from the chord's zero, kept inside the
+// shrinking bracket (a step that leaves it bisects), to FP64 rounding. Four or five
+// iterations of nine dependent operations, where bisection to the same width takes 60.
 __device__ __forceinline__ double hermite_root(double z0, double z1, double dz0, double dz1, double h) {
-    double lo = 0.0, hi = 1.0, flo = z0;
+    const double m0 = h * dz0, m1 = h * dz1, d = z1 - z0;
+    const double c2 = 3.0 * d - 2.0 * m0 - m1, c3 = m0 + m1 - 2.0 * d;
+    double lo = 0.0, hi = 1.0, s = -z0 / d;
+#pragma unroll 1
     for (int it = 0; it < 60; ++it) {
-        const double s = 0.5 * (lo + hi), s2 = s * s, s3 = s2 * s;
-        const double f = (2.0 * s3 - 3.0 * s2 + 1.0) * z0 + (s3 - 2.0 * s2 + s) * h * dz0 +
-                         (-2.0 * s3 + 3.0 * s2) * z1 + (s3 - s2) * h * dz1;
-        if ((f < 0.0) == (flo < 0.0)) { lo = s; flo = f; } else { hi = s; }
+        const double f = z0 + s * (m0 + s * (c2 + s * c3));
+        const double df = m0 + s * (2.0 * c2 + s * (3.0 * c3));
+        if ((f < 0.0) == (z0 < 0.0)) lo = s;
+        else hi = s;
+        double t = s - f / df;
+        if (!(t > lo && t < hi)) t = 0.5 * (lo + hi);
+        const double step = fabs(t - s);
+        s = t;
+        if (step < 1e-15) break;
     }
-    return 0.5 * (lo + hi);
+    return s;
 }
 
 // Keplerian emitter at BL radius rbl seen from the camera: g = (p.u_obs)/(p.u_em),

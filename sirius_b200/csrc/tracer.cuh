@@ -489,18 +489,18 @@ __device__ __noinline__ IslandStep island_attempt(const MetricDev& m, const CfgD
     IslandStep o;
     double k1[8], k7[8];
     rhs<double, FAM>(m, x.v, p.v, k1, k1 + 4);
-    o.err = dp45_attempt_lowreg<FAM>(m, c, x.v, p.v, h, k1, o.xn, o.pn, k7);
+    o.err = dp45_attempt_f64<FAM>(m, c, x.v, p.v, h, k1, o.xn, o.pn, k7);
 #pragma unroll
     for (int i = 0; i < 8; ++i) o.k7[i] = float(k7[i]);
     return o;
 }
 
-// The equatorial crossing of an accepted island step, located in FP64.
+// The equatorial crossing of an accepted FP64 step (out of line: it carries its own attempt).
 template <int FAM>
-__device__ __noinline__ CrossXY island_crossing(const MetricDev& m, const CfgDev& c, const Vec4v x, const Vec4v p,
+__device__ __noinline__ CrossXY crossing_f64(const MetricDev& m, const CfgDev& c, const Vec4v x, const Vec4v p,
                                                 double hs) {
     CrossXY o;
-    locate_equator<double, FAM, true>(m, c, x.v, p.v, hs, o.x, o.y);
+    locate_equator<FAM>(m, c, x.v, p.v, hs, o.x, o.y);
     return o;
 }
 
@@ -658,7 +658,7 @@ __device__ __forceinline__ int advance_post(const Params& P, Ray<MIXED>& s, bool
         const double hs = hermite_root(s.x[3], xn[3], double(s.k[3]), double(k7[3]), hstep) * hstep;
         if constexpr (MIXED) {
             if (island) {
-                const CrossXY o = island_crossing<FAM>(m, c, vec4v(s.x), vec4v(s.p), hs);
+                const CrossXY o = crossing_f64<FAM>(m, c, vec4v(s.x), vec4v(s.p), hs);
                 xc1 = o.x;
                 xc2 = o.y;
             }
@@ -671,7 +671,9 @@ __device__ __forceinline__ int advance_post(const Params& P, Ray<MIXED>& s, bool
                 xc2 = o.y;
             }
         } else {
-            locate_equator<double, FAM>(m, c, s.x, s.p, hs, xc1, xc2);
+            const CrossXY o = crossing_f64<FAM>(m, c, vec4v(s.x), vec4v(s.p), hs);
+            xc1 = o.x;
+            xc2 = o.y;
         }
     }
     double x0[4];
@@ -697,28 +699,29 @@ __device__ __forceinline__ int advance_post(const Params& P, Ray<MIXED>& s, bool
     const bool project = c.proj_period > 0 && (s.steps % c.proj_period) == 0;
     const bool ks_fast = MIXED && is_family<FAM>(m, SIRIUS_METRIC_KERR_SCHILD) && !m.has_lambda;
     if (project) {
-        double pb[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) pb[i] = s.p[i];
         double before;
+        bool stale;  // the projection moved p beyond what the stored f(x, p) resolves: recompute it
         if (ks_fast) {
-            before = project_null_ks_mixed(m, s.x, s.p, rr);
+            before = project_null_ks_mixed(m, s.x, s.p, rr, stale);
         } else {
+            double pb[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) pb[i] = s.p[i];
             InvForm IF;
             inv_form(m, s.x, IF);
             rr = IF.r;
             before = project_null(m, IF, s.p);
+            // 1e-10 relative in FP64, 1e-6 with FP32 storage
+            double dp = 0.0, pm = 0.0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                dp = fmax(dp, fabs(s.p[i] - pb[i]));
+                pm = fmax(pm, fabs(s.p[i]));
+            }
+            stale = dp > (MIXED ? 1e-6 : 1e-10) * pm;
         }
         s.null_max = fmaxf(s.null_max, float(fabs(before)));
-        // a projection that moved p beyond what the stored f(x, p) resolves
-        // (1e-10 relative in FP64, 1e-6 with FP32 storage) makes it stale: recompute it
-        double dp = 0.0, pm = 0.0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            dp = fmax(dp, fabs(s.p[i] - pb[i]));
-            pm = fmax(pm, fabs(s.p[i]));
-        }
-        if (dp > (MIXED ? 1e-6 : 1e-10) * pm) refresh_derivative<MIXED, FAM>(m, s);
+        if (stale) refresh_derivative<MIXED, FAM>(m, s);
     } else if (ks_fast) {
         rr = ks_radius(m, s.x);
     } else {
