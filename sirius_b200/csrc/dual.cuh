@@ -25,21 +25,53 @@
 namespace sirius {
 
 #ifdef __CUDACC__
-// Reciprocal and square root used by the metric code. FP32 uses the
-// fast single-instruction forms (the FP32 path is an approximation by design:
-// its error budget is set by the FP64 state accumulation and FP64 projection);
-// FP64 uses IEEE-rounded division and square root.
-__device__ __forceinline__ float rcp_(float x) { return __fdividef(1.0f, x); }
-__device__ __forceinline__ double rcp_(double x) { return 1.0 / x; }
+// Reciprocal and roots used by the metric code.
+//
+// FP32: the special-function unit's approximations as they are (an approximation
+// by design: the error budget of the FP32 path is set by the FP64 state and
+// projection), without the subnormal scaling that the CUDA functions add around
+// them; every normal argument gives the same bits either way.
+//
+// FP64: the unit's seeds (PTX rcp.approx.ftz.f64 and rsqrt.approx.ftz.f64) and one
+// third-order Householder step, e the seed's residual:
+//   1/x:        e = 1 - x y,    y <- y + y (e + e^2)
+//   1/sqrt(x):  e = 1 - x y^2,  y <- y + y e (1/2 + 3/8 e)
+// A seed good to 2^-20 leaves 2^-60, so the result is within an ulp or so, as the
+// CUDA functions' are; positive normal arguments only, so there is no
+// special-case branch beside each of the three per right-hand side (717 x 405 FP64
+// frame 5.78 -> 4.63 ms, 1024^2 mixed frame 20.3 -> 18.1 ms). Against 1/x and
+// 1/sqrt(x) in extended precision over e^-50..e^50 the largest relative errors are
+// 1.1e-16 and 1.4e-16 (the CUDA functions: 1.1e-16 both). A NaN or an infinite
+// argument gives NaN.
+__device__ __forceinline__ float rcp_(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rsqrt_(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ double rcp_(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ double rsqrt_(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x * y, y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
 __device__ __forceinline__ float sqrt_(float x) { return sqrtf(x); }
 __device__ __forceinline__ double sqrt_(double x) { return sqrt(x); }
-__device__ __forceinline__ float rsqrt_(float x) { return rsqrtf(x); }
 // Square root of a positive argument. FP32: x * rsqrt(x), two instructions with
 // single-precision relative accuracy (the correctly rounded sqrtf is a longer
 // sequence with a special-case branch); FP64: sqrt.
-__device__ __forceinline__ float sqrtp_(float x) { return x * rsqrtf(x); }
+__device__ __forceinline__ float sqrtp_(float x) { return x * rsqrt_(x); }
 __device__ __forceinline__ double sqrtp_(double x) { return sqrt(x); }
-__device__ __forceinline__ double rsqrt_(double x) { return rsqrt(x); }
 __device__ __forceinline__ float exp_(float x) { return __expf(x); }
 __device__ __forceinline__ double exp_(double x) { return exp(x); }
 __device__ __forceinline__ float tanh_(float x) { return tanhf(x); }

@@ -395,7 +395,7 @@ __device__ __forceinline__ void inv_form(const MetricDev& m, const double x[4], 
     const double isd = rsqrt_(disc);
     const double r2 = fmax(0.5 * (Rm2 + disc * isd), 1e-10);
     const double ir = rsqrt_(r2), r = r2 * ir;
-    const double den = r2 + a2, iden = 1.0 / den;
+    const double den = r2 + a2, iden = rcp_(den);
     F.r = r;
     F.d[1] = r * X * isd; F.d[2] = r * Y * isd; F.d[3] = Z * den * ir * isd;
     F.l[0] = -1.0;  // l# = eta l
@@ -467,7 +467,7 @@ __device__ __forceinline__ double project_null_ks_mixed(const MetricDev& m, cons
     const double r2 = fmax(0.5 * (Rm2 + disc2 * isd), 1e-10);
     const double ir = rsqrt_(r2), r = r2 * ir;
     r_out = r;
-    const double den = r2 + a2, iden = 1.0 / den;
+    const double den = r2 + a2, iden = rcp_(den);
     const double l1 = (r * X + a * Y) * iden, l2 = (r * Y - a * X) * iden, l3 = Z * ir;
     const double H = (2.0 * m.M * r - m.Q2) * isd;
     const double lp = -p[0] + l1 * p[1] + l2 * p[2] + l3 * p[3];
