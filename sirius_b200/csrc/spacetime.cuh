@@ -440,9 +440,10 @@ __device__ __forceinline__ double project_null(const MetricDev& m, const InvForm
     const double C = inv_apply(m, F, p, p);
     const double disc = B * B - 4.0 * A * C;
     if (disc < 0.0 || fabs(A) < 1e-15) return C;
-    const double q = -0.5 * (B + (B >= 0.0 ? sqrt(disc) : -sqrt(disc)));
+    const double sq = disc * rsqrt_(fmax(disc, 1e-280));
+    const double q = -0.5 * (B + (B >= 0.0 ? sq : -sq));
     if (q == 0.0) return C;
-    const double alpha = C / q;
+    const double alpha = C * rcp_(q);
 #pragma unroll
     for (int i = 0; i < 4; ++i) p[i] += alpha * F.d[i];
     return C;

@@ -449,7 +449,8 @@ __device__ __forceinline__ double dp45_attempt_f64(const MetricDev& m, const Cfg
         const double s = h * (e[i] + D.E[6] * k7[i]) * rcp_(c.atol + c.rtol * fabs(xn[i]));
         en += s * s;
     }
-    return sqrt(0.25 * en);
+    en *= 0.25;
+    return en * rsqrt_(fmax(en, 1e-280));
 }
 
 template <class T, int FAM = kAnyFamily>

@@ -296,7 +296,8 @@ __device__ __forceinline__ void volumetric_segment(const Params& P, const FrameD
     const int nq = c.vol_sub < 1 ? 1 : (c.vol_sub > 4 ? 4 : c.vol_sub);
     const float E = float(-p[0]);
     const float Lz = float(x1[1] * p[2] - x1[2] * p[1]);
-    const float nu_cam = E / observer_factor<float>(F, E);
+    const float nu_cam = E * rcp_(observer_factor<float>(F, E));
+    const float iaoj = rcp_(c.fvol_aoj);
     const float rin = F.fdisk_in, rout = F.fdisk_out;
     const bool in0 = r0 >= rin && r0 <= rout, in1 = r1 >= rin && r1 <= rout;
     float xf0[3], dxf[3];
@@ -360,15 +361,15 @@ __device__ __forceinline__ void volumetric_segment(const Params& P, const FrameD
         point(fa + span * double(kGLx[nq - 1][s]), xs, ys, zs);
         const float r = ks_r(F.m, xs, ys, zs);
         if (r < rin || r > rout) return;
-        const float zr = zs / (c.fvol_hz * r);
+        const float zr = zs * rcp_(c.fvol_hz * r);
         if (fabsf(zr) > float(kVolCutoff)) return;
         const float g = kepler_g<float>(F.m, xs, ys, zs, r, E, Lz, observer_factor<float>(F, E));
         if (!(g > 0.f)) return;
         const float dl = float(h * span) * kGLw[nq - 1][s];
-        const float jsp = c.fvol_j0 / (r * r) * __expf(-0.5f * zr * zr);
+        const float jsp = c.fvol_j0 * rcp_(r * r) * __expf(-0.5f * zr * zr);
         const float gs = __powf(g, c.fvol_s);  // nu_em^-s = (g/nu_b)^s
-        dts = c.fvol_aoj * jsp * gs * (nu_cam / g) * dl;
-        Ss = g * g * g / c.fvol_aoj;
+        dts = c.fvol_aoj * jsp * gs * (nu_cam * rcp_(g)) * dl;
+        Ss = g * g * g * iaoj;
     };
     // the Gauss-Legendre points in step order, each applied to every bin pair
     // (a point outside the emitting region, or with no redshift, leaves the bins
