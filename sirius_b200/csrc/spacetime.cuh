@@ -214,10 +214,17 @@ SIRIUS_HD __forceinline__ void ks_rhs_terms(const MetricDev& m, const T x[4], co
 // roots and four reciprocals, and 94 operations instead of 143 (717 x 405 FP64
 // frame 8.73 -> 7.45 ms from this alone). The FP32 arithmetic keeps the terms: the two forms round
 // differently, and near the critical curve FP32 roundings reach the image.
+// In three parts: what depends on the position alone (KSGeom), the velocity and the
+// force at a momentum, so that the symplectic integrator, which takes two kicks and
+// a drift at each position, evaluates the geometry once.
 template <class T>
-SIRIUS_HD __forceinline__ void ks_rhs_closed(const MetricDev& m, const T x[4], const T p[4], T k[4], T f[4]) {
+struct KSGeom {
+    T X, Y, Z, r, ir, isd, iden, den, l1, l2, l3, H, w, c, hz;  // c = Lambda R^2 / 3, hz = a^2 z / (r sd)
+};
+
+template <class T>
+SIRIUS_HD __forceinline__ void ks_geom(const MetricDev& m, T X, T Y, T Z, KSGeom<T>& G) {
     const T a = cst<T>(m.a, m.fa), a2 = cst<T>(m.a2, m.fa2), M2 = cst<T>(2.0 * m.M, m.fM2);
-    const T X = x[1], Y = x[2], Z = x[3];
     const T zz = Z * Z;
     const T R2 = X * X + Y * Y + zz;
     const T Rm2 = R2 - a2;
@@ -228,38 +235,60 @@ SIRIUS_HD __forceinline__ void ks_rhs_closed(const MetricDev& m, const T x[4], c
     const T r = r2 * ir;
     const T den = r2 + a2;
     const T iden = rcp_(den);
-    const T l1 = (r * X + a * Y) * iden, l2 = (r * Y - a * X) * iden, l3 = Z * ir;
     const T q = M2 * r - cst<T>(m.Q2, m.fQ2);
-    const T H = q * isd;
-    // k = g^{-1} p = eta p - H l# (l# . p), l# = (-1, l1, l2, l3)
-    const T lp = -p[0] + l1 * p[1] + l2 * p[2] + l3 * p[3];
-    const T Hlp = H * lp;
+    G.X = X; G.Y = Y; G.Z = Z; G.r = r; G.ir = ir; G.isd = isd; G.iden = iden; G.den = den;
+    G.l1 = (r * X + a * Y) * iden;
+    G.l2 = (r * Y - a * X) * iden;
+    G.l3 = Z * ir;
+    G.H = q * isd;
+    G.w = (M2 + T(2) * q * ir - T(4) * G.H * r) * isd;
+    G.hz = a2 * G.l3 * isd;
+    G.c = m.has_lambda ? cst<T>(m.lam3, m.flam3) * R2 : T(0);
+}
+
+// k = g^{-1} p = eta p - H l# (l# . p), l# = (-1, l1, l2, l3); lk = l . k
+template <class T>
+SIRIUS_HD __forceinline__ void ks_velocity(const MetricDev& m, const KSGeom<T>& G, const T p[4], T k[4], T& lk) {
+    const T lp = -p[0] + G.l1 * p[1] + G.l2 * p[2] + G.l3 * p[3];
+    const T Hlp = G.H * lp;
     k[0] = -p[0] + Hlp;
-    k[1] = p[1] - l1 * Hlp;
-    k[2] = p[2] - l2 * Hlp;
-    k[3] = p[3] - l3 * Hlp;
-    T lk = lp;
+    k[1] = p[1] - G.l1 * Hlp;
+    k[2] = p[2] - G.l2 * Hlp;
+    k[3] = p[3] - G.l3 * Hlp;
+    lk = lp;
     if (m.has_lambda) {
-        const T c = cst<T>(m.lam3, m.flam3) * R2;
-        const T w0 = -T(1) - H, w1 = H * l1, w2 = H * l2, w3 = H * l3;
-        const T s = c * (w0 * p[0] + w1 * p[1] + w2 * p[2] + w3 * p[3]) * rcp_(T(1) + c * (T(1) + H));
+        const T w0 = -T(1) - G.H, w1 = G.H * G.l1, w2 = G.H * G.l2, w3 = G.H * G.l3;
+        const T s = G.c * (w0 * p[0] + w1 * p[1] + w2 * p[2] + w3 * p[3]) * rcp_(T(1) + G.c * (T(1) + G.H));
         k[0] += s * w0; k[1] += s * w1; k[2] += s * w2; k[3] += s * w3;
-        lk = k[0] + l1 * k[1] + l2 * k[2] + l3 * k[3];
+        lk = k[0] + G.l1 * k[1] + G.l2 * k[2] + G.l3 * k[3];
     }
-    const T S = (X * k[1] + Y * k[2] - T(2) * r * (l1 * k[1] + l2 * k[2])) * iden - k[3] * l3 * ir;
-    const T w = (M2 + T(2) * q * ir - T(4) * H * r) * isd;
-    const T Hlk = H * lk, e = Hlk * iden;
-    const T g = lk * (T(0.5) * w * lk + H * S) * isd;
-    const T gr = g * r;
+}
+
+// f_i = dp_i / dl, i = 1..3 (f_0 = 0: the metric is static), from the velocity
+template <class T>
+SIRIUS_HD __forceinline__ void ks_force(const MetricDev& m, const KSGeom<T>& G, const T k[4], T lk, T f[4]) {
+    const T a = cst<T>(m.a, m.fa);
+    const T S = (G.X * k[1] + G.Y * k[2] - T(2) * G.r * (G.l1 * k[1] + G.l2 * k[2])) * G.iden - k[3] * G.l3 * G.ir;
+    const T Hlk = G.H * lk, e = Hlk * G.iden;
+    const T g = lk * (T(0.5) * G.w * lk + G.H * S) * G.isd;
+    const T gr = g * G.r;
     f[0] = T(0);
-    f[1] = gr * X + e * (r * k[1] - a * k[2]);
-    f[2] = gr * Y + e * (a * k[1] + r * k[2]);
-    f[3] = ir * (g * den * Z + Hlk * (k[3] - a2 * l3 * isd * lk));
-    // the Lambda term of dp: - Lambda x_i (k^0)^2 / 3
-    if (m.has_lambda) {
+    f[1] = gr * G.X + e * (G.r * k[1] - a * k[2]);
+    f[2] = gr * G.Y + e * (a * k[1] + G.r * k[2]);
+    f[3] = G.ir * (g * G.den * G.Z + Hlk * (k[3] - G.hz * lk));
+    if (m.has_lambda) {  // - Lambda x_i (k^0)^2 / 3
         const T qq = cst<T>(m.lam3, m.flam3) * k[0] * k[0];
-        f[1] -= qq * X; f[2] -= qq * Y; f[3] -= qq * Z;
+        f[1] -= qq * G.X; f[2] -= qq * G.Y; f[3] -= qq * G.Z;
     }
+}
+
+template <class T>
+SIRIUS_HD __forceinline__ void ks_rhs_closed(const MetricDev& m, const T x[4], const T p[4], T k[4], T f[4]) {
+    KSGeom<T> G;
+    T lk;
+    ks_geom(m, x[1], x[2], x[3], G);
+    ks_velocity(m, G, p, k, lk);
+    ks_force(m, G, k, lk, f);
 }
 
 // The Kerr-Schild right-hand side of precision T: the closed form in FP64, the

@@ -85,6 +85,7 @@ struct Ray {
     double x[4], p[4];
     K k[8];
     double h;
+    double r;  // symplectic: the Kerr-Schild radius at x
     double intensity;
     float min_r, null_max, tphi, prev_z;
     float prev_r;  // r at the start of the step (volumetric early-out)
@@ -162,7 +163,8 @@ __device__ __forceinline__ void begin_ray(const Params& P, Ray<MIXED>& s, long l
     s.null_max = 0.f;
     s.tphi = 0.f;
     s.prev_z = float(s.x[3]);
-    s.prev_r = float(ks_radius(F.m, s.x));
+    s.r = ks_radius(F.m, s.x);
+    s.prev_r = float(s.r);
     s.steps = s.rejected = s.attempts = s.ncross = s.eq = s.fp64_steps = 0;
     s.crit = 0;
     if (MIXED && F.gate && P.c.crit_band > 0.0) {
@@ -577,7 +579,7 @@ __device__ __forceinline__ int advance(const Params& P, Ray<MIXED>& s, float& ma
         // does (h0 min(1, ((r - r_+)/r_+)^2), PHSI001A.h:260-263); always accepted
         double hs = c.symp_step;
         if (F.has_horizon) {
-            const double q = (ks_radius(m, s.x) - F.r_plus) / F.r_plus;
+            const double q = (s.r - F.r_plus) * rcp_(F.r_plus);
             hs = fmax(c.hmin, hs * fmin(1.0, q * q));
         }
         s.h = hs;
@@ -588,7 +590,7 @@ __device__ __forceinline__ int advance(const Params& P, Ray<MIXED>& s, float& ma
         K xk[4], pk[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) { xk[i] = K(xn[i]); pk[i] = K(pn[i]); }
-        rhs<K>(m, xk, pk, k7, k7 + 4);
+        rhs<K, FAM>(m, xk, pk, k7, k7 + 4);
         err = 0.0;
     } else if constexpr (MIXED) {
         if (island) {
@@ -697,7 +699,7 @@ __device__ __forceinline__ int advance_post(const Params& P, Ray<MIXED>& s, bool
     // constraint re-projection (E, L_z and Carter preserving); the mixed path
     // forms only the null value in FP64 (Kerr-Schild without Lambda)
     double rr;
-    const bool project = c.proj_period > 0 && (s.steps % c.proj_period) == 0;
+    const bool project = c.proj_period == 1 || (c.proj_period > 1 && (s.steps % c.proj_period) == 0);
     const bool ks_fast = MIXED && is_family<FAM>(m, SIRIUS_METRIC_KERR_SCHILD) && !m.has_lambda;
     if (project) {
         double before;
@@ -730,6 +732,7 @@ __device__ __forceinline__ int advance_post(const Params& P, Ray<MIXED>& s, bool
         inv_form(m, s.x, IF);
         rr = IF.r;
     }
+    s.r = rr;
     if (float(rr) < s.min_r) s.min_r = float(rr);
     if (disk_on && c.enable_vol && !symp)
         s.h = fmax(c.hmin, fmin(s.h, vol_cap<MIXED>(rr, s.x[3], s.k, c, F)));
