@@ -373,37 +373,56 @@ __device__ __forceinline__ void volumetric_segment(const Params& P, const FrameD
         dts = c.fvol_aoj * jsp * gs * (nu_cam * rcp_(g)) * dl;
         Ss = g * g * g * iaoj;
     };
-    // the Gauss-Legendre points in step order, each applied to every bin pair
-    // (a point outside the emitting region, or with no redshift, leaves the bins
-    // as they are)
+    // the Gauss-Legendre points of the step, then every bin pair through all of them
+    // in step order (a point outside the emitting region, or with no redshift, has
+    // dts = 0 and leaves the bins as they are). With the points outside, a pair's
+    // sums are read and written once per step instead of once per point, and the
+    // loop's own instructions are spread over four updates: 1024^2 frame with 16 bins
+    // 17.3 -> 16.5 ms, 128 x 64 sky map with 32 bins 170.6 -> 160.3 ms.
+    float dt[4] = {0.f, 0.f, 0.f, 0.f}, S[4] = {0.f, 0.f, 0.f, 0.f};
+    float deep = 0.f;
+    bool any = false;
 #pragma unroll 1
     for (int s = 0; s < nq; ++s) {
-        float dts, Ss;
-        point_at(s, dts, Ss);
-        if (dts == 0.f) continue;
-        const float2 dt0 = p2(dts), S = p2(Ss);
-        // bins in order of falling optical depth (c.nu_desc): once a pair's deeper
-        // bin is below x = 0.04, where the minimum above is the series, every
-        // later pair takes the series alone (the same values, no exponentials)
-        int j = 0;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) { dt[i] = dt[i + 1]; S[i] = S[i + 1]; }
+        point_at(s, dt[3], S[3]);
+        deep = fmaxf(deep, dt[3]);
+        any |= dt[3] != 0.f;
+    }
+    if (!any) return;
+    // bins in order of falling optical depth (c.nu_desc): once a pair's deeper bin is
+    // below x = 0.04 at every point, where the minimum above is the series, every
+    // later pair takes the series alone (the same values, no exponentials)
+    int j = 0;
 #pragma unroll 1
-        for (; j < c.npair; ++j) {
-            const float2 b = mul2(dt0, c.nu_l2[j]);
-            if (c.nu_desc && b.x > -kSeriesOnlyB) break;
-            const float2 I = vol[j * bd];
-            const float2 T = vol[(c.npair + j) * bd];  // transmittance e^-tau to the camera
-            const float2 om = one_minus_exp(b);
-            vol[j * bd] = fma2(mul2(T, S), om, I);
-            vol[(c.npair + j) * bd] = fma2(neg2(T), om, T);
+    for (; j < c.npair; ++j) {
+        const float2 nu = c.nu_l2[j];
+        if (c.nu_desc && deep * nu.x > -kSeriesOnlyB) break;
+        float2 I = vol[j * bd];
+        float2 T = vol[(c.npair + j) * bd];  // transmittance e^-tau to the camera
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const float2 om = one_minus_exp(mul2(p2(dt[s]), nu));
+            I = fma2(mul2(T, p2(S[s])), om, I);
+            T = fma2(neg2(T), om, T);
         }
+        vol[j * bd] = I;
+        vol[(c.npair + j) * bd] = T;
+    }
 #pragma unroll 1
-        for (; j < c.npair; ++j) {
-            const float2 I = vol[j * bd];
-            const float2 T = vol[(c.npair + j) * bd];
-            const float2 om = series(mul2(dt0, c.nu_l2[j]));
-            vol[j * bd] = fma2(mul2(T, S), om, I);
-            vol[(c.npair + j) * bd] = fma2(neg2(T), om, T);
+    for (; j < c.npair; ++j) {
+        const float2 nu = c.nu_l2[j];
+        float2 I = vol[j * bd];
+        float2 T = vol[(c.npair + j) * bd];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const float2 om = series(mul2(p2(dt[s]), nu));
+            I = fma2(mul2(T, p2(S[s])), om, I);
+            T = fma2(neg2(T), om, T);
         }
+        vol[j * bd] = I;
+        vol[(c.npair + j) * bd] = T;
     }
 }
 
