@@ -8,9 +8,10 @@
 // p_mu) carries two tangent vectors V_u = dy/du, V_v = dy/dv (u, v: the pixel
 // coordinates of its start), which obey the linearised equation
 //   dV/dlambda = (df/dy) V,   f = (dx/dlambda, dp/dlambda)
-// (the geodesic deviation equation in first-order form). df/dy V is a central
-// difference of the right-hand side along V; the ray and its tangents advance
-// together by Dormand-Prince 5(4) steps controlled on the ray. When the ray
+// (the geodesic deviation equation in first-order form). df/dy V is the
+// Jacobian-vector product of the closed-form right-hand side (dual numbers with one
+// tangent); the ray and its tangents advance together by Dormand-Prince 5(4) steps
+// controlled on the ray. When the ray
 // escapes, its unit direction n and the tangents' dn/du, dn/dv give the solid
 // angle the pixel maps to on the sky, |dn/du x dn/dv| du dv; the pixel's own
 // solid angle is |dd/du x dd/dv| du dv with d the start direction in the
@@ -56,37 +57,6 @@ __device__ __forceinline__ void beam_start(const FrameDev& F, double u, double v
     init_state(F, dir, y, y + 4);
 }
 
-__device__ __forceinline__ void beam_f(const MetricDev& m, const double y[8], double f[8]) {
-    rhs<double, kAnyFamily>(m, y, y + 4, f, f + 4);
-}
-
-// f(y) and (df/dy) V for both tangents
-__device__ __forceinline__ void beam_rhs(const MetricDev& m, const double Y[24], double FY[24]) {
-    beam_f(m, Y, FY);
-    double ysc = 1.0;
-    for (int i = 0; i < 8; ++i) ysc = fmax(ysc, fabs(Y[i]));
-#pragma unroll 1
-    for (int t = 0; t < 2; ++t) {
-        const double* V = Y + 8 + 8 * t;
-        double vn = 0.0;
-        for (int i = 0; i < 8; ++i) vn = fmax(vn, fabs(V[i]));
-        double* out = FY + 8 + 8 * t;
-        if (!(vn > 0.0)) {
-            for (int i = 0; i < 8; ++i) out[i] = 0.0;
-            continue;
-        }
-        const double eps = 1e-6 * ysc / vn;
-        double yp[8], ym[8], fp[8], fm[8];
-        for (int i = 0; i < 8; ++i) {
-            yp[i] = Y[i] + eps * V[i];
-            ym[i] = Y[i] - eps * V[i];
-        }
-        beam_f(m, yp, fp);
-        beam_f(m, ym, fm);
-        for (int i = 0; i < 8; ++i) out[i] = (fp[i] - fm[i]) / (2.0 * eps);
-    }
-}
-
 __device__ __forceinline__ void cross3(const double a[3], const double b[3], double c[3]) {
     c[0] = a[1] * b[2] - a[2] * b[1];
     c[1] = a[2] * b[0] - a[0] * b[2];
@@ -103,66 +73,146 @@ struct BeamParams {
     int* status;
 };
 
+// f of a state and of its tangent: y = (x, p) and V in, k and dk out (8 components)
+__device__ __forceinline__ void beam_rhs(const MetricDev& m, const double y[8], const double V[8], double f[8],
+                                         double fV[8]) {
+    D1<double> x[4], p[4], k[4], g[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        x[i] = D1<double>(y[i], V[i]);
+        p[i] = D1<double>(y[4 + i], V[4 + i]);
+    }
+    ks_rhs_closed(m, x, p, k, g);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        f[i] = k[i].v; fV[i] = k[i].d;
+        f[4 + i] = g[i].v; fV[4 + i] = g[i].d;
+    }
+}
+
+// Two neighbouring lanes trace a beam: both carry the ray (the same operations on
+// the same values, so the same bits and the same steps), the even lane the tangent
+// along u and the odd lane the one along v; they meet at the end, for the solid
+// angles. A small map is bound by one beam's dependent chain and a large one by
+// FP64 issue: a lane's stage is one right-hand side with one tangent (about 250
+// operations, three of them roots or reciprocals), where one thread with both
+// tangents as central differences took five right-hand sides a stage and kept its
+// seven stage derivatives of 24 components in local memory (120 x 68 beams to
+// R = 1000 M: 22.3 -> 3.1 ms; magnifications against the same steps with exact
+// tangents in 64 bits: both within the rounding of a float). The sums of the stages
+// are those of dp45_attempt_f64.
 __global__ void __launch_bounds__(64) beam_kernel(const __grid_constant__ BeamParams B) {
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long thread = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long idx = thread >> 1;
+    const int dir = int(thread & 1);  // 0: the tangent along u, 1: along v
     if (idx >= B.total) return;
+    const unsigned pair = 3u << (threadIdx.x & 30);
     const int fi = B.n_frames > 1 ? find_frame(B.frames, B.n_frames, idx) : 0;
     const FrameDev& F = B.frames[fi];
     const CfgDev& c = B.c;
-    const MetricDev& m = F.m;
+    const MetricDev m = F.m;
     const long long pix = idx - F.ray_offset;
     const double u0 = double(pix % F.width) + 0.5, v0 = double(F.row0 + pix / F.width) + 0.5;
-    // start: the ray, its tangents along u and v, and the pixel's solid angle
-    double Y[24];
-    beam_start(F, u0, v0, Y);
-    const double hpx = 1e-3;
-    double dd[2][3];
-    for (int t = 0; t < 2; ++t) {
+    // start: the ray, its tangent along this lane's direction, and the derivative of
+    // the pixel direction
+    double y[8], V[8], dd[3];
+    beam_start(F, u0, v0, y);
+    {
+        const double hpx = 1e-3;
         double yp[8], ym[8], dp[4], dm[4];
-        const double du = t == 0 ? hpx : 0.0, dv = t == 0 ? 0.0 : hpx;
+        const double du = dir == 0 ? hpx : 0.0, dv = dir == 0 ? 0.0 : hpx;
         beam_start(F, u0 + du, v0 + dv, yp);
         beam_start(F, u0 - du, v0 - dv, ym);
-        for (int i = 0; i < 8; ++i) Y[8 + 8 * t + i] = (yp[i] - ym[i]) / (2.0 * hpx);
+        for (int i = 0; i < 8; ++i) V[i] = (yp[i] - ym[i]) / (2.0 * hpx);
         camera_dir_exact(F, u0 + du, v0 + dv, dp);
         camera_dir_exact(F, u0 - du, v0 - dv, dm);
-        for (int i = 0; i < 3; ++i) dd[t][i] = (dp[1 + i] - dm[1 + i]) / (2.0 * hpx);
+        for (int i = 0; i < 3; ++i) dd[i] = (dp[1 + i] - dm[1 + i]) / (2.0 * hpx);
     }
-    double d0[4], cimg[3];
-    camera_dir_exact(F, u0, v0, d0);
-    cross3(dd[0], dd[1], cimg);
-    const double omega_img = sqrt(cimg[0] * cimg[0] + cimg[1] * cimg[1] + cimg[2] * cimg[2]);
-    const double sgn_img = cimg[0] * d0[1] + cimg[1] * d0[2] + cimg[2] * d0[3] >= 0.0 ? 1.0 : -1.0;
 
     const DPTable& D = kDPd;
     double h = c.h0;
-    double K[7][24];
-    beam_rhs(m, Y, K[0]);
+    double k1[8], j1[8];  // f of the ray and of its tangent at the current state
+    beam_rhs(m, y, V, k1, j1);
     int outcome = SIRIUS_MAX_STEPS, steps = 0;
     const unsigned long long t0 = globaltimer();
-    double r_prev = ks_radius(m, Y);
+    double r_prev = ks_radius(m, y);
     for (int it = 0; it < 4 * c.max_steps && steps < c.max_steps; ++it) {
-        if ((it & 63) == 0 && globaltimer() - t0 > B.watchdog_ns) {
-            atomicOr(B.status, 1);
-            break;
-        }
-        // Dormand-Prince 5(4) on the 24 components (the stages' weights from the shared table)
-        double Ys[24];
-        for (int s = 1; s <= 6; ++s) {
-            for (int i = 0; i < 24; ++i) {
-                double acc = 0.0;
-                for (int j = 0; j < s; ++j) acc += D.A[j][s - 1 - j] * K[j][i];
-                Ys[i] = Y[i] + h * acc;
+        if ((it & 63) == 0) {
+            // one answer for the pair: lanes that left the loop apart could not meet again
+            const bool late = globaltimer() - t0 > B.watchdog_ns;
+            if (__any_sync(pair, late)) {
+                atomicOr(B.status, 1);
+                break;
             }
-            beam_rhs(m, Ys, K[s]);
         }
-        // Ys is the fifth-order solution (stage 7 = b weights); error on the position components
+        constexpr int C[7] = {0, 1, 2, 3, 5, 6, 7};  // p_0 and its tangent are constant
+        double k2[8], k3[8], k4[8], j2[8], j3[8], j4[8], yn[8], Vn[8], sy[7], sV[7];
+        double a6[7], b[7], A6[7], Bv[7], e[4];
+        yn[4] = y[4];
+        Vn[4] = V[4];
+        auto stage = [&](double kk[8], double jj[8]) {
+#pragma unroll
+            for (int q = 0; q < 7; ++q) {
+                yn[C[q]] = y[C[q]] + h * sy[q];
+                Vn[C[q]] = V[C[q]] + h * sV[q];
+            }
+            beam_rhs(m, yn, Vn, kk, jj);
+        };
+#pragma unroll
+        for (int q = 0; q < 7; ++q) {
+            sy[q] = D.A[0][0] * k1[C[q]];
+            sV[q] = D.A[0][0] * j1[C[q]];
+        }
+        stage(k2, j2);
+#pragma unroll
+        for (int q = 0; q < 7; ++q) {
+            sy[q] = D.A[0][1] * k1[C[q]] + D.A[1][0] * k2[C[q]];
+            sV[q] = D.A[0][1] * j1[C[q]] + D.A[1][0] * j2[C[q]];
+        }
+        stage(k3, j3);
+#pragma unroll
+        for (int q = 0; q < 7; ++q) {
+            sy[q] = D.A[0][2] * k1[C[q]] + D.A[1][1] * k2[C[q]] + D.A[2][0] * k3[C[q]];
+            sV[q] = D.A[0][2] * j1[C[q]] + D.A[1][1] * j2[C[q]] + D.A[2][0] * j3[C[q]];
+        }
+        stage(k4, j4);
+#pragma unroll
+        for (int q = 0; q < 7; ++q) {
+            const int i = C[q];
+            sy[q] = D.A[0][3] * k1[i] + D.A[1][2] * k2[i] + D.A[2][1] * k3[i] + D.A[3][0] * k4[i];
+            a6[q] = D.A[0][4] * k1[i] + D.A[1][3] * k2[i] + D.A[2][2] * k3[i] + D.A[3][1] * k4[i];
+            b[q] = D.A[0][5] * k1[i] + D.A[2][3] * k3[i] + D.A[3][2] * k4[i];
+            if (i < 4) e[i] = D.E[0] * k1[i] + D.E[2] * k3[i] + D.E[3] * k4[i];
+            sV[q] = D.A[0][3] * j1[i] + D.A[1][2] * j2[i] + D.A[2][1] * j3[i] + D.A[3][0] * j4[i];
+            A6[q] = D.A[0][4] * j1[i] + D.A[1][3] * j2[i] + D.A[2][2] * j3[i] + D.A[3][1] * j4[i];
+            Bv[q] = D.A[0][5] * j1[i] + D.A[2][3] * j3[i] + D.A[3][2] * j4[i];
+        }
+        stage(k2, j2);  // k_5
+#pragma unroll
+        for (int q = 0; q < 7; ++q) {
+            const int i = C[q];
+            sy[q] = a6[q] + D.A[4][0] * k2[i];
+            b[q] += D.A[4][1] * k2[i];
+            if (i < 4) e[i] += D.E[4] * k2[i];
+            sV[q] = A6[q] + D.A[4][0] * j2[i];
+            Bv[q] += D.A[4][1] * j2[i];
+        }
+        stage(k3, j3);  // k_6
+#pragma unroll
+        for (int q = 0; q < 7; ++q) {
+            const int i = C[q];
+            sy[q] = b[q] + D.A[5][0] * k3[i];
+            if (i < 4) e[i] += D.E[5] * k3[i];
+            sV[q] = Bv[q] + D.A[5][0] * j3[i];
+        }
+        stage(k2, j2);  // k_7 at the fifth-order solution (yn, Vn)
+        // error on the position components
         double err2 = 0.0;
+#pragma unroll
         for (int i = 0; i < 4; ++i) {
-            double e = 0.0;
-            for (int j = 0; j < 7; ++j) e += D.E[j] * K[j][i];
-            e *= h;
-            const double sc = c.atol + c.rtol * fmax(fabs(Y[i]), fabs(Ys[i]));
-            err2 += (e / sc) * (e / sc);
+            const double sc = c.atol + c.rtol * fmax(fabs(y[i]), fabs(yn[i]));
+            const double q = h * (e[i] + D.E[6] * k2[i]) * rcp_(sc);
+            err2 += q * q;
         }
         const double err = sqrt(err2 / 4.0);
         if (!(err == err)) {
@@ -173,17 +223,20 @@ __global__ void __launch_bounds__(64) beam_kernel(const __grid_constant__ BeamPa
             h = fmax(c.hmin, optimal_step(h, err, c));
             continue;
         }
-        const double z0 = Y[3];
-        for (int i = 0; i < 24; ++i) Y[i] = Ys[i];
-        for (int i = 0; i < 24; ++i) K[0][i] = K[6][i];
+        const double z0 = y[3];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            y[i] = yn[i]; V[i] = Vn[i];
+            k1[i] = k2[i]; j1[i] = j2[i];
+        }
         ++steps;
         h = optimal_step(h, err, c);
-        const double r = ks_radius(m, Y);
+        const double r = ks_radius(m, y);
         if (F.has_horizon && r < F.r_hor) {
             outcome = SIRIUS_HORIZON;
             break;
         }
-        if (c.enable_disk && z0 * Y[3] < 0.0) {
+        if (c.enable_disk && z0 * y[3] < 0.0) {
             const double rc = 0.5 * (r + r_prev);
             if (rc >= F.disk_in && rc <= F.disk_out) {
                 outcome = SIRIUS_DISK_HIT;
@@ -191,43 +244,36 @@ __global__ void __launch_bounds__(64) beam_kernel(const __grid_constant__ BeamPa
             }
         }
         r_prev = r;
-        const double R2 = Y[1] * Y[1] + Y[2] * Y[2] + Y[3] * Y[3];
-        const double out = Y[1] * K[0][1] + Y[2] * K[0][2] + Y[3] * K[0][3];
+        const double R2 = y[1] * y[1] + y[2] * y[2] + y[3] * y[3];
+        const double out = y[1] * k1[1] + y[2] * k1[2] + y[3] * k1[3];
         if (R2 > c.escape_r * c.escape_r && out > 0.0) {
             outcome = SIRIUS_ESCAPED;
             break;
         }
     }
+    __syncwarp(pair);
+    // n = k / |k| (spatial, contravariant), dn = (dk - n (n . dk)) / |k| along this lane's tangent
+    const double kn = sqrt(k1[1] * k1[1] + k1[2] * k1[2] + k1[3] * k1[3]);
+    const double n[3] = {k1[1] / kn, k1[2] / kn, k1[3] / kn};
+    const double nd = n[0] * j1[1] + n[1] * j1[2] + n[2] * j1[3];
+    double dn[3], ddo[3], dno[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        dn[i] = (j1[1 + i] - n[i] * nd) / kn;
+        ddo[i] = __shfl_xor_sync(pair, dd[i], 1);
+        dno[i] = __shfl_xor_sync(pair, dn[i], 1);
+    }
+    if (dir != 0) return;
     sirius_beam_result res{};
     res.outcome = outcome;
     res.steps = steps;
     if (outcome == SIRIUS_ESCAPED) {
-        // n = k / |k| (spatial, contravariant), dn = (dk - n (n . dk)) / |k| along each tangent
-        double k[8];
-        beam_f(m, Y, k);
-        const double kn = sqrt(k[1] * k[1] + k[2] * k[2] + k[3] * k[3]);
-        double n[3] = {k[1] / kn, k[2] / kn, k[3] / kn}, dn[2][3];
-        double ysc = 1.0;
-        for (int i = 0; i < 8; ++i) ysc = fmax(ysc, fabs(Y[i]));
-        for (int t = 0; t < 2; ++t) {
-            const double* V = Y + 8 + 8 * t;
-            double vn = 0.0;
-            for (int i = 0; i < 8; ++i) vn = fmax(vn, fabs(V[i]));
-            const double eps = vn > 0.0 ? 1e-6 * ysc / vn : 0.0;
-            double yp[8], ym[8], fp[8], fm[8];
-            for (int i = 0; i < 8; ++i) {
-                yp[i] = Y[i] + eps * V[i];
-                ym[i] = Y[i] - eps * V[i];
-            }
-            beam_f(m, yp, fp);
-            beam_f(m, ym, fm);
-            double dk[3];
-            for (int i = 0; i < 3; ++i) dk[i] = eps > 0.0 ? (fp[1 + i] - fm[1 + i]) / (2.0 * eps) : 0.0;
-            const double nd = n[0] * dk[0] + n[1] * dk[1] + n[2] * dk[2];
-            for (int i = 0; i < 3; ++i) dn[t][i] = (dk[i] - n[i] * nd) / kn;
-        }
-        double cs[3];
-        cross3(dn[0], dn[1], cs);
+        double d0[4], cimg[3], cs[3];
+        camera_dir_exact(F, u0, v0, d0);
+        cross3(dd, ddo, cimg);
+        const double omega_img = sqrt(cimg[0] * cimg[0] + cimg[1] * cimg[1] + cimg[2] * cimg[2]);
+        const double sgn_img = cimg[0] * d0[1] + cimg[1] * d0[2] + cimg[2] * d0[3] >= 0.0 ? 1.0 : -1.0;
+        cross3(dn, dno, cs);
         const double omega_src = sqrt(cs[0] * cs[0] + cs[1] * cs[1] + cs[2] * cs[2]);
         const double sgn_src = cs[0] * n[0] + cs[1] * n[1] + cs[2] * n[2] >= 0.0 ? 1.0 : -1.0;
         res.magnification = omega_src > 0.0 ? float(omega_img / omega_src) : 1e30f;

@@ -91,6 +91,60 @@ inline float tanh_(float x) { return std::tanh(x); }
 inline double tanh_(double x) { return std::tanh(x); }
 #endif
 
+// The type of a function's constants when its variables are of type T.
+template <class T>
+struct scalar_of {
+    using type = T;
+};
+
+// A value and its derivative along one direction: a function instantiated with D1
+// gives its value and its Jacobian-vector product. Constants stay plain scalars
+// (scalar_of), so nothing multiplies a zero tangent.
+template <class T>
+struct D1 {
+    T v, d;
+    D1() = default;
+    SIRIUS_HD explicit D1(T value, T tangent = T(0)) : v(value), d(tangent) {}
+};
+template <class T>
+struct scalar_of<D1<T>> {
+    using type = T;
+};
+template <class T>
+SIRIUS_HD __forceinline__ D1<T> operator+(D1<T> a, D1<T> b) { return D1<T>(a.v + b.v, a.d + b.d); }
+template <class T>
+SIRIUS_HD __forceinline__ D1<T> operator-(D1<T> a, D1<T> b) { return D1<T>(a.v - b.v, a.d - b.d); }
+template <class T>
+SIRIUS_HD __forceinline__ D1<T> operator*(D1<T> a, D1<T> b) { return D1<T>(a.v * b.v, a.d * b.v + a.v * b.d); }
+template <class T>
+SIRIUS_HD __forceinline__ D1<T> operator-(D1<T> a) { return D1<T>(-a.v, -a.d); }
+template <class T>
+SIRIUS_HD __forceinline__ D1<T> operator+(D1<T> a, T s) { return D1<T>(a.v + s, a.d); }
+template <class T>
+SIRIUS_HD __forceinline__ D1<T> operator+(T s, D1<T> a) { return a + s; }
+template <class T>
+SIRIUS_HD __forceinline__ D1<T> operator-(D1<T> a, T s) { return D1<T>(a.v - s, a.d); }
+template <class T>
+SIRIUS_HD __forceinline__ D1<T> operator-(T s, D1<T> a) { return D1<T>(s - a.v, -a.d); }
+template <class T>
+SIRIUS_HD __forceinline__ D1<T> operator*(T s, D1<T> a) { return D1<T>(s * a.v, s * a.d); }
+template <class T>
+SIRIUS_HD __forceinline__ D1<T> operator*(D1<T> a, T s) { return s * a; }
+template <class T>
+SIRIUS_HD __forceinline__ D1<T>& operator+=(D1<T>& a, D1<T> b) { a = a + b; return a; }
+template <class T>
+SIRIUS_HD __forceinline__ D1<T>& operator-=(D1<T>& a, D1<T> b) { a = a - b; return a; }
+template <class T>
+SIRIUS_HD __forceinline__ D1<T> rcp_(D1<T> a) {
+    const T y = rcp_(a.v);
+    return D1<T>(y, -y * y * a.d);
+}
+template <class T>
+SIRIUS_HD __forceinline__ D1<T> rsqrt_(D1<T> a) {
+    const T y = rsqrt_(a.v);
+    return D1<T>(y, T(-0.5) * y * y * y * a.d);
+}
+
 template <class T>
 struct D3 {
     T v;

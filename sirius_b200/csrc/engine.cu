@@ -1785,7 +1785,7 @@ int sirius_cuda_trace_beams(sirius_cuda_handle h, const sirius_frame* frames, in
     B.status = H->d_status;
     cudaError_t e = cudaMemsetAsync(H->d_status, 0, sizeof(int), H->stream);
     if (e == cudaSuccess) {
-        beam_kernel<<<int((total + 63) / 64), 64, 0, H->stream>>>(B);
+        beam_kernel<<<int((total + 31) / 32), 64, 0, H->stream>>>(B);  // two lanes per beam
         e = cudaGetLastError();
     }
     int status = 0;

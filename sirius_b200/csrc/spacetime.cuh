@@ -58,6 +58,8 @@ inline MetricDev metric_dev(const sirius_metric& s) {
 
 template <class T>
 SIRIUS_HD __forceinline__ T tmax(T a, T b) { return a > b ? a : b; }
+template <class T>
+SIRIUS_HD __forceinline__ D1<T> tmax(D1<T> a, T b) { return a.v > b ? a : D1<T>(b); }
 
 // ---------------------------------------------------------------------------
 // Kerr-Schild family (PHMT100A.h:198-396): H and l_i as dual numbers.
@@ -224,31 +226,33 @@ struct KSGeom {
 
 template <class T>
 SIRIUS_HD __forceinline__ void ks_geom(const MetricDev& m, T X, T Y, T Z, KSGeom<T>& G) {
-    const T a = cst<T>(m.a, m.fa), a2 = cst<T>(m.a2, m.fa2), M2 = cst<T>(2.0 * m.M, m.fM2);
+    using C = typename scalar_of<T>::type;
+    const C a = cst<C>(m.a, m.fa), a2 = cst<C>(m.a2, m.fa2), M2 = cst<C>(2.0 * m.M, m.fM2);
     const T zz = Z * Z;
     const T R2 = X * X + Y * Y + zz;
     const T Rm2 = R2 - a2;
-    const T disc = tmax(Rm2 * Rm2 + T(4) * a2 * zz, T(1e-20));
+    const T disc = tmax(Rm2 * Rm2 + C(4) * a2 * zz, C(1e-20));
     const T isd = rsqrt_(disc);
-    const T r2 = tmax((Rm2 + disc * isd) * T(0.5), T(1e-10));
+    const T r2 = tmax((Rm2 + disc * isd) * C(0.5), C(1e-10));
     const T ir = rsqrt_(r2);
     const T r = r2 * ir;
     const T den = r2 + a2;
     const T iden = rcp_(den);
-    const T q = M2 * r - cst<T>(m.Q2, m.fQ2);
+    const T q = M2 * r - cst<C>(m.Q2, m.fQ2);
     G.X = X; G.Y = Y; G.Z = Z; G.r = r; G.ir = ir; G.isd = isd; G.iden = iden; G.den = den;
     G.l1 = (r * X + a * Y) * iden;
     G.l2 = (r * Y - a * X) * iden;
     G.l3 = Z * ir;
     G.H = q * isd;
-    G.w = (M2 + T(2) * q * ir - T(4) * G.H * r) * isd;
+    G.w = (M2 + C(2) * q * ir - C(4) * G.H * r) * isd;
     G.hz = a2 * G.l3 * isd;
-    G.c = m.has_lambda ? cst<T>(m.lam3, m.flam3) * R2 : T(0);
+    G.c = m.has_lambda ? cst<C>(m.lam3, m.flam3) * R2 : T(0);
 }
 
 // k = g^{-1} p = eta p - H l# (l# . p), l# = (-1, l1, l2, l3); lk = l . k
 template <class T>
 SIRIUS_HD __forceinline__ void ks_velocity(const MetricDev& m, const KSGeom<T>& G, const T p[4], T k[4], T& lk) {
+    using C = typename scalar_of<T>::type;
     const T lp = -p[0] + G.l1 * p[1] + G.l2 * p[2] + G.l3 * p[3];
     const T Hlp = G.H * lp;
     k[0] = -p[0] + Hlp;
@@ -257,8 +261,8 @@ SIRIUS_HD __forceinline__ void ks_velocity(const MetricDev& m, const KSGeom<T>& 
     k[3] = p[3] - G.l3 * Hlp;
     lk = lp;
     if (m.has_lambda) {
-        const T w0 = -T(1) - G.H, w1 = G.H * G.l1, w2 = G.H * G.l2, w3 = G.H * G.l3;
-        const T s = G.c * (w0 * p[0] + w1 * p[1] + w2 * p[2] + w3 * p[3]) * rcp_(T(1) + G.c * (T(1) + G.H));
+        const T w0 = -C(1) - G.H, w1 = G.H * G.l1, w2 = G.H * G.l2, w3 = G.H * G.l3;
+        const T s = G.c * (w0 * p[0] + w1 * p[1] + w2 * p[2] + w3 * p[3]) * rcp_(C(1) + G.c * (C(1) + G.H));
         k[0] += s * w0; k[1] += s * w1; k[2] += s * w2; k[3] += s * w3;
         lk = k[0] + G.l1 * k[1] + G.l2 * k[2] + G.l3 * k[3];
     }
@@ -267,17 +271,18 @@ SIRIUS_HD __forceinline__ void ks_velocity(const MetricDev& m, const KSGeom<T>& 
 // f_i = dp_i / dl, i = 1..3 (f_0 = 0: the metric is static), from the velocity
 template <class T>
 SIRIUS_HD __forceinline__ void ks_force(const MetricDev& m, const KSGeom<T>& G, const T k[4], T lk, T f[4]) {
-    const T a = cst<T>(m.a, m.fa);
-    const T S = (G.X * k[1] + G.Y * k[2] - T(2) * G.r * (G.l1 * k[1] + G.l2 * k[2])) * G.iden - k[3] * G.l3 * G.ir;
+    using C = typename scalar_of<T>::type;
+    const C a = cst<C>(m.a, m.fa);
+    const T S = (G.X * k[1] + G.Y * k[2] - C(2) * G.r * (G.l1 * k[1] + G.l2 * k[2])) * G.iden - k[3] * G.l3 * G.ir;
     const T Hlk = G.H * lk, e = Hlk * G.iden;
-    const T g = lk * (T(0.5) * G.w * lk + G.H * S) * G.isd;
+    const T g = lk * (C(0.5) * G.w * lk + G.H * S) * G.isd;
     const T gr = g * G.r;
     f[0] = T(0);
     f[1] = gr * G.X + e * (G.r * k[1] - a * k[2]);
     f[2] = gr * G.Y + e * (a * k[1] + G.r * k[2]);
     f[3] = G.ir * (g * G.den * G.Z + Hlk * (k[3] - G.hz * lk));
     if (m.has_lambda) {  // - Lambda x_i (k^0)^2 / 3
-        const T qq = cst<T>(m.lam3, m.flam3) * k[0] * k[0];
+        const T qq = cst<C>(m.lam3, m.flam3) * k[0] * k[0];
         f[1] -= qq * G.X; f[2] -= qq * G.Y; f[3] -= qq * G.Z;
     }
 }
