@@ -2033,8 +2033,8 @@ int sirius_cuda_surrogate_load(sirius_cuda_handle h, const float* params, int64_
         // [0] error, [2..3] MLP tile counter, [8..12] the audit's sums and maxima
         if (cudaMalloc((void**)&H->d_sur_err, 16 * sizeof(int)) != cudaSuccess)
             return fail(H, SIRIUS_ERR_OUT_OF_MEMORY, "cudaMalloc surrogate status");
-        CK(cudaFuncSetAttribute(surrogate::mlp_kernel_ts, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                surrogate::kTsSmBytes));
+        CK(cudaFuncSetAttribute(surrogate::mlp_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                surrogate::kPairSmBytes));
     }
     CK(cudaMemcpyAsync(H->d_surrogate, img.data(), surrogate::kImageBytes, cudaMemcpyHostToDevice, H->stream));
     CK(cudaStreamSynchronize(H->stream));
@@ -2046,13 +2046,13 @@ static int surrogate_launch(Handle* H, const float* d_features, long long n, flo
                             const unsigned* rows = nullptr) {
     if (!H->d_surrogate) return fail(H, SIRIUS_ERR_NOT_CONFIGURED, "no surrogate weights loaded");
     if (n <= 0) return SIRIUS_OK;
-    const long long tiles = (n + surrogate::kTileM - 1) / surrogate::kTileM;
-    const int grid = int(std::min<long long>(tiles, H->num_sms));
+    const long long tiles = (n + 2 * surrogate::kTileM - 1) / (2 * surrogate::kTileM);
+    const int grid = 2 * int(std::min<long long>(tiles, std::max(H->num_sms / 2, 1)));  // a pair of CTAs per tile
     // bound on any wait inside the kernel: the configured watchdog (default 30 s)
     const unsigned long long limit = (unsigned long long)(H->cfg.watchdog_ms > 0 ? H->cfg.watchdog_ms : 30000) * 1000000ull;
     unsigned long long* counter = reinterpret_cast<unsigned long long*>(H->d_sur_err + 2);
     CK(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st));
-    surrogate::mlp_kernel_ts<<<grid, surrogate::kThreads, surrogate::kTsSmBytes, st>>>(
+    surrogate::mlp_pair_kernel<<<grid, surrogate::kPairThreads, surrogate::kPairSmBytes, st>>>(
         H->d_surrogate, d_features, n, d_out, H->d_sur_err, counter, limit, rows);
     CK(cudaGetLastError());
     return SIRIUS_OK;

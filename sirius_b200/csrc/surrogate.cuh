@@ -2,32 +2,31 @@
 //
 // Network (the surrogate configuration): 5 -> 256 -> 256 -> 256 -> 256 -> 4,
 // SiLU after each hidden layer, BF16 weights and activations, FP32
-// accumulation, FP32 biases. One CTA of 256 threads owns one SM and walks
-// 128-row tiles of the input:
+// accumulation, FP32 biases. A pair of CTAs (a cluster of two, one per SM)
+// walks 256-row tiles of the input, 128 rows each:
 //
+//   * tcgen05.mma.cta_group::2 (M = 256, N = 256 or 16, K = 16): each CTA holds
+//     its own rows of A and D and half of the weights' N rows, so all the
+//     network's weights stay in shared memory (208 KB per SM) for the whole
+//     launch, and nothing is streamed per tile.
 //   * B operands (weights, N x K) sit in shared memory, K-major, in the
 //     no-swizzle core-matrix layout of the UMMA shared-memory descriptor:
 //     element (row, k) at byte (row % 8) * 16 + (row / 8) * SBO + (k / 8) * 128
 //     + (k % 8) * 2, SBO = (K / 8) * 128.
-//   * The FP32 accumulator and the BF16 activations (the A operand of layers
-//     2-5) live in tensor memory; layer 1 reads its 16-wide padded input from
-//     shared memory: each feature as two BF16 terms (hi, lo) against W1
-//     repeated in two column groups, so the inputs keep 16 significant bits
-//     (pack_input_row). One thread issues tcgen05.mma (M = 128, N = 128 or 16,
-//     K = 16 per instruction) and commits each N-half to its own mbarrier.
-//   * The 128 KB weight images of layers 2-4 stream from global memory by a
-//     bulk TMA copy (cp.async.bulk, no tensor map, no multicast) into one
-//     buffer, each issued as soon as the previous layer's MMAs have drained it,
-//     so the copy overlaps the epilogue. Layer 1 (K 2 x 5 padded to 16) and layer 5
-//     (N padded 4 -> 16) weights and all biases stay resident.
+//   * Layer 1 reads its 16-wide padded input from shared memory: each feature as
+//     two BF16 terms (hi, lo) against W1 repeated in two column groups, so the
+//     inputs keep 16 significant bits (pack_input_row). The other layers read
+//     their activations from tensor memory, where the epilogue left them in
+//     place of the accumulator columns they came from.
 //   * Epilogue: 8 warps read the accumulator with tcgen05.ld, add the bias,
 //     apply SiLU x (1 + tanh(x / 2)) / 2 (one MUFU op), round to BF16 and write
-//     the next layer's A operand with tcgen05.st; half 0 of a layer converts
-//     while the tensor core still works on half 1.
+//     the next layer's A operand with tcgen05.st, 64 columns at a time. The MMAs
+//     of the next layer take each 64 columns of K as soon as both CTAs have
+//     written them, so tensor core and epilogue work at the same time.
 //
-// Every mbarrier wait is bounded by the device clock; on a timeout the block
-// agrees (a block-wide vote) to stop, records an error flag, waits (bounded)
-// for its copy in flight and frees its TMEM.
+// Every mbarrier wait is bounded by the device clock; a role whose wait runs out
+// records an error flag and leaves its loop, the others run out after it, and the
+// CTAs meet (and free their TMEM) at the end in any case.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -38,7 +37,7 @@
 namespace sirius {
 namespace surrogate {
 
-constexpr int kIn = 5, kInPad = 16, kHid = 256, kOut = 4, kOutPad = 16, kTileM = 128, kThreads = 256;
+constexpr int kIn = 5, kInPad = 16, kHid = 256, kOut = 4, kOutPad = 16, kTileM = 128;
 // packed weight image (bytes): W2 | W3 | W4 | W1 | W5 | b1 b2 b3 b4 (256 f32 each) | b5 (16 f32)
 constexpr int kBigBytes = kHid * kHid * 2;            // 131072
 constexpr int kW1Bytes = kHid * kInPad * 2;           // 8192
@@ -53,241 +52,316 @@ using namespace ::sirius::tc;
 
 #ifdef __CUDACC__
 // ---------------------------------------------------------------------------
-// The MLP kernel, with its activations in tensor memory.
+// The MLP kernel.
 //
-// TMEM (512 columns, one CTA per SM): columns [0, 256) the FP32 accumulator,
-// [256, 384) and [384, 512) two BF16 activation buffers (row m in lane m,
-// element k in column k / 2, even k in the low half), used in turn as the A
-// operand of tcgen05.mma (the form that reads A from tensor memory) and as the
-// epilogue's destination. Each layer's MMAs run as two N-halves committed to
-// separate mbarriers, so the epilogue of half 0 (TMEM -> bias -> SiLU -> BF16
-// -> tcgen05.st) overlaps the tensor core's work on half 1. Layer 1 reads its
-// 16-wide (padded) input from shared memory.
+// What bounds it: per 128 rows and hidden layer an SM needs 2048 cycles of tensor
+// core (8.4 M multiply-adds) and 2048 of MUFU (32768 tanh at 16 a cycle). A layer's
+// MMAs may start on K columns 0..63 when the epilogue of the layer before has done a
+// quarter, so the two overlap but for the last quarter's MMAs (512 cycles) and the
+// hand-offs between the CTAs (about 200 cycles to the issuer, 350 back): a layer takes
+// about 3600 cycles. 2^22 rows: 2.91 -> 1.79 ms (573 -> 930 TFLOP/s, 57 % of the
+// measured bf16 peak; MUFU 55 % and tensor pipe 43 % active) against one CTA per tile
+// with a 128 KB weight buffer refilled per layer, where the two took turns; outputs
+// bit for bit the same. Eight epilogue warps instead of sixteen take 1 % more; MMAs of
+// N = 128, which let the first half's epilogue start earlier, 22 % more (they run at
+// half the rate of N = 256 with A in tensor memory).
+//
+// TMEM (512 columns): two halves U and V of 256. Layer 1 accumulates in U, layer 2 in
+// V, layer 3 in U, layer 4 in V, layer 5 (16 columns) in U; the next tile starts with
+// the halves exchanged. Epilogue warp w owns lanes 32 (w % 4).. and, of each 64
+// columns, the 16 at 16 (w / 4): it writes their 16 BF16 activations, one K step of the
+// next layer, into the first 8 of those same columns, so no warp overwrites what
+// another has yet to read.
+//
+// Roles: warps 0..15 epilogue (the first 8 also the input rows); warp 16 copies the
+// CTA's weights in and, in the even CTA, one of its threads issues every MMA of the
+// pair; in the even CTA a thread of warp 17 takes tiles from a counter (a cluster that
+// starts late, its SMs still busy with another kernel, takes fewer).
 // ---------------------------------------------------------------------------
-constexpr int kTsSmWbuf = 0, kTsSmW1 = kBigBytes, kTsSmW5 = kTsSmW1 + kW1Bytes, kTsSmX = kTsSmW5 + kW5Bytes,
-              kTsSmBias = kTsSmX + kTileM * kInPad * 2, kTsSmBar = kTsSmBias + kBiasBytes,
-              kTsSmTmemSlot = kTsSmBar + 32, kTsSmBytes = kTsSmTmemSlot + 16;
-static_assert(kTsSmBytes <= 227 * 1024, "the MLP kernel's shared memory fits one SM");
-static_assert(kTsSmBar % 8 == 0, "mbarriers are 8-byte aligned");
-constexpr uint32_t kTmemAcc = 0, kTmemA0 = 256, kTmemA1 = 384, kTmemCols = 512;
+constexpr int kEpiWarps = 16, kPairThreads = 32 * (kEpiWarps + 2);
+constexpr int kSmW = 0, kSmW1 = 3 * (kBigBytes / 2), kSmW5 = kSmW1 + kW1Bytes / 2, kSmX = kSmW5 + kW5Bytes / 2,
+              kSmBias = kSmX + kTileM * kInPad * 2, kSmTile = kSmBias + kBiasBytes, kSmBar = kSmTile + 16;
+enum PairBar : int {  // mbarriers, 8 bytes each from kSmBar
+    kBarW = 0,          // [4] this CTA's weights have landed: W1 and W5, W2, W3, W4
+    kBarWReady = 4,     // [4] even CTA: the other CTA's have
+    kBarX = 8,          // even CTA: both CTAs' input rows are in shared memory
+    kBarA = 9,          // [4] even CTA: 64 columns of activations are in both CTAs' TMEM
+    kBarD = 13,         // a hidden layer's accumulator is complete
+    kBarOut = 14,       // the output layer's is
+    kBarTile = 15,      // the next tile's index is in shared memory
+    kBarFirst = 16,     // even CTA: a tile's first layer is complete
+    kBarCount = 17
+};
+constexpr int kSmSlot = kSmBar + 8 * (kBarCount + 1), kPairSmBytes = kSmSlot + 16;
+static_assert(kPairSmBytes <= 227 * 1024, "the MLP kernel's shared memory fits one SM");
+static_assert(kSmTile % 16 == 0, "the tile index and the mbarriers are aligned");
+constexpr uint32_t kTmemCols = 512;
 
-// Epilogue of accumulator half H (columns 128 H ..): bias + SiLU -> BF16 pairs
-// into the activation buffer at TMEM column a_next. Warp w: lanes 32 (w % 4)..,
-// columns 128 H + 64 (w / 4)...
-__device__ __forceinline__ void epilogue_half_ts(uint32_t tmem, int H, const float* bias, uint32_t a_next) {
-    const int warp = threadIdx.x >> 5;
-    const uint32_t lanes = uint32_t((warp & 3) * 32) << 16;
-    // both 32-column loads in flight before one wait
-    const int col0 = 128 * H + 64 * (warp >> 2);
-    float v[64];
-    tmem_ld32_nowait(tmem + kTmemAcc + lanes + uint32_t(col0), v);
-    tmem_ld32_nowait(tmem + kTmemAcc + lanes + uint32_t(col0 + 32), v + 32);
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-        uint32_t r[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-            r[i] = pack_bf16x2(silu(v[32 * c + 2 * i] + bias[col0 + 32 * c + 2 * i]),
-                               silu(v[32 * c + 2 * i + 1] + bias[col0 + 32 * c + 2 * i + 1]));
-        tmem_st16(tmem + a_next + lanes + uint32_t((col0 + 32 * c) / 2), r);
-    }
-}
+// the TMEM column, within its half, of K step s (16 elements) of the activations
+__device__ __forceinline__ uint32_t act_column(int s) { return uint32_t(16 * s); }
 
-__global__ void __launch_bounds__(kThreads, 1)
-    mlp_kernel_ts(const unsigned char* __restrict__ wimg, const float* __restrict__ feat, long long n,
-                  float* __restrict__ out, int* err, unsigned long long* tile_counter,
-                  unsigned long long wait_limit_ns, const unsigned* __restrict__ rows) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+    mlp_pair_kernel(const unsigned char* __restrict__ wimg, const float* __restrict__ feat, long long n,
+                    float* __restrict__ out, int* err, unsigned long long* tile_counter,
+                    unsigned long long wait_limit_ns, const unsigned* __restrict__ rows) {
     extern __shared__ __align__(1024) unsigned char sm[];
-    unsigned char* Wbuf = sm + kTsSmWbuf;
-    unsigned char* W1s = sm + kTsSmW1;
-    unsigned char* W5s = sm + kTsSmW5;
-    unsigned char* Xs = sm + kTsSmX;
-    float* bias = reinterpret_cast<float*>(sm + kTsSmBias);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + kTsSmTmemSlot);
-    long long* next_s = reinterpret_cast<long long*>(sm + kTsSmTmemSlot + 8);  // the next tile to take
-    const uint32_t bar_a = smem_u32(sm + kTsSmBar), bar_b = smem_u32(sm + kTsSmBar + 8),
-                   bar_tma = smem_u32(sm + kTsSmBar + 16);
+    float* bias = reinterpret_cast<float*>(sm + kSmBias);
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + kSmSlot);
+    volatile unsigned long long* tile_s = reinterpret_cast<volatile unsigned long long*>(sm + kSmTile);
+    const uint32_t sm0 = smem_u32(sm), bar0 = sm0 + kSmBar;
+    auto bar = [&](int b) { return bar0 + 8u * uint32_t(b); };
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const long long ntiles = (n + kTileM - 1) / kTileM;
+    const uint32_t rank = cluster_rank();
+    const long long ntiles = (n + 2 * kTileM - 1) / (2 * kTileM);
 
     if (tid == 0) {
-        mbar_init(bar_a, 1);
-        mbar_init(bar_b, 1);
-        mbar_init(bar_tma, 1);
+        for (int i = 0; i < 4; ++i) {
+            mbar_init(bar(kBarW + i), 1);
+            mbar_init(bar(kBarWReady + i), 1);
+            mbar_init(bar(kBarA + i), 2 * kEpiWarps);
+        }
+        mbar_init(bar(kBarX), 16);
+        mbar_init(bar(kBarD), 1);
+        mbar_init(bar(kBarOut), 1);
+        mbar_init(bar(kBarTile), 1);
+        mbar_init(bar(kBarFirst), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
+    if (warp == kEpiWarps) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
                      "r"(kTmemCols));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
     }
-    // tiles come from a counter, so a CTA that starts late (its SM still busy
-    // with another kernel's blocks) takes fewer of them
-    if (tid == 32) *next_s = (long long)atomicAdd(tile_counter, 1ull);
-    {  // resident operands: W1 | W5 (contiguous in the image and in shared memory) and the biases
-        const uint4* src1 = reinterpret_cast<const uint4*>(wimg + kOffW1);
-        uint4* dst1 = reinterpret_cast<uint4*>(W1s);
-        for (int i = tid; i < (kW1Bytes + kW5Bytes) / 16; i += kThreads) dst1[i] = src1[i];
-        const float4* srcb = reinterpret_cast<const float4*>(wimg + kOffBias);
-        float4* dstb = reinterpret_cast<float4*>(bias);
-        for (int i = tid; i < kBiasBytes / 16; i += kThreads) dstb[i] = srcb[i];
-    }
-    fence_async_smem();
+    for (int i = tid; i < kBiasBytes / 16; i += kPairThreads)
+        reinterpret_cast<float4*>(bias)[i] = reinterpret_cast<const float4*>(wimg + kOffBias)[i];
     tc_fence_before();
     __syncthreads();
+    cluster_sync();  // both CTAs' barriers and TMEM are set up
     tc_fence_after();
     const uint32_t tmem = *tslot;
+    bool ok = true;
 
-    uint32_t ph_a = 0, ph_b = 0, ph_tma = 0;
-    bool tma_pending = false, ok = true;
-    long long tile = *next_s;
-    // this thread's input row (tid / 2) of the tile to come, gathered a tile ahead
-    // so that the gather's latency (row index, then the row) overlaps the current
-    // tile's layers; rows past n read as zeros, which pack to zero operands
-    const int in_r = tid >> 1, in_chunk = tid & 1;
-    float xin[kIn];
-    auto fetch_row = [&](long long t) {
-        const long long gr = t * kTileM + in_r;
-        const bool live = t < ntiles && gr < n;
-        const float* f = feat + (live ? (rows ? (long long)rows[gr] : gr) : 0LL) * kIn;
+    if (warp == kEpiWarps) {
+        if (lane == 0) {
+            // this CTA's half of the weights: each layer's N rows 128 rank.. (8 rank.. of W5's 16)
+            auto copy = [&](int dst, size_t src, uint32_t bytes, int b) {
+                asm volatile(
+                    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sm0 + dst),
+                    "l"(wimg + src + size_t(rank) * bytes), "r"(bytes), "r"(bar(b))
+                    : "memory");
+            };
+            mbar_expect_tx(bar(kBarW), kW1Bytes / 2 + kW5Bytes / 2);
+            copy(kSmW1, kOffW1, kW1Bytes / 2, kBarW);
+            copy(kSmW5, kOffW5, kW5Bytes / 2, kBarW);
+            for (int l = 0; l < 3; ++l) {
+                mbar_expect_tx(bar(kBarW + 1 + l), kBigBytes / 2);
+                copy(kSmW + l * (kBigBytes / 2), size_t(l) * kBigBytes, kBigBytes / 2, kBarW + 1 + l);
+            }
+            if (rank == 1)
+                for (int i = 0; i < 4; ++i) {
+                    ok = mbar_wait(bar(kBarW + i), 0, wait_limit_ns) && ok;
+                    mbar_arrive_cluster(peer_addr(bar(kBarWReady + i), 0));
+                }
+            if (rank == 0) {
+                const uint32_t id256 = instr_desc_pair(kHid), id16 = instr_desc_pair(kOutPad);
+                const uint32_t sbo1 = (kInPad / 8) * 128, sbo = (kHid / 8) * 128;
+                uint32_t ph_x = 0, ph_a = 0, ph_out = 0, ph_tile = 0;
+                auto operand = [&](int c) {  // 64 columns of the operand are there
+                    ok = mbar_wait_cluster(bar(kBarA + c), ph_a, wait_limit_ns);
+                    tc_fence_after();
+                    return ok;
+                };
+                int n_w = 0;  // weight groups known to be in both CTAs' shared memory
+                auto weights = [&](int i) {
+                    for (; ok && n_w <= i; ++n_w)
+                        ok = mbar_wait(bar(kBarW + n_w), 0, wait_limit_ns) &&
+                             mbar_wait_cluster(bar(kBarWReady + n_w), 0, wait_limit_ns);
+                    return ok;
+                };
+                auto more = [&]() {  // whether there is another tile
+                    ok = ok && mbar_wait_cluster(bar(kBarTile), ph_tile, wait_limit_ns);
+                    ph_tile ^= 1;
+                    return ok && (long long)*tile_s < ntiles;
+                };
+                uint32_t U = tmem, V = tmem + 256;
+                while (more()) {
+                    if (!weights(0) || !(ok = mbar_wait_cluster(bar(kBarX), ph_x, wait_limit_ns))) break;
+                    ph_x ^= 1;
+                    tc_fence_after();
+                    mma_bf16_pair(U, smem_desc(sm0 + kSmX, sbo1), smem_desc(sm0 + kSmW1, sbo1), id256, 0u);
+                    mma_commit_pair(bar(kBarD));
+                    mma_commit_pair_own(bar(kBarFirst));
+                    uint32_t A = U, D = V;
+                    for (int l = 0; l < 3; ++l) {  // layers 2, 3, 4
+                        if (!weights(1 + l)) break;
+                        const uint32_t wl = sm0 + kSmW + uint32_t(l) * (kBigBytes / 2);
+                        for (int c = 0; c < 4; ++c) {
+                            if (!operand(c)) break;
 #pragma unroll
-        for (int k = 0; k < kIn; ++k) xin[k] = live ? f[k] : 0.f;
-    };
-    fetch_row(tile);
-    if (tid == 0 && tile < ntiles) bulk_load(smem_u32(Wbuf), wimg, kBigBytes, bar_tma);
-    tma_pending = tile < ntiles;
-    const uint32_t idesc128 = instr_desc(128), idesc16 = instr_desc(kOutPad);
-
-    while (tile < ntiles) {
-        const long long row0 = tile * kTileM;
-        __syncthreads();  // every thread has read *next_s
-        if (tid == 32) *next_s = (long long)atomicAdd(tile_counter, 1ull);
-        {  // input tile: 128 rows x 16 BF16 (features 0..4 as two BF16 terms, zero padding)
+                            for (int s = 4 * c; s < 4 * c + 4; ++s)
+                                mma_bf16_ts_pair(D, A + act_column(s), smem_desc(wl + s * 256, sbo), id256, s > 0);
+                        }
+                        if (!ok) break;
+                        ph_a ^= 1;
+                        mma_commit_pair(bar(kBarD));
+                        const uint32_t t = A;
+                        A = D;
+                        D = t;
+                    }
+                    for (int c = 0; ok && c < 4; ++c) {  // the output layer
+                        if (!operand(c)) break;
+#pragma unroll
+                        for (int s = 4 * c; s < 4 * c + 4; ++s)
+                            mma_bf16_ts_pair(D, A + act_column(s), smem_desc(sm0 + kSmW5 + s * 256, sbo), id16, s > 0);
+                    }
+                    if (!ok) break;
+                    ph_a ^= 1;
+                    mma_commit_pair(bar(kBarOut));
+                    // the next tile's first layer overwrites the operand of the output layer
+                    if (!(ok = mbar_wait(bar(kBarOut), ph_out, wait_limit_ns))) break;
+                    ph_out ^= 1;
+                    const uint32_t t = U;
+                    U = V;
+                    V = t;
+                }
+                if (!ok) {  // whatever was issued drains before the end, and no copy lands after it
+                    mma_commit_pair(bar(kBarOut));
+                    mbar_wait(bar(kBarOut), ph_out, wait_limit_ns);
+                }
+                for (; n_w < 4; ++n_w) ok = mbar_wait(bar(kBarW + n_w), 0, wait_limit_ns) && ok;
+            }
+            if (!ok) atomicOr(err, 1);
+        }
+        __syncwarp();
+    } else if (warp == kEpiWarps + 1) {
+        if (rank == 0 && lane == 0) {
+            auto next_tile = [&]() {  // taken from the counter and told to both CTAs
+                const unsigned long long t = atomicAdd(tile_counter, 1ull);
+#pragma unroll
+                for (uint32_t r = 0; r < 2; ++r) {
+                    st_cluster_u64(peer_addr(sm0 + kSmTile, r), t);
+                    mbar_arrive_cluster(peer_addr(bar(kBarTile), r));
+                }
+                return (long long)t;
+            };
+            // the next one once a tile's first layer is complete: every thread has then read
+            // the tile's index, and none asks for the next before it has been told
+            for (uint32_t ph = 0; ok && next_tile() < ntiles; ph ^= 1) ok = mbar_wait(bar(kBarFirst), ph, wait_limit_ns);
+            if (!ok) atomicOr(err, 1);
+        }
+        __syncwarp();
+    } else {
+        const uint32_t lanes = uint32_t((warp & 3) * 32) << 16;
+        const int group = warp >> 2;
+        const int in_r = tid >> 1, in_chunk = tid & 1;
+        float xin[kIn];
+        // this thread's input row (tid / 2) of a tile; rows past n read as zeros, which
+        // pack to zero operands
+        auto fetch_row = [&](long long t) {
+            const long long gr = t * (2 * kTileM) + long(rank) * kTileM + in_r;
+            const bool live = gr < n && in_r < kTileM;
+            const float* f = feat + (live ? (rows ? (long long)rows[gr] : gr) : 0LL) * kIn;
+#pragma unroll
+            for (int k = 0; k < kIn; ++k) xin[k] = live ? f[k] : 0.f;
+        };
+        const uint32_t bar_x = peer_addr(bar(kBarX), 0);
+        auto store_row = [&]() {
+            if (in_r >= kTileM) return;  // (whole warps)
             uint4 c0, c1;
             pack_input_row(xin, c0, c1);
-            *reinterpret_cast<uint4*>(Xs + packed_offset(in_r, in_chunk * 8, kInPad)) = in_chunk == 0 ? c0 : c1;
+            *reinterpret_cast<uint4*>(sm + kSmX + packed_offset(in_r, in_chunk * 8, kInPad)) = in_chunk == 0 ? c0 : c1;
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster_relaxed(bar_x);
+        };
+        auto all = [&](bool v) { return __all_sync(0xffffffffu, v) != 0; };
+        uint32_t ph_tile = 0, ph_d = 0, ph_out = 0;
+        uint32_t bar_a[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) bar_a[c] = peer_addr(bar(kBarA + c), 0);
+        auto get_tile = [&](long long& t) {
+            const bool got = all(mbar_wait_cluster(bar(kBarTile), ph_tile, wait_limit_ns));
+            ph_tile ^= 1;
+            t = (long long)*tile_s;
+            return got;
+        };
+        long long tile = 0;
+        ok = get_tile(tile);
+        if (ok && tile < ntiles) {
+            fetch_row(tile);
+            store_row();
         }
-        fence_async_smem();
-        __syncthreads();
-        const long long next = *next_s;
-        fetch_row(next);  // in flight during this tile's layers
-        // layer 1 (A from shared memory, K = 16): two N-halves
-        if (tid == 0) {
-            tc_fence_after();
-            const uint32_t sbo = (kInPad / 8) * 128;
-            mma_bf16(tmem + kTmemAcc, smem_desc(smem_u32(Xs), sbo), smem_desc(smem_u32(W1s), sbo), idesc128, 0u);
-            mma_commit(bar_a);
-            mma_bf16(tmem + kTmemAcc + 128, smem_desc(smem_u32(Xs), sbo), smem_desc(smem_u32(W1s) + 16 * sbo, sbo),
-                     idesc128, 0u);
-            mma_commit(bar_b);
-        }
-        uint32_t a_cur = kTmemA0, a_nxt = kTmemA1;
-        // epilogue of layer 1 into a_cur
-        ok = mbar_wait(bar_a, ph_a, wait_limit_ns);
-        ph_a ^= 1;
-        ok = __syncthreads_and(ok);
-        if (!ok) break;
-        tc_fence_after();
-        epilogue_half_ts(tmem, 0, bias, a_cur);
-        ok = mbar_wait(bar_b, ph_b, wait_limit_ns);
-        ph_b ^= 1;
-        ok = __syncthreads_and(ok);
-        if (!ok) break;
-        tc_fence_after();
-        epilogue_half_ts(tmem, 1, bias, a_cur);
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        tc_fence_before();
-        __syncthreads();
-        // layers 2..4 (A from tensor memory, K = 256): weights streamed into Wbuf
-        for (int L = 0; L < 3 && ok; ++L) {
-            ok = mbar_wait(bar_tma, ph_tma, wait_limit_ns);
-            ok = __syncthreads_and(ok);
-            if (!ok) break;
-            ph_tma ^= 1;
-            tma_pending = false;
-            if (tid == 0) {
+        uint32_t U = tmem, V = tmem + 256;
+        while (ok && tile < ntiles) {
+            long long next = ntiles;
+            uint32_t src = U;
+#pragma unroll 1
+            for (int l = 0; l < 4; ++l) {
+                if (!(ok = all(mbar_wait(bar(kBarD), ph_d, wait_limit_ns)))) break;
+                ph_d ^= 1;
                 tc_fence_after();
-                const uint32_t sbo = (kHid / 8) * 128;
-#pragma unroll 1
-                for (int hh = 0; hh < 2; ++hh) {
-#pragma unroll 1
-                    for (int s = 0; s < kHid / 16; ++s)
-                        mma_bf16_ts(tmem + kTmemAcc + 128 * hh, tmem + a_cur + 8 * s,
-                                    smem_desc(smem_u32(Wbuf) + hh * (kBigBytes / 2) + s * 256, sbo), idesc128,
-                                    s > 0);
-                    mma_commit(hh == 0 ? bar_a : bar_b);
+                const uint32_t col = src + lanes + uint32_t(16 * group);
+                const float4* b4 = reinterpret_cast<const float4*>(bias + l * kHid + 16 * group);
+                uint32_t v[2][16];
+                tmem_ld16_async(col, v[0]);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    tmem_wait_ld16(v[c & 1]);
+                    if (c < 3) tmem_ld16_async(col + 64 * (c + 1), v[(c + 1) & 1]);
+                    uint32_t r[8];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float4 b = b4[16 * c + i];
+                        const uint32_t* q = v[c & 1] + 4 * i;
+                        const float2 y0 = silu_bias2(make_float2(__uint_as_float(q[0]), __uint_as_float(q[1])),
+                                                     make_float2(b.x, b.y));
+                        const float2 y1 = silu_bias2(make_float2(__uint_as_float(q[2]), __uint_as_float(q[3])),
+                                                     make_float2(b.z, b.w));
+                        r[2 * i] = pack_bf16x2(y0.x, y0.y);
+                        r[2 * i + 1] = pack_bf16x2(y1.x, y1.y);
+                    }
+                    tmem_st8(col + 64 * c, r);
+                    tmem_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster_relaxed(bar_a[c]);
+                }
+                src = src == U ? V : U;
+                if (l == 1) {  // the next tile's rows: on their way during layer 3
+                    if (!(ok = get_tile(next))) break;
+                    if (next < ntiles) fetch_row(next);
+                } else if (l == 2 && next < ntiles) {
+                    store_row();
                 }
             }
-            const float* b = bias + (L + 1) * kHid;
-            ok = mbar_wait(bar_a, ph_a, wait_limit_ns);
-            ph_a ^= 1;
-            ok = __syncthreads_and(ok);
             if (!ok) break;
+            if (!(ok = all(mbar_wait(bar(kBarOut), ph_out, wait_limit_ns)))) break;
+            ph_out ^= 1;
             tc_fence_after();
-            epilogue_half_ts(tmem, 0, b, a_nxt);
-            ok = mbar_wait(bar_b, ph_b, wait_limit_ns);
-            ph_b ^= 1;
-            ok = __syncthreads_and(ok);
-            if (!ok) break;
-            // Wbuf is drained: bring the next layer's weights (or layer 2's for the next tile)
-            if (L < 2 || next < ntiles) {
-                if (tid == 0) bulk_load(smem_u32(Wbuf), wimg + size_t(L < 2 ? L + 1 : 0) * kBigBytes, kBigBytes, bar_tma);
-                tma_pending = true;
+            if (warp < 4) {
+                float v[16];
+                tmem_ld16(U + lanes, v);
+                const long long gr = tile * (2 * kTileM) + long(rank) * kTileM + warp * 32 + lane;
+                if (gr < n) {
+                    const float* b5 = bias + 4 * kHid;
+                    *reinterpret_cast<float4*>(out + (rows ? (long long)rows[gr] : gr) * kOut) =
+                        make_float4(v[0] + b5[0], v[1] + b5[1], v[2] + b5[2], v[3] + b5[3]);
+                }
+                tc_fence_before();
             }
-            tc_fence_after();
-            epilogue_half_ts(tmem, 1, b, a_nxt);
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            tc_fence_before();
-            __syncthreads();
-            const uint32_t t = a_cur;
-            a_cur = a_nxt;
-            a_nxt = t;
+            const uint32_t t = U;
+            U = V;
+            V = t;
+            tile = next;
         }
-        if (!ok) break;
-        // layer 5: N = 16 (4 outputs used), A from tensor memory
-        if (tid == 0) {
-            tc_fence_after();
-            const uint32_t sbo = (kHid / 8) * 128;
-#pragma unroll 1
-            for (int s = 0; s < kHid / 16; ++s)
-                mma_bf16_ts(tmem + kTmemAcc, tmem + a_cur + 8 * s, smem_desc(smem_u32(W5s) + s * 256, sbo), idesc16,
-                            s > 0);
-            mma_commit(bar_a);
-        }
-        ok = mbar_wait(bar_a, ph_a, wait_limit_ns);
-        ph_a ^= 1;
-        ok = __syncthreads_and(ok);
-        if (!ok) break;
-        tc_fence_after();
-        if (warp < 4) {
-            float v[16];
-            tmem_ld16(tmem + kTmemAcc + (uint32_t(warp * 32) << 16), v);
-            const long long gr = row0 + warp * 32 + lane;
-            if (gr < n) {
-                const float* b5 = bias + 4 * kHid;
-                *reinterpret_cast<float4*>(out + (rows ? (long long)rows[gr] : gr) * kOut) =
-                    make_float4(v[0] + b5[0], v[1] + b5[1], v[2] + b5[2], v[3] + b5[3]);
-            }
-        }
-        tc_fence_before();
-        __syncthreads();
-        tile = next;
-    }
-    if (!ok) {
-        if (tid == 0) atomicOr(err, 1);
-        mbar_wait(bar_a, ph_a, wait_limit_ns);
-        mbar_wait(bar_b, ph_b, wait_limit_ns);
-    }
-    if (tma_pending) {
-        const bool landed = mbar_wait(bar_tma, ph_tma, wait_limit_ns);
-        if (!landed && tid == 0) atomicOr(err, 2);
+        if (!ok && lane == 0) atomicOr(err, 1);
     }
     tc_fence_before();
     __syncthreads();
+    cluster_sync();  // neither CTA leaves while the other may still reach its memory
     tc_fence_after();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+    if (warp == kEpiWarps)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
 }
 #endif  // __CUDACC__
 
