@@ -76,6 +76,8 @@ __device__ __forceinline__ float exp_(float x) { return __expf(x); }
 __device__ __forceinline__ double exp_(double x) { return exp(x); }
 __device__ __forceinline__ float tanh_(float x) { return tanhf(x); }
 __device__ __forceinline__ double tanh_(double x) { return tanh(x); }
+__device__ __forceinline__ void sincos_(float x, float& s, float& c) { sincosf(x, &s, &c); }
+__device__ __forceinline__ void sincos_(double x, double& s, double& c) { sincos(x, &s, &c); }
 #else
 inline float rcp_(float x) { return 1.0f / x; }
 inline double rcp_(double x) { return 1.0 / x; }
@@ -90,6 +92,13 @@ inline double exp_(double x) { return std::exp(x); }
 inline float tanh_(float x) { return std::tanh(x); }
 inline double tanh_(double x) { return std::tanh(x); }
 #endif
+
+// Whether tanh(x) is exactly 1 in precision T: 1 - tanh(x) = 2 / (e^2x + 1) is below a
+// quarter of the spacing under 1 (2^-26 in FP32, 2^-55 in FP64).
+SIRIUS_HD __forceinline__ bool tanh_is_one(float x) { return x > 9.4f; }
+SIRIUS_HD __forceinline__ bool tanh_is_one(double x) { return x > 19.5; }
+template <class T>
+SIRIUS_HD __forceinline__ bool tanh_is_one(T) { return false; }  // (an operation count takes the general path)
 
 // The type of a function's constants when its variables are of type T.
 template <class T>

@@ -50,5 +50,9 @@ using ::cos;  // keep the float/double overloads visible next to the Counted one
 using ::sin;
 inline Counted sin(Counted a) { return tick(std::sin(a.v)); }
 inline Counted cos(Counted a) { return tick(std::cos(a.v)); }
+inline void sincos_(Counted a, Counted& s, Counted& c) {
+    s = sin(a);
+    c = cos(a);
+}
 
 }  // namespace sirius

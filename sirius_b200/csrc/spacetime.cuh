@@ -324,7 +324,8 @@ SIRIUS_HD __forceinline__ D3<T> mt_grr(const MetricDev& m, T r) {
 template <class T>
 SIRIUS_HD __forceinline__ void mt_rhs(const MetricDev& m, const T x[4], const T p[4], T k[4], T f[4]) {
     const T r = tmax(x[1], T(m.b0) * T(1.001));
-    const T s = sin(x[2]), c = cos(x[2]);
+    T s, c;
+    sincos_(x[2], s, c);
     const T s2 = tmax(s * s, T(1e-24));
     const D3<T> grr = mt_grr(m, x[1]);
     const T r2 = r * r;
@@ -348,6 +349,10 @@ SIRIUS_HD __forceinline__ D3<T> alc_f(const MetricDev& m, T x, T y, T z) {
     const T irs = rcp_(rs);
     const D3<T> R = dwith(rs, x * irs, y * irs, z * irs);
     const T sg = T(m.sigma), Rb = T(m.Rb);
+    // outside the bubble's wall both tanh are exactly 1, and f and its gradient exactly
+    // 0: nearly all of a ray's path, without its two tanh (12 frames of four families,
+    // 64^2 to 320^2: 10.12 -> 9.67 ms with the reciprocals of the other forms)
+    if (tanh_is_one((rs - Rb) * sg) && tanh_is_one((rs + Rb) * sg)) return dconst(T(0));
     return (dtanh((R + Rb) * sg) - dtanh((R - Rb) * sg)) * T(m.inv_2tanhsR);
 }
 
@@ -410,15 +415,16 @@ __device__ __forceinline__ void inv_form(const MetricDev& m, const double x[4], 
         const D3<double> grr = mt_grr<double>(m, x[1]);
         F.r = x[1];
         F.d[1] = 1.0; F.d[2] = 0.0; F.d[3] = 0.0;
-        F.diag[0] = 1.0 / m.gtt_mt; F.diag[1] = 1.0 / grr.v; F.diag[2] = 1.0 / (r * r); F.diag[3] = 1.0 / (r * r * s2);
+        const double ir2 = rcp_(r * r);
+        F.diag[0] = rcp_(m.gtt_mt); F.diag[1] = rcp_(grr.v); F.diag[2] = ir2; F.diag[3] = ir2 * rcp_(s2);
         return;
     }
     const double X = x[1], Y = x[2], Z = x[3];
     const double R2 = X * X + Y * Y + Z * Z;
     if (m.family == SIRIUS_METRIC_ALCUBIERRE) {
-        const double Rr = sqrt(R2);
+        const double iR = rsqrt_(R2), Rr = R2 * iR;
         F.r = Rr;
-        F.d[1] = X / Rr; F.d[2] = Y / Rr; F.d[3] = Z / Rr;
+        F.d[1] = X * iR; F.d[2] = Y * iR; F.d[3] = Z * iR;
         const D3<double> f = alc_f<double>(m, X, Y, Z);
         F.vf = m.vs * f.v;
         return;
