@@ -1076,6 +1076,16 @@ int launch_trace(Handle* H, int n_frames, long long total, sirius_ray_result* d_
         host->done = true;
         n_launches = 0;  // the pieces were the launch
     }
+    // a batch's per-family launches side by side, each after the first on a stream of its
+    // own: the next family's blocks fill the SMs as one family's last wave drains (12
+    // frames of 64^2 to 320^2: 9.73 -> 7.48 ms). Launches from prepared or static scratch, which
+    // may be captured, stay on the caller's stream.
+    const bool side = n_launches > 1 && !scratch;
+    if (side) {
+        const int rc = ensure_piece_streams(H);
+        if (rc != SIRIUS_OK) return rc;
+        CK(cudaEventRecord(H->piece_ev[0], st));
+    }
     for (int i = 0; i < n_launches; ++i) {
         P.family = launch_family[i];
         int g = grid;
@@ -1085,9 +1095,15 @@ int launch_trace(Handle* H, int n_frames, long long total, sirius_ray_result* d_
             g = tab_grid[i];
             if (g == 0) continue;
         }
-        launch_fn[i]<<<g, block, shmem_launch, st>>>(P);
+        cudaStream_t si = side && i > 0 ? H->piece_stream[i - 1] : st;
+        if (si != st) CK(cudaStreamWaitEvent(si, H->piece_ev[0], 0));
+        launch_fn[i]<<<g, block, shmem_launch, si>>>(P);
         CK(cudaGetLastError());
+        if (si != st) CK(cudaEventRecord(H->piece_ev[1 + i], si));
     }
+    if (side)
+        for (int i = 1; i < n_launches; ++i)
+            if (!use_table || tab_grid[i] != 0) CK(cudaStreamWaitEvent(st, H->piece_ev[1 + i], 0));
     if (timed) CK(cudaEventRecord(H->ev[2], st));
     // the pieces' copies: after the end event, which times the kernels alone
     for (int k = 1; k < n_pieces; ++k) CK(cudaStreamWaitEvent(st, H->piece_ev[1 + kMaxPieces + k], 0));
