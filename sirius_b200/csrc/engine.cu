@@ -553,7 +553,10 @@ struct Handle {
     float* d_pass_spectra = nullptr;
     size_t pass_cap = 0;
     unsigned char* d_surrogate = nullptr;  // packed surrogate weight image (surrogate::kImageBytes)
-    int* d_sur_err = nullptr;
+    int* d_sur_err = nullptr;              // [2..3] the MLP's tile counter, [8..12] the audit's sums and maxima
+    volatile int* h_sur_flag = nullptr;    // the MLP kernel's error flag, in page-locked memory the kernel can write
+    unsigned char* d_tmp = nullptr;        // inputs and outputs of the calls on host buffers (beams, metric, steps)
+    size_t tmp_cap = 0;
     // surrogate-gated rendering scratch
     SurFrameDev* d_sur_frames = nullptr;
     SurFrameDev* h_sur_frames = nullptr;  // pinned staging: per-frame basics, then with the curves
@@ -1611,6 +1614,8 @@ int sirius_cuda_destroy(sirius_cuda_handle h) {
     cudaFree(H->d_pass_image); cudaFree(H->d_pass_spectra); cudaFree(H->d_pass_frames); cudaFree(H->d_prep);
     if (H->h_sur_frames) cudaFreeHost(H->h_sur_frames);
     if (H->h_list_len) cudaFreeHost(H->h_list_len);
+    if (H->h_sur_flag) cudaFreeHost(const_cast<int*>(H->h_sur_flag));
+    cudaFree(H->d_tmp);
     train_free(H->train);
     for (auto& e : H->sev) if (e) cudaEventDestroy(e);
     for (auto& e : H->fev) if (e) cudaEventDestroy(e);
@@ -1789,8 +1794,8 @@ int sirius_cuda_trace_beams(sirius_cuda_handle h, const sirius_frame* frames, in
     long long total = 0;
     int rc = upload_frames(H, frames, n_frames, &total);
     if (rc != SIRIUS_OK) return rc;
-    sirius_beam_result* d_out = nullptr;
-    CK(cudaMalloc((void**)&d_out, size_t(total) * sizeof(sirius_beam_result)));
+    if ((rc = ensure(H, H->d_tmp, H->tmp_cap, size_t(total) * sizeof(sirius_beam_result))) != SIRIUS_OK) return rc;
+    sirius_beam_result* d_out = reinterpret_cast<sirius_beam_result*>(H->d_tmp);
     BeamParams B{};
     B.frames = H->d_frames;
     B.n_frames = n_frames;
@@ -1810,7 +1815,6 @@ int sirius_cuda_trace_beams(sirius_cuda_handle h, const sirius_frame* frames, in
                             H->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&status, H->d_status, sizeof(int), cudaMemcpyDeviceToHost, H->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(H->stream);
-    cudaFree(d_out);
     if (e != cudaSuccess) return fail(H, SIRIUS_ERR_CUDA, std::string("beam trace: ") + cudaGetErrorString(e));
     if (status & 1) return fail(H, SIRIUS_ERR_TIMEOUT, "beam kernel stopped by its watchdog");
     return SIRIUS_OK;
@@ -1913,10 +1917,9 @@ int sirius_cuda_metric_evaluate(sirius_cuda_handle h, const sirius_metric* metri
     int rc = validate_metric(H, *metric);
     if (rc != SIRIUS_OK) return rc;
     CK(cudaSetDevice(H->device));
-    double *dp = nullptr, *dgp = nullptr, *ddg = nullptr;
-    CK(cudaMalloc((void**)&dp, size_t(n) * 4 * sizeof(double)));
-    CK(cudaMalloc((void**)&dgp, size_t(n) * 16 * sizeof(double)));
-    CK(cudaMalloc((void**)&ddg, size_t(n) * 64 * sizeof(double)));
+    if ((rc = ensure(H, H->d_tmp, H->tmp_cap, size_t(n) * 84 * sizeof(double))) != SIRIUS_OK) return rc;
+    double* dp = reinterpret_cast<double*>(H->d_tmp);
+    double *dgp = dp + 4 * size_t(n), *ddg = dgp + 16 * size_t(n);
     cudaStream_t st = H->stream;
     CK(cudaMemcpyAsync(dp, positions, size_t(n) * 4 * sizeof(double), cudaMemcpyHostToDevice, st));
     metric_kernel<<<unsigned((n + 127) / 128), 128, 0, st>>>(make_metric(*metric), dp, n, precision == SIRIUS_PRECISION_MIXED,
@@ -1925,7 +1928,6 @@ int sirius_cuda_metric_evaluate(sirius_cuda_handle h, const sirius_metric* metri
     CK(cudaMemcpyAsync(g, dgp, size_t(n) * 16 * sizeof(double), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(dg, ddg, size_t(n) * 64 * sizeof(double), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    cudaFree(dp); cudaFree(dgp); cudaFree(ddg);
     return SIRIUS_OK;
 }
 
@@ -1936,12 +1938,10 @@ int sirius_cuda_dp45_step(sirius_cuda_handle h, const sirius_metric* metric, dou
     int rc = validate_metric(H, *metric);
     if (rc != SIRIUS_OK) return rc;
     CK(cudaSetDevice(H->device));
-    double *ds = nullptr, *dh = nullptr, *de = nullptr;
-    int* da = nullptr;
-    CK(cudaMalloc((void**)&ds, size_t(n) * 8 * sizeof(double)));
-    CK(cudaMalloc((void**)&dh, size_t(n) * sizeof(double)));
-    CK(cudaMalloc((void**)&de, size_t(n) * sizeof(double)));
-    CK(cudaMalloc((void**)&da, size_t(n) * sizeof(int)));
+    if ((rc = ensure(H, H->d_tmp, H->tmp_cap, size_t(n) * (10 * sizeof(double) + sizeof(int)))) != SIRIUS_OK) return rc;
+    double* ds = reinterpret_cast<double*>(H->d_tmp);
+    double *dh = ds + 8 * size_t(n), *de = dh + n;
+    int* da = reinterpret_cast<int*>(de + n);
     cudaStream_t st = H->stream;
     CK(cudaMemcpyAsync(ds, state, size_t(n) * 8 * sizeof(double), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(dh, hh, size_t(n) * sizeof(double), cudaMemcpyHostToDevice, st));
@@ -1952,7 +1952,6 @@ int sirius_cuda_dp45_step(sirius_cuda_handle h, const sirius_metric* metric, dou
     CK(cudaMemcpyAsync(err, de, size_t(n) * sizeof(double), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(accepted, da, size_t(n) * sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    cudaFree(ds); cudaFree(dh); cudaFree(de); cudaFree(da);
     return SIRIUS_OK;
 }
 
@@ -2046,9 +2045,10 @@ int sirius_cuda_surrogate_load(sirius_cuda_handle h, const float* params, int64_
     if (!H->d_surrogate) {
         if (cudaMalloc((void**)&H->d_surrogate, surrogate::kImageBytes) != cudaSuccess)
             return fail(H, SIRIUS_ERR_OUT_OF_MEMORY, "cudaMalloc surrogate weights");
-        // [0] error, [2..3] MLP tile counter, [8..12] the audit's sums and maxima
         if (cudaMalloc((void**)&H->d_sur_err, 16 * sizeof(int)) != cudaSuccess)
             return fail(H, SIRIUS_ERR_OUT_OF_MEMORY, "cudaMalloc surrogate status");
+        CK(cudaMemsetAsync(H->d_sur_err, 0, 16 * sizeof(int), H->stream));
+        CK(cudaHostAlloc((void**)&H->h_sur_flag, sizeof(int), cudaHostAllocMapped));
         CK(cudaFuncSetAttribute(surrogate::mlp_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 surrogate::kPairSmBytes));
     }
@@ -2066,12 +2066,29 @@ static int surrogate_launch(Handle* H, const float* d_features, long long n, flo
     const int grid = 2 * int(std::min<long long>(tiles, std::max(H->num_sms / 2, 1)));  // a pair of CTAs per tile
     // bound on any wait inside the kernel: the configured watchdog (default 30 s)
     const unsigned long long limit = (unsigned long long)(H->cfg.watchdog_ms > 0 ? H->cfg.watchdog_ms : 30000) * 1000000ull;
+    // (the kernel leaves the counter at zero)
     unsigned long long* counter = reinterpret_cast<unsigned long long*>(H->d_sur_err + 2);
-    CK(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st));
+    int* flag = nullptr;
+    CK(cudaHostGetDevicePointer((void**)&flag, const_cast<int*>(H->h_sur_flag), 0));
     surrogate::mlp_pair_kernel<<<grid, surrogate::kPairThreads, surrogate::kPairSmBytes, st>>>(
-        H->d_surrogate, d_features, n, d_out, H->d_sur_err, counter, limit, rows);
+        H->d_surrogate, d_features, n, d_out, flag, counter, limit, rows);
     CK(cudaGetLastError());
     return SIRIUS_OK;
+}
+
+// Before a call's MLP launches (none of the handle's is in flight: every call that launches one
+// waits for it): after an error the tile counter starts over.
+static int surrogate_begin(Handle* H, cudaStream_t st) {
+    if (!H->h_sur_flag) return SIRIUS_OK;
+    if (*H->h_sur_flag) CK(cudaMemsetAsync(H->d_sur_err, 0, 16 * sizeof(int), st));
+    *H->h_sur_flag = 0;
+    return SIRIUS_OK;
+}
+
+// The MLP kernels' error flag, once their stream has been waited for.
+static int surrogate_check(Handle* H) {
+    if (!*H->h_sur_flag) return SIRIUS_OK;
+    return fail(H, SIRIUS_ERR_TIMEOUT, "surrogate MLP kernel stopped by its wait bound");
 }
 
 int sirius_cuda_surrogate_infer(sirius_cuda_handle h, const float* d_features, int64_t n, float* d_out,
@@ -2080,14 +2097,11 @@ int sirius_cuda_surrogate_infer(sirius_cuda_handle h, const float* d_features, i
     if (!H || !d_features || !d_out || n < 0) return SIRIUS_ERR_INVALID_ARGUMENT;
     CK(cudaSetDevice(H->device));
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : cudaStreamLegacy;
-    if (H->d_sur_err) CK(cudaMemsetAsync(H->d_sur_err, 0, sizeof(int), st));
-    int rc = surrogate_launch(H, d_features, n, d_out, st);
+    int rc = surrogate_begin(H, st);
     if (rc != SIRIUS_OK) return rc;
-    int err = 0;
-    CK(cudaMemcpyAsync(&err, H->d_sur_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    if ((rc = surrogate_launch(H, d_features, n, d_out, st)) != SIRIUS_OK) return rc;
     CK(cudaStreamSynchronize(st));
-    if (err) return fail(H, SIRIUS_ERR_TIMEOUT, "surrogate MLP kernel stopped by its wait bound");
-    return SIRIUS_OK;
+    return surrogate_check(H);
 }
 
 // ---- surrogate training ----
@@ -2456,7 +2470,7 @@ static int render_surrogate_pass(Handle* H, const sirius_frame* frames, int n_fr
     }
     // 1. features, the inner-disk gate's coarse MLP pass, the gate and the
     // compacted list of rays to integrate
-    CK(cudaMemsetAsync(H->d_sur_err, 0, sizeof(int), st));
+    if ((rc = surrogate_begin(H, st)) != SIRIUS_OK) return rc;
     CK(cudaEventRecord(H->sev[0], st));
     if ((rc = surrogate_features_launch(H, frames, n_frames, total, st)) != SIRIUS_OK) return rc;
     if ((rc = surrogate_gate_launch(H, frames, n_frames, total, sc, d_gate, st, d_image_mlp == nullptr)) != SIRIUS_OK)
@@ -2506,13 +2520,12 @@ static int render_surrogate_pass(Handle* H, const sirius_frame* frames, int n_fr
     sur_audit_kernel<<<int((total + 255) / 256), 256, 0, st>>>(d_gate, d_image, H->d_mlp_out, total, audit);
     CK(cudaGetLastError());
     CK(cudaEventRecord(H->sev[4], st));
-    int err = 0, status = 0;
+    int status = 0;
     float aud[5] = {};
-    CK(cudaMemcpyAsync(&err, H->d_sur_err, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(aud, audit, sizeof(aud), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(&status, H->d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    if (err) return fail(H, SIRIUS_ERR_TIMEOUT, "surrogate MLP kernel stopped by its wait bound");
+    if ((rc = surrogate_check(H)) != SIRIUS_OK) return rc;
     if (n_int > 0 && (status & 1)) return fail(H, SIRIUS_ERR_TIMEOUT, "trace kernel stopped by its watchdog");
     if (stats) {
         *stats = sirius_surrogate_stats{};
@@ -2571,6 +2584,7 @@ int sirius_cuda_surrogate_features(sirius_cuda_handle h, const sirius_frame* fra
     int rc = upload_frames(H, frames, n_frames, &total);
     H->stream = keep;
     if (rc != SIRIUS_OK) return rc;
+    if ((rc = surrogate_begin(H, st)) != SIRIUS_OK) return rc;
     if ((rc = surrogate_features_launch(H, frames, n_frames, total, st)) != SIRIUS_OK) return rc;
     if ((rc = surrogate_gate_launch(H, frames, n_frames, total, sc, d_gate, st)) != SIRIUS_OK) return rc;
     CK(cudaMemcpyAsync(d_features, H->d_feat, size_t(total) * 5 * sizeof(float), cudaMemcpyDeviceToDevice, st));

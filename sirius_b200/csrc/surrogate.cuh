@@ -102,7 +102,7 @@ __device__ __forceinline__ uint32_t act_column(int s) { return uint32_t(16 * s);
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     mlp_pair_kernel(const unsigned char* __restrict__ wimg, const float* __restrict__ feat, long long n,
-                    float* __restrict__ out, int* err, unsigned long long* tile_counter,
+                    float* __restrict__ out, volatile int* err, unsigned long long* tile_counter,
                     unsigned long long wait_limit_ns, const unsigned* __restrict__ rows) {
     extern __shared__ __align__(1024) unsigned char sm[];
     float* bias = reinterpret_cast<float*>(sm + kSmBias);
@@ -230,7 +230,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
                 }
                 for (; n_w < 4; ++n_w) ok = mbar_wait(bar(kBarW + n_w), 0, wait_limit_ns) && ok;
             }
-            if (!ok) atomicOr(err, 1);
+            if (!ok) *err = 1;
         }
         __syncwarp();
     } else if (warp == kEpiWarps + 1) {
@@ -245,9 +245,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
                 return (long long)t;
             };
             // the next one once a tile's first layer is complete: every thread has then read
-            // the tile's index, and none asks for the next before it has been told
-            for (uint32_t ph = 0; ok && next_tile() < ntiles; ph ^= 1) ok = mbar_wait(bar(kBarFirst), ph, wait_limit_ns);
-            if (!ok) atomicOr(err, 1);
+            // the tile's index, and none asks for the next before it has been told. Every
+            // cluster takes one index past the end, and the last to do so leaves the counter
+            // at zero for the next launch (after an error the host does).
+            long long t = next_tile();
+            for (uint32_t ph = 0; ok && t < ntiles; ph ^= 1)
+                if ((ok = mbar_wait(bar(kBarFirst), ph, wait_limit_ns))) t = next_tile();
+            if (t == ntiles + (long long)(gridDim.x / 2) - 1) *tile_counter = 0;
+            if (!ok) *err = 1;
         }
         __syncwarp();
     } else {
@@ -354,7 +359,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
             V = t;
             tile = next;
         }
-        if (!ok && lane == 0) atomicOr(err, 1);
+        if (!ok && lane == 0) *err = 1;
     }
     tc_fence_before();
     __syncthreads();

@@ -61,3 +61,12 @@ def test_sizes_equal_one_launch(engine, full, n):
         engine.surrogate_infer(part.data_ptr(), n, out.data_ptr())
         assert torch.equal(out[:n], y[first:first + n])
         assert torch.isnan(out[n:]).all()
+
+
+def test_launches_of_any_size_in_turn(engine, full):
+    """The tile counter, which the kernel itself leaves at zero, serves launches of other sizes in any order."""
+    torch, _, x, y = full
+    for n in (300, 148 * 256, 1, 4000, 257):
+        out = torch.empty(n, 4, device="cuda")
+        engine.surrogate_infer(x.data_ptr(), n, out.data_ptr())
+        assert torch.equal(out, y[:n])
