@@ -489,16 +489,20 @@ __device__ __forceinline__ double project_null(const MetricDev& m, const InvForm
     return C;
 }
 
-// The same re-projection for the mixed-precision path, Kerr-Schild family
-// without Lambda. Only the null value C = g^{-1}(p, p) needs FP64: it is a
-// difference of O(p^2) terms that must survive to ~1e-16 of them, so r, H and
-// l are FP64 (two reciprocal square roots and one reciprocal). The direction dr
-// and the coefficients A = g^{-1}(dr, dr), B = 2 g^{-1}(p, dr) only set alpha =
-// C / q, which needs single-precision relative accuracy; they are FP32, and
-// the constraint left after the update is ~1e-7 C. Returns C; r_out = r;
-// moved: the update is beyond what an f(x, p) stored in FP32 resolves (1e-6 of p).
-__device__ __forceinline__ double project_null_ks_mixed(const MetricDev& m, const double x[4], double p[4],
-                                                        double& r_out, bool& moved) {
+// The same re-projection for the Kerr-Schild family without Lambda, where the
+// coefficients are short: l is tangent to the null congruence on which r is an affine
+// parameter, so l . dr = 1, and |dr|^2 = (r^2 + a^2) / sd, which leaves
+//   A = g^{-1}(dr, dr) = (r^2 + a^2) / sd - H,   B / 2 = g^{-1}(p, dr) = p . dr - H l#.p.
+// Only the null value C = g^{-1}(p, p) always needs FP64: it is a difference of O(p^2)
+// terms that must survive to ~1e-16 of them. The mixed path (T = float) takes the
+// direction dr and the coefficients in FP32: they only set alpha = C / q, which needs
+// single-precision relative accuracy there, and the constraint left after the update is
+// ~1e-7 C; the FP64 path (T = double) keeps everything in FP64. Returns C; r_out = r;
+// moved: the update is beyond what the stored f(x, p) resolves (1e-6 of p with FP32
+// storage, 1e-10 in FP64).
+template <class T>
+__device__ __forceinline__ double project_null_ks(const MetricDev& m, const double x[4], double p[4], double& r_out,
+                                                  bool& moved) {
     moved = false;
     const double X = x[1], Y = x[2], Z = x[3];
     const double a = m.a, a2 = m.a2;
@@ -513,26 +517,28 @@ __device__ __forceinline__ double project_null_ks_mixed(const MetricDev& m, cons
     const double H = (2.0 * m.M * r - m.Q2) * isd;
     const double lp = -p[0] + l1 * p[1] + l2 * p[2] + l3 * p[3];
     const double C = -p[0] * p[0] + p[1] * p[1] + p[2] * p[2] + p[3] * p[3] - H * lp * lp;
-    const float isdf = float(isd), rs = float(r) * isdf;
-    const float d1 = rs * float(X), d2 = rs * float(Y), d3 = float(Z) * float(den) * isdf * float(ir);
-    const float p1 = float(p[1]), p2 = float(p[2]), p3 = float(p[3]);
-    const float Hf = float(H);
-    const float ld = float(l1) * d1 + float(l2) * d2 + float(l3) * d3;
-    const float A = d1 * d1 + d2 * d2 + d3 * d3 - Hf * ld * ld;
-    const float pd = p1 * d1 + p2 * d2 + p3 * d3;
-    const float B = 2.f * (pd - Hf * float(lp) * ld);
-    const float Cf = float(C);
-    const float disc = B * B - 4.f * A * Cf;
-    if (!(disc >= 0.f) || fabsf(A) < 1e-15f) return C;
-    const float q = -0.5f * (B + copysignf(sqrtf(disc), B));
-    if (q == 0.f) return C;
-    const float al = Cf * rcp_(q);
+    const T isdt = T(isd), rs = T(r) * isdt, dt = T(den) * isdt;
+    const T d1 = rs * T(X), d2 = rs * T(Y), d3 = T(Z) * dt * T(ir);
+    const T p1 = T(p[1]), p2 = T(p[2]), p3 = T(p[3]);
+    const T Ht = T(H);
+    const T A = dt - Ht;
+    const T B = T(2) * (p1 * d1 + p2 * d2 + p3 * d3 - Ht * T(lp));
+    const T Ct = T(C);
+    const T disc = B * B - T(4) * A * Ct;
+    if (!(disc >= T(0)) || fabs(A) < T(1e-15)) return C;
+    T sq;
+    if constexpr (sizeof(T) == sizeof(double)) sq = disc * rsqrt_(fmax(disc, 1e-280));
+    else sq = sqrtf(disc);
+    const T q = T(-0.5) * (B + (B >= T(0) ? sq : -sq));
+    if (q == T(0)) return C;
+    const T al = Ct * rcp_(q);
     const double alpha = double(al);
     p[1] += alpha * double(d1);
     p[2] += alpha * double(d2);
     p[3] += alpha * double(d3);
-    const float pm = fmaxf(fmaxf(fabsf(float(p[0])), fabsf(p1)), fmaxf(fabsf(p2), fabsf(p3)));
-    moved = fabsf(al) * fmaxf(fmaxf(fabsf(d1), fabsf(d2)), fabsf(d3)) > 1e-6f * pm;
+    const float pm = fmaxf(fmaxf(fabsf(float(p[0])), fabsf(float(p1))), fmaxf(fabsf(float(p2)), fabsf(float(p3))));
+    const float dm = fmaxf(fmaxf(fabsf(float(d1)), fabsf(float(d2))), fabsf(float(d3)));
+    moved = fabsf(float(al)) * dm > (sizeof(T) == sizeof(double) ? 1e-10f : 1e-6f) * pm;
     return C;
 }
 

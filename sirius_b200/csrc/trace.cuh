@@ -633,8 +633,7 @@ __device__ __forceinline__ double volume_step_cap(double r, double z, double vx,
                                                   double r_in, double r_out) {
     const double H = hz * fmin(fmax(r, r_in), r_out);
     const double dist = fmax(fmax(r_in - r, r - r_out), fabs(z) - kVolCutoff * H);
-    const double v = sqrt(vx * vx + vy * vy + vz * vz);
-    return fmax(0.5 * H, dist) / fmax(v, 1e-3);
+    return fmax(0.5 * H, dist) * rsqrt_(fmax(vx * vx + vy * vy + vz * vz, 1e-6));
 }
 
 // The same cap in FP32 for the mixed path (a step-size bound needs a few digits).

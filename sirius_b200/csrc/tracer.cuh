@@ -245,35 +245,37 @@ __device__ __forceinline__ void end_ray(const Params& P, const Ray<MIXED>& s, in
     R->flags = flags;
 }
 
-// A point of the step's cubic Hermite interpolant at parameter q in [0, 1].
-__device__ __forceinline__ void hermite_xyz(const double x0[4], const double x1[4], const float k0[4],
-                                            const float k1[4], double h, double q, float& xs, float& ys, float& zs) {
-    const double q2 = q * q, q3 = q2 * q;
-    const double h00 = 2.0 * q3 - 3.0 * q2 + 1.0, h10 = (q3 - 2.0 * q2 + q) * h, h01 = -2.0 * q3 + 3.0 * q2,
-                 h11 = (q3 - q2) * h;
-    xs = float(h00 * x0[1] + h10 * k0[1] + h01 * x1[1] + h11 * k1[1]);
-    ys = float(h00 * x0[2] + h10 * k0[2] + h01 * x1[2] + h11 * k1[2]);
-    zs = float(h00 * x0[3] + h10 * k0[3] + h01 * x1[3] + h11 * k1[3]);
-}
-
 __device__ __forceinline__ float ks_r(const MetricDev& m, float x, float y, float z) {
     const float a2 = m.fa2, R2 = x * x + y * y + z * z, Rm2 = R2 - a2;
     const float sd = sqrtp_(fmaxf(Rm2 * Rm2 + 4.f * a2 * z * z, 1e-20f));
     return sqrtp_(fmaxf(0.5f * (Rm2 + sd), 1e-10f));
 }
 
-// A point of the step's cubic Hermite interpolant at parameter q in [0, 1], in
-// FP32 relative to the step's start: x(q) = x0 + h10 k0 + h01 (x1 - x0) + h11 k1
-// (the mixed path; the step is short against |x0|, so the offset carries the
-// digits that matter).
-__device__ __forceinline__ void hermite_xyz_f(const float x0[3], const float dx[3], const float k0[4],
-                                              const float k1[4], float h, float q, float& xs, float& ys, float& zs) {
-    const float q2 = q * q, q3 = q2 * q;
-    const float h10 = (q3 - 2.f * q2 + q) * h, h01 = 3.f * q2 - 2.f * q3, h11 = (q3 - q2) * h;
-    xs = x0[0] + (h10 * k0[1] + h01 * dx[0] + h11 * k1[1]);
-    ys = x0[1] + (h10 * k0[2] + h01 * dx[1] + h11 * k1[2]);
-    zs = x0[2] + (h10 * k0[3] + h01 * dx[2] + h11 * k1[3]);
-}
+// The step's cubic Hermite interpolant in powers of q in [0, 1] relative to the step's
+// start, x(q) = x0 + q (m0 + q (c2 + q c3)): with the coefficients formed once a step,
+// each of its points (four quadrature points and up to three on an annulus edge) is three
+// multiply-adds a coordinate. In FP32 on the mixed path (the step is short against |x0|,
+// so the offset carries the digits that matter), FP64 on the FP64 path.
+template <class T>
+struct StepCubic {
+    T x0[3], m0[3], c2[3], c3[3];
+    __device__ __forceinline__ StepCubic(const double a[4], const double b[4], const float k0[4], const float k1[4],
+                                         double h) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const T d = T(b[i + 1] - a[i + 1]), m1 = T(h) * T(k1[i + 1]);
+            x0[i] = T(a[i + 1]);
+            m0[i] = T(h) * T(k0[i + 1]);
+            c2[i] = T(3) * d - T(2) * m0[i] - m1;
+            c3[i] = m0[i] + m1 - T(2) * d;
+        }
+    }
+    __device__ __forceinline__ void at(T q, float& xs, float& ys, float& zs) const {
+        xs = float(x0[0] + q * (m0[0] + q * (c2[0] + q * c3[0])));
+        ys = float(x0[1] + q * (m0[1] + q * (c2[1] + q * c3[1])));
+        zs = float(x0[2] + q * (m0[2] + q * (c2[2] + q * c3[2])));
+    }
+};
 
 // |b| (base-2 exponent of a bin's optical depth) below which the series alone
 // is the bin's 1 - e^-x: x = |b| ln 2 < 0.04
@@ -289,7 +291,7 @@ constexpr float kSeriesOnlyB = 0.04f / 0.693147180559945309f;
 //   dtau = alpha (nu_cam/g) dl, S = g^3 / c_a.
 // The bins are updated in pairs with packed FP32 arithmetic: vol[j * blockDim]
 // holds (I_2j, I_2j+1), vol[(npair + j) * blockDim] (T_2j, T_2j+1). MIXED
-// evaluates the interpolant in FP32 (hermite_xyz_f); the FP64 path in FP64.
+// evaluates the interpolant in FP32, the FP64 path in FP64 (StepCubic).
 template <bool MIXED>
 __device__ __forceinline__ void volumetric_segment(const Params& P, const FrameDev& F, const double x0[4],
                                                 const double x1[4], const float k0[4], const float k1[4],
@@ -302,15 +304,9 @@ __device__ __forceinline__ void volumetric_segment(const Params& P, const FrameD
     const float iaoj = rcp_(c.fvol_aoj);
     const float rin = F.fdisk_in, rout = F.fdisk_out;
     const bool in0 = r0 >= rin && r0 <= rout, in1 = r1 >= rin && r1 <= rout;
-    float xf0[3], dxf[3];
-    if constexpr (MIXED) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) { xf0[i] = float(x0[i + 1]); dxf[i] = float(x1[i + 1] - x0[i + 1]); }
-    }
-    auto point = [&](double q, float& xs, float& ys, float& zs) {
-        if constexpr (MIXED) hermite_xyz_f(xf0, dxf, k0, k1, float(h), float(q), xs, ys, zs);
-        else hermite_xyz(x0, x1, k0, k1, h, q, xs, ys, zs);
-    };
+    using K = typename Ray<MIXED>::K;
+    const StepCubic<K> path(x0, x1, k0, k1, h);
+    auto point = [&](double q, float& xs, float& ys, float& zs) { path.at(K(q), xs, ys, zs); };
     double fa = 0.0, fb = 1.0;
     if (in0 != in1) {
         // the annulus edge on the step's Hermite interpolant: regula falsi
@@ -719,12 +715,12 @@ __device__ __forceinline__ int advance_post(const Params& P, Ray<MIXED>& s, bool
     // forms only the null value in FP64 (Kerr-Schild without Lambda)
     double rr;
     const bool project = c.proj_period == 1 || (c.proj_period > 1 && (s.steps % c.proj_period) == 0);
-    const bool ks_fast = MIXED && is_family<FAM>(m, SIRIUS_METRIC_KERR_SCHILD) && !m.has_lambda;
+    const bool ks_fast = is_family<FAM>(m, SIRIUS_METRIC_KERR_SCHILD) && !m.has_lambda;
     if (project) {
         double before;
         bool stale;  // the projection moved p beyond what the stored f(x, p) resolves: recompute it
         if (ks_fast) {
-            before = project_null_ks_mixed(m, s.x, s.p, rr, stale);
+            before = project_null_ks<K>(m, s.x, s.p, rr, stale);
         } else {
             double pb[4];
 #pragma unroll
