@@ -1272,7 +1272,8 @@ struct TrainState {
     float* m2 = nullptr;
     __nv_bfloat16* wbf = nullptr;  // BF16 copies the GEMMs read (train::kBfTotal elements)
     train::StepState* st = nullptr;
-    int* err = nullptr;
+    int* err = nullptr;  // [0] error flag, [2..3] the forward kernel's tile counter (which it leaves at zero)
+    CUtensorMap wmap[4] = {};  // W2, W3, W4, W5 of wbf for the forward kernel
     long long cap = 0;  // rows the activation buffers hold
     __nv_bfloat16* x0 = nullptr;
     __nv_bfloat16* h[4] = {};
@@ -1351,10 +1352,8 @@ void gemm_launch(const train::GemmArgs& g0, cudaStream_t s) {
 
 int train_set_attributes(Handle* H) {
     using namespace train;
-    CK(cudaFuncSetAttribute(gemm_kernel<256, kEpiHidden, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            GemmSmem<256>::Bytes));
-    CK(cudaFuncSetAttribute(gemm_kernel<256, kEpiHidden, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            GemmSmem<256>::Bytes));
+    CK(cudaFuncSetAttribute(surrogate::train_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            surrogate::kPairSmBytes));
     CK(cudaFuncSetAttribute(gemm_kernel<256, kEpiDHidden, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             GemmSmem<256>::Bytes));
     CK(cudaFuncSetAttribute(gemm_kernel<256, kEpiDHidden, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1435,36 +1434,19 @@ void use_tma(train::GemmArgs& g, int bn, bool a, bool b) {
 // forward over the first `rows` gathered rows: Z_l, H_l (l = 1..4) and Y
 void train_forward(const Handle* H, TrainState* T, int rows, cudaStream_t s) {
     using namespace train;
-    GemmArgs g{};
-    g.err = T->err;
-    g.wait_limit_ns = train_wait_limit(H);
-    g.M = rows;
-    g.N = kHid;
+    surrogate::TrainForward f{};
+    f.x0 = T->x0;
+    f.w1 = T->wbf + kBfW1;
+    for (int l = 0; l < 5; ++l) f.bias[l] = T->params + kOffB[l];
     for (int l = 0; l < 4; ++l) {
-        const int K = l == 0 ? kInPad : kHid;
-        g.a = Operand{l == 0 ? T->x0 : T->h[l - 1], K, 1, rows};
-        g.b = Operand{T->wbf + kTrainBf[l], K, 1, kHid};
-        g.K = g.k_per_cta = K;
-        g.e = EpiArgs{};
-        g.e.bias = T->params + kOffB[l];
-        g.e.z = T->z[l];
-        g.e.ldz = kHid;
-        g.e.h = T->h[l];
-        g.e.ldh = kHid;
-        use_tma(g, 256, l > 0, l > 0);
-        gemm_launch<256, kEpiHidden>(g, s);
+        f.z[l] = T->z[l];
+        f.h[l] = T->h[l];
     }
-    g.a = Operand{T->h[3], kHid, 1, rows};
-    g.b = Operand{T->wbf + kBfW5, kHid, 1, kOutPad};
-    g.N = kOutPad;
-    g.K = g.k_per_cta = kHid;
-    g.e = EpiArgs{};
-    g.e.bias = T->params + kOffB[4];
-    g.e.y = T->y;
-    g.e.ldy = kOut;
-    g.e.ny = kOut;
-    use_tma(g, 16, true, true);
-    gemm_launch<16, kEpiOutput>(g, s);
+    for (int l = 0; l < 4; ++l) f.w[l] = T->wmap[l];
+    const int tiles = (rows + 2 * surrogate::kTileM - 1) / (2 * surrogate::kTileM);
+    const int grid = 2 * std::min(tiles, std::max(H->num_sms / 2, 1));
+    surrogate::train_forward_kernel<<<grid, surrogate::kPairThreads, surrogate::kPairSmBytes, s>>>(
+        f, rows, T->y, T->err, reinterpret_cast<unsigned long long*>(T->err + 2), train_wait_limit(H));
 }
 
 void train_loss(TrainState* T, int rows, bool with_grad, cudaStream_t s) {
@@ -2144,9 +2126,13 @@ int sirius_cuda_train_init(sirius_cuda_handle h, const float* params, const siri
         CK(cudaMalloc((void**)&T->m2, pb));
         CK(cudaMalloc((void**)&T->wbf, train::kBfTotal * sizeof(__nv_bfloat16)));
         CK(cudaMalloc((void**)&T->st, sizeof(train::StepState)));
-        CK(cudaMalloc((void**)&T->err, sizeof(int)));
+        CK(cudaMalloc((void**)&T->err, 4 * sizeof(int)));
         const int rc = train_set_attributes(H);
         if (rc != SIRIUS_OK) return rc;
+        const long long w[4] = {train::kBfW2, train::kBfW3, train::kBfW4, train::kBfW5};
+        for (int l = 0; l < 4; ++l)
+            if (!kmajor_map(&T->wmap[l], T->wbf + w[l], l < 3 ? 256 : 16, 256, 256, l < 3 ? 128 : 8))
+                return fail(H, SIRIUS_ERR_CUDA, "no tensor map for the training weights");
     }
     TrainState* T = H->train;
     train_drop_graph(T);  // the captured step embeds the configuration
@@ -2160,7 +2146,7 @@ int sirius_cuda_train_init(sirius_cuda_handle h, const float* params, const siri
     CK(cudaMemsetAsync(T->m2, 0, pb, H->stream));
     CK(cudaMemsetAsync(T->wbf, 0, train::kBfTotal * sizeof(__nv_bfloat16), H->stream));
     CK(cudaMemsetAsync(T->st, 0, sizeof(train::StepState), H->stream));
-    CK(cudaMemsetAsync(T->err, 0, sizeof(int), H->stream));
+    CK(cudaMemsetAsync(T->err, 0, 4 * sizeof(int), H->stream));
     train::weights_to_bf16_kernel<<<H->num_sms, 256, 0, H->stream>>>(T->params, T->wbf);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(H->stream));

@@ -29,6 +29,7 @@
 // CTAs meet (and free their TMEM) at the end in any case.
 #pragma once
 
+#include <cuda.h>  // CUtensorMap (a plain 128-byte descriptor type; nothing from the driver library is linked)
 #include <cuda_bf16.h>
 #include <cstdint>
 
@@ -100,10 +101,31 @@ constexpr uint32_t kTmemCols = 512;
 // the TMEM column, within its half, of K step s (16 elements) of the activations
 __device__ __forceinline__ uint32_t act_column(int s) { return uint32_t(16 * s); }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
-    mlp_pair_kernel(const unsigned char* __restrict__ wimg, const float* __restrict__ feat, long long n,
-                    float* __restrict__ out, volatile int* err, unsigned long long* tile_counter,
-                    unsigned long long wait_limit_ns, const unsigned* __restrict__ rows) {
+// The training forward pass over the same network: input rows already packed (BF16, 16
+// wide), the weights the optimiser's row-major BF16 copies (layers 2..5 by TMA with the
+// 128-byte swizzle), and every layer's pre-activations (FP32) and activations (BF16) kept
+// for the backward pass.
+struct TrainForward {
+    const __nv_bfloat16* x0;  // n x 16
+    const __nv_bfloat16* w1;  // 256 x 16
+    const float* bias[5];
+    float* z[4];              // n x 256
+    __nv_bfloat16* h[4];      // n x 256
+    CUtensorMap w[4];         // W2, W3, W4 in 128 x 64 boxes, W5 (16 x 256) in 8 x 64 boxes
+};
+
+// 32 bytes of global memory (32-byte aligned) in one instruction
+__device__ __forceinline__ void st_global_32(void* p, const uint32_t r[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+                 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+
+template <bool TRAIN>
+__device__ __forceinline__ void mlp_pair_body(const unsigned char* __restrict__ wimg, const float* __restrict__ feat,
+                                              long long n, float* __restrict__ out, volatile int* err,
+                                              unsigned long long* tile_counter, unsigned long long wait_limit_ns,
+                                              const unsigned* __restrict__ rows, const TrainForward* tf) {
     extern __shared__ __align__(1024) unsigned char sm[];
     float* bias = reinterpret_cast<float*>(sm + kSmBias);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + kSmSlot);
@@ -132,8 +154,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
                      "r"(kTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
     }
-    for (int i = tid; i < kBiasBytes / 16; i += kPairThreads)
-        reinterpret_cast<float4*>(bias)[i] = reinterpret_cast<const float4*>(wimg + kOffBias)[i];
+    if constexpr (TRAIN) {
+        for (int i = tid; i < 4 * kHid; i += kPairThreads) bias[i] = tf->bias[i / kHid][i % kHid];
+        if (tid < kOutPad) bias[4 * kHid + tid] = tid < kOut ? tf->bias[4][tid] : 0.f;
+        // this CTA's 128 rows of W1, into the core-matrix layout
+        for (int i = tid; i < kTileM * 2; i += kPairThreads)
+            *reinterpret_cast<uint4*>(sm + kSmW1 + packed_offset(i >> 1, (i & 1) * 8, kInPad)) =
+                reinterpret_cast<const uint4*>(tf->w1 + size_t(rank) * kTileM * kInPad)[i];
+        fence_async_smem();
+    } else {
+        for (int i = tid; i < kBiasBytes / 16; i += kPairThreads)
+            reinterpret_cast<float4*>(bias)[i] = reinterpret_cast<const float4*>(wimg + kOffBias)[i];
+    }
     tc_fence_before();
     __syncthreads();
     cluster_sync();  // both CTAs' barriers and TMEM are set up
@@ -150,12 +182,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
                     "l"(wimg + src + size_t(rank) * bytes), "r"(bytes), "r"(bar(b))
                     : "memory");
             };
-            mbar_expect_tx(bar(kBarW), kW1Bytes / 2 + kW5Bytes / 2);
-            copy(kSmW1, kOffW1, kW1Bytes / 2, kBarW);
-            copy(kSmW5, kOffW5, kW5Bytes / 2, kBarW);
-            for (int l = 0; l < 3; ++l) {
-                mbar_expect_tx(bar(kBarW + 1 + l), kBigBytes / 2);
-                copy(kSmW + l * (kBigBytes / 2), size_t(l) * kBigBytes, kBigBytes / 2, kBarW + 1 + l);
+            if constexpr (TRAIN) {
+                mbar_expect_tx(bar(kBarW), kW5Bytes / 2);
+                for (int c = 0; c < 4; ++c)
+                    tma_load_2d(sm0 + kSmW5 + c * 1024, &tf->w[3], 64 * c, 8 * int(rank), bar(kBarW));
+                for (int l = 0; l < 3; ++l) {
+                    mbar_expect_tx(bar(kBarW + 1 + l), kBigBytes / 2);
+                    for (int c = 0; c < 4; ++c)
+                        tma_load_2d(sm0 + kSmW + l * (kBigBytes / 2) + c * 16384, &tf->w[l], 64 * c, 128 * int(rank),
+                                    bar(kBarW + 1 + l));
+                }
+            } else {
+                mbar_expect_tx(bar(kBarW), kW1Bytes / 2 + kW5Bytes / 2);
+                copy(kSmW1, kOffW1, kW1Bytes / 2, kBarW);
+                copy(kSmW5, kOffW5, kW5Bytes / 2, kBarW);
+                for (int l = 0; l < 3; ++l) {
+                    mbar_expect_tx(bar(kBarW + 1 + l), kBigBytes / 2);
+                    copy(kSmW + l * (kBigBytes / 2), size_t(l) * kBigBytes, kBigBytes / 2, kBarW + 1 + l);
+                }
             }
             if (rank == 1)
                 for (int i = 0; i < 4; ++i) {
@@ -165,6 +209,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
             if (rank == 0) {
                 const uint32_t id256 = instr_desc_pair(kHid), id16 = instr_desc_pair(kOutPad);
                 const uint32_t sbo1 = (kInPad / 8) * 128, sbo = (kHid / 8) * 128;
+                // the descriptor of K step s of a layer's weights; chunk: bytes of 64 columns (swizzled)
+                auto wdesc = [&](uint32_t w, int s, uint32_t chunk) {
+                    return TRAIN ? smem_desc_sw128(w + uint32_t(s >> 2) * chunk + uint32_t(s & 3) * 32)
+                                 : smem_desc(w + uint32_t(s) * 256, sbo);
+                };
                 uint32_t ph_x = 0, ph_a = 0, ph_out = 0, ph_tile = 0;
                 auto operand = [&](int c) {  // 64 columns of the operand are there
                     ok = mbar_wait_cluster(bar(kBarA + c), ph_a, wait_limit_ns);
@@ -199,7 +248,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
                             if (!operand(c)) break;
 #pragma unroll
                             for (int s = 4 * c; s < 4 * c + 4; ++s)
-                                mma_bf16_ts_pair(D, A + act_column(s), smem_desc(wl + s * 256, sbo), id256, s > 0);
+                                mma_bf16_ts_pair(D, A + act_column(s), wdesc(wl, s, 16384), id256, s > 0);
                         }
                         if (!ok) break;
                         ph_a ^= 1;
@@ -212,7 +261,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
                         if (!operand(c)) break;
 #pragma unroll
                         for (int s = 4 * c; s < 4 * c + 4; ++s)
-                            mma_bf16_ts_pair(D, A + act_column(s), smem_desc(sm0 + kSmW5 + s * 256, sbo), id16, s > 0);
+                            mma_bf16_ts_pair(D, A + act_column(s), wdesc(sm0 + kSmW5, s, 1024), id16, s > 0);
                     }
                     if (!ok) break;
                     ph_a ^= 1;
@@ -260,11 +309,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
         const int group = warp >> 2;
         const int in_r = tid >> 1, in_chunk = tid & 1;
         float xin[kIn];
+        uint4 xrow;  // TRAIN: this thread's half row
         // this thread's input row (tid / 2) of a tile; rows past n read as zeros, which
         // pack to zero operands
         auto fetch_row = [&](long long t) {
             const long long gr = t * (2 * kTileM) + long(rank) * kTileM + in_r;
             const bool live = gr < n && in_r < kTileM;
+            if constexpr (TRAIN) {
+                xrow = live ? reinterpret_cast<const uint4*>(tf->x0)[2 * gr + in_chunk] : make_uint4(0, 0, 0, 0);
+                return;
+            }
             const float* f = feat + (live ? (rows ? (long long)rows[gr] : gr) : 0LL) * kIn;
 #pragma unroll
             for (int k = 0; k < kIn; ++k) xin[k] = live ? f[k] : 0.f;
@@ -272,9 +326,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
         const uint32_t bar_x = peer_addr(bar(kBarX), 0);
         auto store_row = [&]() {
             if (in_r >= kTileM) return;  // (whole warps)
-            uint4 c0, c1;
-            pack_input_row(xin, c0, c1);
-            *reinterpret_cast<uint4*>(sm + kSmX + packed_offset(in_r, in_chunk * 8, kInPad)) = in_chunk == 0 ? c0 : c1;
+            if constexpr (!TRAIN) {
+                uint4 c0, c1;
+                pack_input_row(xin, c0, c1);
+                xrow = in_chunk == 0 ? c0 : c1;
+            }
+            *reinterpret_cast<uint4*>(sm + kSmX + packed_offset(in_r, in_chunk * 8, kInPad)) = xrow;
             fence_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster_relaxed(bar_x);
@@ -300,6 +357,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
         while (ok && tile < ntiles) {
             long long next = ntiles;
             uint32_t src = U;
+            // the row of this thread's TMEM lane
+            const long long gr_out = tile * (2 * kTileM) + long(rank) * kTileM + (warp & 3) * 32 + lane;
 #pragma unroll 1
             for (int l = 0; l < 4; ++l) {
                 if (!(ok = all(mbar_wait(bar(kBarD), ph_d, wait_limit_ns)))) break;
@@ -314,9 +373,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
                     tmem_wait_ld16(v[c & 1]);
                     if (c < 3) tmem_ld16_async(col + 64 * (c + 1), v[(c + 1) & 1]);
                     uint32_t r[8];
+                    if constexpr (TRAIN) {  // Z = acc + bias, kept
+                        uint32_t* q = v[c & 1];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float4 b = b4[16 * c + i];
+                            q[4 * i] = __float_as_uint(__uint_as_float(q[4 * i]) + b.x);
+                            q[4 * i + 1] = __float_as_uint(__uint_as_float(q[4 * i + 1]) + b.y);
+                            q[4 * i + 2] = __float_as_uint(__uint_as_float(q[4 * i + 2]) + b.z);
+                            q[4 * i + 3] = __float_as_uint(__uint_as_float(q[4 * i + 3]) + b.w);
+                        }
+                        if (gr_out < n) {
+                            float* zr = tf->z[l] + gr_out * kHid + 64 * c + 16 * group;
+                            st_global_32(zr, q);
+                            st_global_32(zr + 8, q + 8);
+                        }
+                    }
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
-                        const float4 b = b4[16 * c + i];
+                        const float4 b = TRAIN ? make_float4(0.f, 0.f, 0.f, 0.f) : b4[16 * c + i];
                         const uint32_t* q = v[c & 1] + 4 * i;
                         const float2 y0 = silu_bias2(make_float2(__uint_as_float(q[0]), __uint_as_float(q[1])),
                                                      make_float2(b.x, b.y));
@@ -326,6 +401,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
                         r[2 * i + 1] = pack_bf16x2(y1.x, y1.y);
                     }
                     tmem_st8(col + 64 * c, r);
+                    if constexpr (TRAIN)
+                        if (gr_out < n) st_global_32(tf->h[l] + gr_out * kHid + 64 * c + 16 * group, r);
                     tmem_wait_st();
                     tc_fence_before();
                     __syncwarp();
@@ -346,10 +423,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
             if (warp < 4) {
                 float v[16];
                 tmem_ld16(U + lanes, v);
-                const long long gr = tile * (2 * kTileM) + long(rank) * kTileM + warp * 32 + lane;
-                if (gr < n) {
+                if (gr_out < n) {
                     const float* b5 = bias + 4 * kHid;
-                    *reinterpret_cast<float4*>(out + (rows ? (long long)rows[gr] : gr) * kOut) =
+                    *reinterpret_cast<float4*>(out + (rows ? (long long)rows[gr_out] : gr_out) * kOut) =
                         make_float4(v[0] + b5[0], v[1] + b5[1], v[2] + b5[2], v[3] + b5[3]);
                 }
                 tc_fence_before();
@@ -367,6 +443,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     tc_fence_after();
     if (warp == kEpiWarps)
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+    mlp_pair_kernel(const unsigned char* __restrict__ wimg, const float* __restrict__ feat, long long n,
+                    float* __restrict__ out, volatile int* err, unsigned long long* tile_counter,
+                    unsigned long long wait_limit_ns, const unsigned* __restrict__ rows) {
+    mlp_pair_body<false>(wimg, feat, n, out, err, tile_counter, wait_limit_ns, rows, nullptr);
+}
+
+// n rows of the training set's batch; y: n x 4. Bound by what it keeps, 6 KB a row: 201 MB
+// for 32768 rows are 31 us at the measured copy bandwidth, and the stores, 32 bytes of a
+// row per lane, take the SMs' store path about twice that (67 us; five GEMM launches that
+// read every activation back took 95).
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+    train_forward_kernel(const __grid_constant__ TrainForward tf, long long n, float* __restrict__ y, volatile int* err,
+                         unsigned long long* tile_counter, unsigned long long wait_limit_ns) {
+    mlp_pair_body<true>(nullptr, nullptr, n, y, err, tile_counter, wait_limit_ns, nullptr, &tf);
 }
 #endif  // __CUDACC__
 

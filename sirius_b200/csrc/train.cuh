@@ -8,7 +8,8 @@
 //               tile X0 (B x 16, features 0..4 as two BF16 terms, zero padding) and FP32
 //               targets / weights; zeroes the loss sums
 //   forward     Z_l = H_{l-1} W_l^T + b_l, H_l = BF16(SiLU(Z_l)) for l = 1..4
-//               and Y = H_4 W_5^T + b_5 (tcgen05 GEMMs, epilogue fused)
+//               and Y = H_4 W_5^T + b_5: one kernel, the inference kernel's, which
+//               keeps Z_l and H_l (train_forward_kernel in surrogate.cuh)
 //   loss        batch sums, then dL/dY (BF16, 16 wide) and the b_5 gradient
 //   backward    dW_5^T = H_4^T dY, dH_4 = dY W_5, and for l = 4..1
 //               dZ_l = dH_l * SiLU'(Z_l) (fused into the dH GEMM's epilogue,
@@ -41,7 +42,6 @@
 // rounded to BF16 as GEMM operands, the bias gradients are FP32 sums.
 #pragma once
 
-#include <cuda.h>  // CUtensorMap (a plain 128-byte descriptor type; nothing from the driver library is linked)
 #include <cuda_bf16.h>
 #include <cstdint>
 
@@ -80,17 +80,13 @@ struct Operand {
     int rows;                // rows present (a multiple of 8 for an M-major source); rows beyond read as zero
 };
 
-enum Epi : int { kEpiHidden = 0, kEpiOutput = 1, kEpiDHidden = 2, kEpiDWeight = 3, kEpiDWeightT = 4 };
+enum Epi : int { kEpiDHidden = 2, kEpiDWeight = 3, kEpiDWeightT = 4 };
 
 struct EpiArgs {
-    const float* bias;      // Hidden, Output: per-column FP32 bias
-    float* z;               // Hidden: pre-activations out; DHidden: pre-activations in (FP32, ld ldz)
+    const float* z;         // DHidden: pre-activations (FP32, ld ldz)
     long long ldz;
-    __nv_bfloat16* h;       // Hidden: activations out; DHidden: dZ out (BF16, ld ldh)
+    __nv_bfloat16* h;       // DHidden: dZ out (BF16, ld ldh)
     long long ldh;
-    float* y;               // Output: first ny columns, ld ldy
-    long long ldy;
-    int ny;
     float* grad;            // DHidden: per-column sums; DWeight: grad[m * ldg + n]; DWeightT: grad[n * ldg + m]
     long long ldg;
     int ng;                 // DWeight / DWeightT: columns n < ng are accumulated
@@ -267,20 +263,8 @@ __device__ __forceinline__ void warp_pieces_to_rows(float* t, const float4 q[8],
     __syncwarp();
 }
 
-// Rows at or beyond rows_end are left alone.
-__device__ __forceinline__ void warp_rows_f32_out(float* t, const float v[32], float* dst, long long ld,
-                                                  long long row0, long long rows_end) {
-    const int lane = threadIdx.x & 31;
-    float4 q[8];
-    warp_rows_to_pieces(t, v, q);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const long long r = row0 + 4 * i + (lane >> 3);
-        if (r < rows_end) *reinterpret_cast<float4*>(dst + r * ld + (lane & 7) * 4) = q[i];
-    }
-}
-
-// The same for BF16 values (eight 64-byte row segments per store instruction; tile rows of 20 words).
+// A warp's 32 x 32 block as BF16 to global memory through its tile (rows of 20 words):
+// eight 64-byte row segments per store instruction. Rows at or beyond rows_end are left alone.
 __device__ __forceinline__ void warp_rows_bf16_out(float* tf, const float v[32], __nv_bfloat16* dst, long long ld,
                                                    long long row0, long long rows_end) {
     const int lane = threadIdx.x & 31;
@@ -337,9 +321,7 @@ __device__ __forceinline__ void gemm_epilogue(const GemmArgs& g, uint32_t tmem, 
         // (unrolled over the 16 columns so that v stays in registers)
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-            if constexpr (E == kEpiOutput) {
-                if (j < g.e.ny) g.e.y[row * g.e.ldy + j] = v[j] + g.e.bias[j];
-            } else if constexpr (E == kEpiDWeight) {
+            if constexpr (E == kEpiDWeight) {
                 // fold > 0: columns c and c + fold hold the same weight (W1's two input terms)
                 const int c = n0 + j, cf = g.e.fold > 0 ? c % g.e.fold : c;
                 if (j < g.e.ng && c < g.N) atomicAdd(g.e.grad + row * g.e.ldg + cf, v[j]);
@@ -358,18 +340,7 @@ __device__ __forceinline__ void gemm_epilogue(const GemmArgs& g, uint32_t tmem, 
             float v[32];
             tmem_ld32(tl + uint32_t(c0), v);
             const int n = n0 + c0;
-            if constexpr (E == kEpiHidden) {
-                // Z = acc + bias (FP32, kept for the backward pass), H = SiLU(Z) (BF16)
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float4 b = __ldg(reinterpret_cast<const float4*>(g.e.bias + n) + i);
-                    v[4 * i] += b.x; v[4 * i + 1] += b.y; v[4 * i + 2] += b.z; v[4 * i + 3] += b.w;
-                }
-                warp_rows_f32_out(t, v, g.e.z + n, g.e.ldz, row0, g.M);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = silu(v[i]);
-                warp_rows_bf16_out(t, v, g.e.h + n, g.e.ldh, row0, g.M);
-            } else if constexpr (E == kEpiDHidden) {
+            if constexpr (E == kEpiDHidden) {
                 // dZ = dH SiLU'(Z) (BF16) and the bias gradient (column sums)
                 float z[32];
                 warp_pieces_to_rows(t, zq, z);
