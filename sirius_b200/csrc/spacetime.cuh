@@ -525,7 +525,8 @@ __device__ __forceinline__ double project_null_ks(const MetricDev& m, const doub
     const T B = T(2) * (p1 * d1 + p2 * d2 + p3 * d3 - Ht * T(lp));
     const T Ct = T(C);
     const T disc = B * B - T(4) * A * Ct;
-    if (!(disc >= T(0)) || fabs(A) < T(1e-15)) return C;
+    // (at the horizon A = 0, exactly so in FP32 for some rays: C / q needs no division by A)
+    if (!(disc >= T(0)) || (sizeof(T) == sizeof(double) && fabs(A) < T(1e-15))) return C;
     T sq;
     if constexpr (sizeof(T) == sizeof(double)) sq = disc * rsqrt_(fmax(disc, 1e-280));
     else sq = sqrtf(disc);
