@@ -531,13 +531,13 @@ def beam_leg(eng, abi, side=256):
 TRAIN_FLOP_PER_ROW = 3 * 2 * 198912 - 2 * 5 * 256  # forward, dW and dH (no dH for the input layer)
 # Algorithmic HBM bytes per training row of one step, from the kernels' operands:
 # gather 92 (features, targets, weight in; the BF16 input row, targets, weight
-# out); forward 8,240 (layer 1: input 32, Z 1024 FP32, H 512 BF16; layers 2-4:
-# H in 512, Z 1024 and H 512 out; output layer: H 512 in, y 16 out); loss 68;
+# out); forward 6,192 (input 32 in; Z 1024 FP32 and H 512 BF16 out for each of
+# four layers; y 16 out); loss 68;
 # backward 11,872 (dW5: H4 512 + dY 32; dH4: dY 32, Z4 1024 in, dZ 512 out;
 # layers 4..2: dW 512 + 512, dH 512 + Z 1024 in and dZ 512 out; dW1: 512 + 32);
 # Adam 5.6 MB of parameters and moments per step over the batch (171 B/row at
 # 32768 rows). Weights are re-read from L2 and not counted.
-TRAIN_BYTES_PER_ROW = 92 + 8240 + 68 + 11872 + 171
+TRAIN_BYTES_PER_ROW = 92 + 6192 + 68 + 11872 + 171
 
 
 def train_leg(eng, abi, np, torch, dev, rows=1 << 21, batch=32768, steps=64):

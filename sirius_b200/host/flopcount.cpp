@@ -14,9 +14,9 @@ extern "C" {
 // combination 8 x 9 = 72 and its FP64 accumulation 8 x 2 = 16, the error
 // estimate 4 x 11 + 4 x 5 + 2 = 66.
 static constexpr double kStageAlgebraFlops = 280 + 72 + 16 + 66;
-// FP64 constraint re-projection of an accepted step: inv_form (46) and
-// project_null (3 bilinear forms of 24, the root and the update: 90).
-static constexpr double kProjectionFlops = 136;
+// Constraint re-projection of an accepted step (project_null_ks): r, l and H 36, the
+// null value 16, the direction and the coefficients 18, the root and the update 14.
+static constexpr double kProjectionFlops = 84;
 
 int sirius_cuda_flop_count(const sirius_metric* metric, double* rhs_flops, double* attempt_flops,
                            double* accepted_step_flops) {
