@@ -2149,12 +2149,14 @@ int sirius_cuda_train_init(sirius_cuda_handle h, const float* params, const siri
         CK(cudaEventCreateWithFlags(&T->join, cudaEventDisableTiming));
         const int rc = train_set_attributes(H);
         if (rc != SIRIUS_OK) return rc;
-        const long long w[4] = {train::kBfW2, train::kBfW3, train::kBfW4, train::kBfW5};
-        for (int l = 0; l < 4; ++l)
-            if (!kmajor_map(&T->wmap[l], T->wbf + w[l], l < 3 ? 256 : 16, 256, 256, l < 3 ? 128 : 8))
-                return fail(H, SIRIUS_ERR_CUDA, "no tensor map for the training weights");
     }
     TrainState* T = H->train;
+    if (!T->wbf || !T->err || !T->side || !T->fork || !T->join)  // an earlier call ran out of resources here
+        return fail(H, SIRIUS_ERR_CUDA, "training state is incomplete");
+    const long long w[4] = {train::kBfW2, train::kBfW3, train::kBfW4, train::kBfW5};
+    for (int l = 0; l < 4; ++l)
+        if (!kmajor_map(&T->wmap[l], T->wbf + w[l], l < 3 ? 256 : 16, 256, 256, l < 3 ? 128 : 8))
+            return fail(H, SIRIUS_ERR_CUDA, "no tensor map for the training weights");
     train_drop_graph(T);  // the captured step embeds the configuration
     T->cfg = c;
     const int rc = train_rows(H, T, c.batch);
