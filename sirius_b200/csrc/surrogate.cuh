@@ -85,7 +85,8 @@ constexpr int kSmW = 0, kSmW1 = 3 * (kBigBytes / 2), kSmW5 = kSmW1 + kW1Bytes / 
 enum PairBar : int {  // mbarriers, 8 bytes each from kSmBar
     kBarW = 0,          // [4] this CTA's weights have landed: W1 and W5, W2, W3, W4
     kBarWReady = 4,     // [4] even CTA: the other CTA's have
-    kBarX = 8,          // even CTA: both CTAs' input rows are in shared memory
+    kBarX = 8,          // even CTA: both CTAs' input rows are in shared memory, and every epilogue warp has read
+                        // the tile's index
     kBarA = 9,          // [4] even CTA: 64 columns of activations are in both CTAs' TMEM
     kBarD = 13,         // a hidden layer's accumulator is complete
     kBarOut = 14,       // the output layer's is
@@ -142,7 +143,7 @@ __device__ __forceinline__ void mlp_pair_body(const unsigned char* __restrict__ 
             mbar_init(bar(kBarWReady + i), 1);
             mbar_init(bar(kBarA + i), 2 * kEpiWarps);
         }
-        mbar_init(bar(kBarX), 16);
+        mbar_init(bar(kBarX), 2 * kEpiWarps);
         mbar_init(bar(kBarD), 1);
         mbar_init(bar(kBarOut), 1);
         mbar_init(bar(kBarTile), 1);
@@ -293,8 +294,9 @@ __device__ __forceinline__ void mlp_pair_body(const unsigned char* __restrict__ 
                 }
                 return (long long)t;
             };
-            // the next one once a tile's first layer is complete: every thread has then read
-            // the tile's index, and none asks for the next before it has been told. Every
+            // the next one once a tile's first layer is complete: it waited for the arrivals of
+            // all epilogue warps of both CTAs on kBarX, which come after they have read the
+            // tile's index, and the issuer had read it too. Every
             // cluster takes one index past the end, and the last to do so leaves the counter
             // at zero for the next launch (after an error the host does).
             long long t = next_tile();
@@ -324,15 +326,18 @@ __device__ __forceinline__ void mlp_pair_body(const unsigned char* __restrict__ 
             for (int k = 0; k < kIn; ++k) xin[k] = live ? f[k] : 0.f;
         };
         const uint32_t bar_x = peer_addr(bar(kBarX), 0);
+        // every warp arrives, also those without rows: the first layer, after which the next
+        // index is told, then waits until all have read this one
         auto store_row = [&]() {
-            if (in_r >= kTileM) return;  // (whole warps)
-            if constexpr (!TRAIN) {
-                uint4 c0, c1;
-                pack_input_row(xin, c0, c1);
-                xrow = in_chunk == 0 ? c0 : c1;
+            if (in_r < kTileM) {  // (whole warps)
+                if constexpr (!TRAIN) {
+                    uint4 c0, c1;
+                    pack_input_row(xin, c0, c1);
+                    xrow = in_chunk == 0 ? c0 : c1;
+                }
+                *reinterpret_cast<uint4*>(sm + kSmX + packed_offset(in_r, in_chunk * 8, kInPad)) = xrow;
+                fence_async_smem();
             }
-            *reinterpret_cast<uint4*>(sm + kSmX + packed_offset(in_r, in_chunk * 8, kInPad)) = xrow;
-            fence_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster_relaxed(bar_x);
         };
