@@ -327,7 +327,8 @@ __device__ __forceinline__ void mlp_pair_body(const unsigned char* __restrict__ 
         };
         const uint32_t bar_x = peer_addr(bar(kBarX), 0);
         // every warp arrives, also those without rows: the first layer, after which the next
-        // index is told, then waits until all have read this one
+        // index is told, then waits until all have read this one. The arrival is a release:
+        // the rows are ordinary stores of 32 lanes, read by an MMA that the other CTA may issue
         auto store_row = [&]() {
             if (in_r < kTileM) {  // (whole warps)
                 if constexpr (!TRAIN) {
@@ -339,7 +340,7 @@ __device__ __forceinline__ void mlp_pair_body(const unsigned char* __restrict__ 
                 fence_async_smem();
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster_relaxed(bar_x);
+            if (lane == 0) mbar_arrive_cluster(bar_x);
         };
         auto all = [&](bool v) { return __all_sync(0xffffffffu, v) != 0; };
         uint32_t ph_tile = 0, ph_d = 0, ph_out = 0;

@@ -252,8 +252,8 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
 }
 
 // The same without the release of ordinary memory at cluster scope, whose fence costs
-// more than the arrival: for work in tensor memory, which tcgen05.fence orders, and for
-// operands in this CTA's shared memory behind a proxy fence.
+// more than the arrival: for work in tensor memory alone, which tcgen05.fence orders (a
+// proxy fence does not: it orders one thread's accesses, and hands none over to another).
 __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
