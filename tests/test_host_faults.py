@@ -1,0 +1,73 @@
+"""The library's host code on a CUDA runtime of the tests' own (fake_cuda.py): what a call allocates and keeps, and what it
+does when an allocation, a launch or a kernel's wait fails. No kernel runs: outputs are not looked at."""
+import os
+import sys
+
+import numpy as np
+import pytest
+
+sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
+import fake_cuda  # noqa: E402
+
+from sirius_b200 import abi  # noqa: E402
+from sirius_b200.engine import Engine, SiriusError, load_library  # noqa: E402
+
+WEIGHTS = os.path.join(os.path.dirname(abi.__file__), "data", "surrogate_kerr.npy")
+MLP, MLP_FLAG = "mlp_pair_kernel", 4  # the inference kernel and the place of its error flag among its arguments
+
+
+@pytest.fixture(scope="module")
+def library(tmp_path_factory):
+    return fake_cuda.link(str(tmp_path_factory.mktemp("fake")))
+
+
+@pytest.fixture
+def fake(library):
+    f = fake_cuda.Fake(library)
+    f.reset()
+    yield f
+    f.reset()
+
+
+@pytest.fixture
+def eng(library, fake):
+    e = Engine(0, lib=load_library(library))
+    yield e
+    e.close()
+    assert fake.device_bytes == 0 and fake.pinned == 0 and fake.streams == 0 and fake.events == 0
+
+
+def weights():
+    return np.load(WEIGHTS).astype(np.float32).ravel()
+
+
+def infer(eng, n=300):
+    x, y = np.zeros((n, 5), np.float32), np.zeros((n, 4), np.float32)
+    eng.surrogate_infer(x.ctypes.data, n, y.ctypes.data)
+
+
+def test_weights_take_no_page_locked_memory(eng, fake):
+    eng.surrogate_load(weights())
+    assert fake.pinned == 0
+    fake.reset()
+    infer(eng)
+    assert fake.calls("cudaMemcpyAsync") == fake.calls("cudaMemsetAsync") == 0 and fake.launches(MLP) == 1
+
+
+@pytest.mark.parametrize("watchdog,sync", [(50, 0), (200, 120)])
+def test_a_wait_that_ran_out_is_reported_and_cleared(eng, fake, watchdog, sync):
+    """A call that took long enough for a wait to run out, or whose bound is short, reads the kernel's flag."""
+    eng.configure(abi.default_config(watchdog_ms=watchdog))
+    eng.surrogate_load(weights())
+    infer(eng)
+    fake.hook(MLP, MLP_FLAG, 1)
+    fake.sync_ms(sync)
+    with pytest.raises(SiriusError) as e:
+        infer(eng)
+    assert e.value.code == abi.ERR_TIMEOUT
+    fake.reset()
+    fake.sync_ms(sync)
+    infer(eng)  # flag and counter start over
+    assert fake.calls("cudaMemsetAsync") == 1
+    infer(eng)
+    assert fake.calls("cudaMemsetAsync") == 1
