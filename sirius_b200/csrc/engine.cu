@@ -2611,7 +2611,7 @@ int sirius_cuda_surrogate_features(sirius_cuda_handle h, const sirius_frame* fra
     if ((rc = surrogate_gate_launch(H, frames, n_frames, total, sc, d_gate, st)) != SIRIUS_OK) return rc;
     CK(cudaMemcpyAsync(d_features, H->d_feat, size_t(total) * 5 * sizeof(float), cudaMemcpyDeviceToDevice, st));
     CK(cudaStreamSynchronize(st));
-    return SIRIUS_OK;
+    return surrogate_check(H, st);
 }
 
 int sirius_cuda_render_surrogate_device(sirius_cuda_handle h, const sirius_frame* frames, int32_t n_frames,

@@ -71,3 +71,27 @@ def test_a_wait_that_ran_out_is_reported_and_cleared(eng, fake, watchdog, sync):
     assert fake.calls("cudaMemsetAsync") == 1
     infer(eng)
     assert fake.calls("cudaMemsetAsync") == 1
+
+
+def frame(w=32, h=32, **metric):
+    cam = abi.make_camera(r=100.0, theta_deg=60.0, width=w, height=h, fov=30.0)
+    return abi.make_frame(abi.make_metric(**(metric or {"a": 0.9})), cam, 0.0, 30.0)
+
+
+def features(eng):
+    x, gate = np.zeros((32 * 32, 5), np.float32), np.zeros(32 * 32, np.uint8)
+    eng.surrogate_features([frame()], x.ctypes.data, gate.ctypes.data)
+
+
+def test_features_report_a_wait_that_ran_out(eng, fake):
+    """The gate rests on the network's coarse pass: its error is the call's."""
+    eng.configure(abi.default_config(watchdog_ms=50))
+    features(eng)  # without weights there is no coarse pass, and no error to read
+    eng.surrogate_load(weights())
+    features(eng)
+    fake.hook(MLP, MLP_FLAG, 1)
+    with pytest.raises(SiriusError) as e:
+        features(eng)
+    assert e.value.code == abi.ERR_TIMEOUT
+    fake.reset()
+    features(eng)
