@@ -554,8 +554,7 @@ struct Handle {
     size_t pass_cap = 0;
     unsigned char* d_surrogate = nullptr;  // packed surrogate weight image (surrogate::kImageBytes)
     int* d_sur_err = nullptr;  // [0] the MLP kernel's error flag, [2..3] its tile counter, [8..12] the audit's sums and maxima
-    bool sur_failed = false;   // the flag was found set: flag and counter start over
-    std::chrono::steady_clock::time_point sur_start;  // of the call whose MLP launches are under way
+    bool sur_failed = false;   // the last call's MLP launches ended with an error: flag and counter start over
     unsigned char* d_tmp = nullptr;        // inputs and outputs of the calls on host buffers (beams, metric, steps)
     size_t tmp_cap = 0;
     // surrogate-gated rendering scratch
@@ -2075,34 +2074,57 @@ static int surrogate_launch(Handle* H, const float* d_features, long long n, flo
     return SIRIUS_OK;
 }
 
-// Before a call's MLP launches (none of the handle's is in flight: every call that launches one
-// waits for it): after an error the flag and the tile counter start over.
-static int surrogate_begin(Handle* H, cudaStream_t st) {
-    if (!H->d_sur_err) return SIRIUS_OK;
-    if (H->sur_failed) CK(cudaMemsetAsync(H->d_sur_err, 0, 16 * sizeof(int), st));
-    H->sur_failed = false;
-    H->sur_start = std::chrono::steady_clock::now();
-    return SIRIUS_OK;
-}
+// The MLP launches of one call. None of the handle's others is in flight when it begins: every call
+// waits for its own, also where it ends early with an error (the destructor).
+struct SurrogateCall {
+    Handle* H;
+    cudaStream_t st;
+    bool open = false;
+    std::chrono::steady_clock::time_point start{};
 
-// The MLP kernels' error flag, once their stream has been waited for. A wait that runs out takes
-// its whole bound, and it began after the call did: a call that ended within half the bound
-// (the two clocks are not compared any closer) has no flag to read. That saves the copy (with the
-// memsets, which the kernel's own counter made needless, 1000 rows 36 -> 27 us) without page-locked
-// memory for the flag (1.4 to 3 ms to allocate with a new handle's weights). Bounds below 100 ms
-// always read it.
-static int surrogate_check(Handle* H, cudaStream_t st) {
-    if (!H->d_sur_err) return SIRIUS_OK;
-    const double limit = double(surrogate_wait_ns(H));
-    const double took = std::chrono::duration<double, std::nano>(std::chrono::steady_clock::now() - H->sur_start).count();
-    if (limit >= 1e8 && took < 0.5 * limit) return SIRIUS_OK;
-    int err = 0;
-    CK(cudaMemcpyAsync(&err, H->d_sur_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    if (!err) return SIRIUS_OK;
-    H->sur_failed = true;
-    return fail(H, SIRIUS_ERR_TIMEOUT, "surrogate MLP kernel stopped by its wait bound");
-}
+    SurrogateCall(Handle* h, cudaStream_t s) : H(h), st(s) {}
+    SurrogateCall(const SurrogateCall&) = delete;
+    SurrogateCall& operator=(const SurrogateCall&) = delete;
+
+    // before the launches: after an error the flag and the tile counter start over
+    int begin() {
+        if (!H->d_sur_err) return SIRIUS_OK;
+        if (H->sur_failed) CK(cudaMemsetAsync(H->d_sur_err, 0, 16 * sizeof(int), st));
+        H->sur_failed = false;
+        open = true;
+        start = std::chrono::steady_clock::now();
+        return SIRIUS_OK;
+    }
+
+    // The kernels' error flag, once their stream has been waited for. A wait that runs out takes
+    // its whole bound, and it began after the call did: a call that ended within half the bound
+    // (the two clocks are not compared any closer) has no flag to read. That saves the copy (with the
+    // memsets, which the kernel's own counter made needless, 1000 rows 36 -> 27 us) without page-locked
+    // memory for the flag (1.4 to 3 ms to allocate with a new handle's weights). Bounds below 100 ms
+    // always read it.
+    int finish() {
+        if (!open) return SIRIUS_OK;
+        const double limit = double(surrogate_wait_ns(H));
+        const double took = std::chrono::duration<double, std::nano>(std::chrono::steady_clock::now() - start).count();
+        int err = 0;
+        if (limit < 1e8 || took >= 0.5 * limit) {
+            CK(cudaMemcpyAsync(&err, H->d_sur_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+            CK(cudaStreamSynchronize(st));
+        }
+        open = false;
+        if (!err) return SIRIUS_OK;
+        H->sur_failed = true;
+        return fail(H, SIRIUS_ERR_TIMEOUT, "surrogate MLP kernel stopped by its wait bound");
+    }
+
+    ~SurrogateCall() {
+        if (!open) return;
+        H->sur_failed = true;
+        cudaStreamSynchronize(st);
+        for (auto& q : H->sur_stream)
+            if (q) cudaStreamSynchronize(q);
+    }
+};
 
 int sirius_cuda_surrogate_infer(sirius_cuda_handle h, const float* d_features, int64_t n, float* d_out,
                                 void* stream) {
@@ -2110,11 +2132,12 @@ int sirius_cuda_surrogate_infer(sirius_cuda_handle h, const float* d_features, i
     if (!H || !d_features || !d_out || n < 0) return SIRIUS_ERR_INVALID_ARGUMENT;
     CK(cudaSetDevice(H->device));
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : cudaStreamLegacy;
-    int rc = surrogate_begin(H, st);
+    SurrogateCall mlp(H, st);
+    int rc = mlp.begin();
     if (rc != SIRIUS_OK) return rc;
     if ((rc = surrogate_launch(H, d_features, n, d_out, st)) != SIRIUS_OK) return rc;
     CK(cudaStreamSynchronize(st));
-    return surrogate_check(H, st);
+    return mlp.finish();
 }
 
 // ---- surrogate training ----
@@ -2492,7 +2515,8 @@ static int render_surrogate_pass(Handle* H, const sirius_frame* frames, int n_fr
     }
     // 1. features, the inner-disk gate's coarse MLP pass, the gate and the
     // compacted list of rays to integrate
-    if ((rc = surrogate_begin(H, st)) != SIRIUS_OK) return rc;
+    SurrogateCall mlp(H, st);
+    if ((rc = mlp.begin()) != SIRIUS_OK) return rc;
     CK(cudaEventRecord(H->sev[0], st));
     if ((rc = surrogate_features_launch(H, frames, n_frames, total, st)) != SIRIUS_OK) return rc;
     if ((rc = surrogate_gate_launch(H, frames, n_frames, total, sc, d_gate, st, d_image_mlp == nullptr)) != SIRIUS_OK)
@@ -2547,7 +2571,7 @@ static int render_surrogate_pass(Handle* H, const sirius_frame* frames, int n_fr
     CK(cudaMemcpyAsync(aud, audit, sizeof(aud), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(&status, H->d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    if ((rc = surrogate_check(H, st)) != SIRIUS_OK) return rc;
+    if ((rc = mlp.finish()) != SIRIUS_OK) return rc;
     if (n_int > 0 && (status & 1)) return fail(H, SIRIUS_ERR_TIMEOUT, "trace kernel stopped by its watchdog");
     if (stats) {
         *stats = sirius_surrogate_stats{};
@@ -2606,12 +2630,13 @@ int sirius_cuda_surrogate_features(sirius_cuda_handle h, const sirius_frame* fra
     int rc = upload_frames(H, frames, n_frames, &total);
     H->stream = keep;
     if (rc != SIRIUS_OK) return rc;
-    if ((rc = surrogate_begin(H, st)) != SIRIUS_OK) return rc;
+    SurrogateCall mlp(H, st);
+    if ((rc = mlp.begin()) != SIRIUS_OK) return rc;
     if ((rc = surrogate_features_launch(H, frames, n_frames, total, st)) != SIRIUS_OK) return rc;
     if ((rc = surrogate_gate_launch(H, frames, n_frames, total, sc, d_gate, st)) != SIRIUS_OK) return rc;
     CK(cudaMemcpyAsync(d_features, H->d_feat, size_t(total) * 5 * sizeof(float), cudaMemcpyDeviceToDevice, st));
     CK(cudaStreamSynchronize(st));
-    return surrogate_check(H, st);
+    return mlp.finish();
 }
 
 int sirius_cuda_render_surrogate_device(sirius_cuda_handle h, const sirius_frame* frames, int32_t n_frames,

@@ -95,11 +95,12 @@ long fake_device_bytes() {
 long fake_pinned() { return long(pinned.size()); }
 long fake_streams() { return long(streams.size()); }
 long fake_events() { return long(events.size()); }
-long fake_pending() {
-    long n = legacy.work;
+long fake_pending_own() {  // on the library's own streams
+    long n = 0;
     for (Stream* s : streams) n += s->work;
     return n;
 }
+long fake_pending() { return fake_pending_own() + legacy.work; }
 
 // ---- registration and launches
 void** __cudaRegisterFatBinary(void*) {

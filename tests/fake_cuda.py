@@ -29,7 +29,7 @@ class Fake:
         self.lib = C.CDLL(path)
         for n in ("calls", "launches"):
             getattr(self.lib, "fake_" + n).argtypes = [C.c_char_p]
-        for n in ("calls", "launches", "device_bytes", "pinned", "streams", "events", "pending"):
+        for n in ("calls", "launches", "device_bytes", "pinned", "streams", "events", "pending", "pending_own"):
             getattr(self.lib, "fake_" + n).restype = C.c_long
         self.lib.fake_fail.argtypes = [C.c_char_p, C.c_long, C.c_int]
         self.lib.fake_hook.argtypes = [C.c_char_p, C.c_int, C.c_int]
@@ -52,5 +52,5 @@ class Fake:
     def launches(self, part):
         return self.lib.fake_launches(part.encode())
 
-    def __getattr__(self, name):  # device_bytes, pinned, streams, events, pending
+    def __getattr__(self, name):  # device_bytes, pinned, streams, events, pending, pending_own
         return getattr(self.lib, "fake_" + name)()

@@ -95,3 +95,48 @@ def test_features_report_a_wait_that_ran_out(eng, fake):
     assert e.value.code == abi.ERR_TIMEOUT
     fake.reset()
     features(eng)
+
+
+def render(eng):
+    img, gate = np.zeros(32 * 32, np.float32), np.zeros(32 * 32, np.uint8)
+    eng.render_surrogate_device([frame()], img.ctypes.data, None, gate.ctypes.data)
+
+
+def failures(fake, name, call):
+    """Have the 1st, 2nd, ... call of a runtime function within `call` fail, each in a call of its own; yields after each."""
+    nth = 1
+    while True:
+        fake.reset()
+        fake.fail(name, nth, fake_cuda.INVALID_VALUE)
+        try:
+            call()
+        except SiriusError:
+            yield nth
+        else:
+            break
+        nth += 1
+    assert nth > 1
+    fake.reset()
+
+
+@pytest.mark.parametrize("call,name", [(c, n) for c, names in (
+    (render, "cudaLaunchKernel cudaEventRecord cudaMemcpyAsync cudaMemsetAsync cudaStreamWaitEvent cudaEventSynchronize "
+             "cudaStreamSynchronize"),
+    (features, "cudaLaunchKernel cudaMemcpyAsync cudaStreamSynchronize"),
+    (infer, "cudaStreamSynchronize")) for n in names.split()])
+def test_error_exits_leave_no_network_launch_in_flight(eng, fake, name, call):
+    """A call that fails after it launched the network waits for what it has launched, and the next call starts the
+    kernel's counter over."""
+    eng.configure(abi.default_config(precision=abi.PRECISION_MIXED))
+    eng.surrogate_load(weights())
+    call(eng)
+    seen = 0
+    for _ in failures(fake, name, lambda: call(eng)):
+        if fake.launches(MLP) == 0:
+            continue
+        seen += 1
+        assert fake.pending == 0
+        fake.reset()
+        call(eng)
+        assert fake.calls("cudaMemsetAsync") >= 1 and fake.pending == 0
+    assert seen > 0
