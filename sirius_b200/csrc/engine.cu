@@ -874,6 +874,21 @@ int ensure_piece_streams(Handle* H) {
     return SIRIUS_OK;
 }
 
+// Launches on the piece streams within one call: an error exit waits for them, since what the caller
+// does next is ordered after its own stream alone.
+struct PieceGuard {
+    Handle* H;
+    bool armed = false;
+    explicit PieceGuard(Handle* h) : H(h) {}
+    PieceGuard(const PieceGuard&) = delete;
+    PieceGuard& operator=(const PieceGuard&) = delete;
+    ~PieceGuard() {
+        if (!armed) return;
+        for (auto& q : H->piece_stream)
+            if (q) cudaStreamSynchronize(q);
+    }
+};
+
 int launch_trace(Handle* H, int n_frames, long long total, sirius_ray_result* d_results, float* d_image,
                  float* d_spectra, const sirius_camera_ray* d_rays, cudaStream_t st, bool timed,
                  const LaunchScratch* scratch = nullptr, const unsigned* d_list = nullptr, bool flux_ready = false,
@@ -1045,9 +1060,11 @@ int launch_trace(Handle* H, int n_frames, long long total, sirius_ray_result* d_
     const int tile_rows = P.tiled ? int(tiled_blocks / tiles_x) : 0;
     const int n_pieces = (host && P.tiled && n_launches == 1 && tiled_blocks >= kPieceMinBlocks)
                              ? std::min(kMaxPieces, tile_rows) : 0;
+    PieceGuard pieces(H);
     if (n_pieces > 1) {
         const int rc = ensure_piece_streams(H);
         if (rc != SIRIUS_OK) return rc;
+        pieces.armed = true;
         cudaEvent_t* E = H->piece_ev;
         CK(cudaEventRecord(E[0], st));
         for (int k = 1; k < n_pieces; ++k) CK(cudaStreamWaitEvent(H->piece_stream[k - 1], E[0], 0));
@@ -1087,6 +1104,7 @@ int launch_trace(Handle* H, int n_frames, long long total, sirius_ray_result* d_
     if (side) {
         const int rc = ensure_piece_streams(H);
         if (rc != SIRIUS_OK) return rc;
+        pieces.armed = true;
         CK(cudaEventRecord(H->piece_ev[0], st));
     }
     for (int i = 0; i < n_launches; ++i) {
@@ -1110,6 +1128,7 @@ int launch_trace(Handle* H, int n_frames, long long total, sirius_ray_result* d_
     if (timed) CK(cudaEventRecord(H->ev[2], st));
     // the pieces' copies: after the end event, which times the kernels alone
     for (int k = 1; k < n_pieces; ++k) CK(cudaStreamWaitEvent(st, H->piece_ev[1 + kMaxPieces + k], 0));
+    pieces.armed = false;
     H->stats.grid_blocks = grid;
     H->stats.block_size = block;
     H->stats.kernel_launches = (n_pieces > 1 ? n_pieces : n_launches) + extra_launches;

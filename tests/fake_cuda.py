@@ -46,6 +46,10 @@ class Fake:
     def sync_ms(self, ms):
         self.lib.fake_sync_ms(ms)
 
+    def wait(self):
+        """As a caller that waits for its own (the legacy default) stream."""
+        self.lib.cudaStreamSynchronize(None)
+
     def calls(self, name):
         return self.lib.fake_calls(name.encode())
 

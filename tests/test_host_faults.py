@@ -140,3 +140,32 @@ def test_error_exits_leave_no_network_launch_in_flight(eng, fake, name, call):
         call(eng)
         assert fake.calls("cudaMemsetAsync") >= 1 and fake.pending == 0
     assert seen > 0
+
+
+def batch():
+    """Frames of two families: their launches run side by side, one of them on a stream of the library's own."""
+    frames, n = [], 0
+    for m in ({"a": 0.9}, {"family": abi.MORRIS_THORNE}, {"a": 0.5}):
+        f = frame(16, 8, **m)
+        f.ray_offset = n
+        n += 16 * 8
+        frames.append(f)
+    return (abi.Frame * len(frames))(*frames), len(frames), n
+
+
+@pytest.mark.parametrize("name", ["cudaLaunchKernel", "cudaEventRecord", "cudaStreamWaitEvent"])
+def test_error_exits_of_a_batch_leave_no_side_launch_in_flight(eng, fake, name):
+    """Whatever fails, a caller that waits for its own stream has waited for every launch."""
+    import ctypes
+    arr, k, n = batch()
+    img = np.zeros(n, np.float32)
+
+    def call():
+        eng.trace_frames_device(ctypes.addressof(arr), k, n, None, img.ctypes.data, None, None)
+
+    eng.configure(abi.default_config(precision=abi.PRECISION_MIXED))
+    call()
+    assert fake.launches("trace_kernel") == 2 and fake.pending_own > 0
+    for _ in failures(fake, name, call):
+        fake.wait()
+        assert fake.pending_own == 0
