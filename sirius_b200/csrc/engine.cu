@@ -867,10 +867,18 @@ int validate_config(Handle* H, const sirius_trace_config& c) {
 // Launch the tracer over [0, total) of already-uploaded frames.
 
 
-int ensure_piece_streams(Handle* H) {
-    if (H->piece_stream[kMaxPieces - 2]) return SIRIUS_OK;
-    for (auto& q : H->piece_stream) CK(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
-    for (auto& e : H->piece_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+// The streams of launches 1..n-1 and the events of n launches (copies: and of their copies to the
+// host); those a handle has not yet, so that a batch's first call makes one or two streams, where
+// a frame in pieces needs 7 and 17 events (about 0.7 ms).
+int ensure_piece_streams(Handle* H, int n, bool copies) {
+    auto event = [&](cudaEvent_t& e) { return e ? cudaSuccess : cudaEventCreateWithFlags(&e, cudaEventDisableTiming); };
+    CK(event(H->piece_ev[0]));
+    for (int k = 0; k < n; ++k) {
+        if (k > 0 && !H->piece_stream[k - 1])
+            CK(cudaStreamCreateWithFlags(&H->piece_stream[k - 1], cudaStreamNonBlocking));
+        if (k > 0 || copies) CK(event(H->piece_ev[1 + k]));
+        if (copies) CK(event(H->piece_ev[1 + kMaxPieces + k]));
+    }
     return SIRIUS_OK;
 }
 
@@ -1062,7 +1070,7 @@ int launch_trace(Handle* H, int n_frames, long long total, sirius_ray_result* d_
                              ? std::min(kMaxPieces, tile_rows) : 0;
     PieceGuard pieces(H);
     if (n_pieces > 1) {
-        const int rc = ensure_piece_streams(H);
+        const int rc = ensure_piece_streams(H, n_pieces, true);
         if (rc != SIRIUS_OK) return rc;
         pieces.armed = true;
         cudaEvent_t* E = H->piece_ev;
@@ -1102,7 +1110,7 @@ int launch_trace(Handle* H, int n_frames, long long total, sirius_ray_result* d_
     // may be captured, stay on the caller's stream.
     const bool side = n_launches > 1 && !scratch;
     if (side) {
-        const int rc = ensure_piece_streams(H);
+        const int rc = ensure_piece_streams(H, n_launches, false);
         if (rc != SIRIUS_OK) return rc;
         pieces.armed = true;
         CK(cudaEventRecord(H->piece_ev[0], st));

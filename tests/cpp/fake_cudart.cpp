@@ -227,7 +227,7 @@ cudaError_t cudaHostGetDevicePointer(void** d, void* h, unsigned) {
 }
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
     std::memset(a, 0, sizeof(*a));
-    a->type = cudaMemoryTypeUnregistered;
+    a->type = cudaMemoryTypeHost;
     return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t st) {

@@ -169,3 +169,24 @@ def test_error_exits_of_a_batch_leave_no_side_launch_in_flight(eng, fake, name):
     for _ in failures(fake, name, call):
         fake.wait()
         assert fake.pending_own == 0
+
+
+def test_a_batch_makes_the_streams_and_events_it_uses(eng, fake):
+    """One stream and one event for each launch after the first, and the event they wait for."""
+    import ctypes
+    arr, k, n = batch()
+    img = np.zeros(n, np.float32)
+    eng.configure(abi.default_config(precision=abi.PRECISION_MIXED))
+    streams, events = fake.streams, fake.events
+    eng.trace_frames_device(ctypes.addressof(arr), 1, 16 * 8, None, img.ctypes.data, None, None)
+    assert (fake.streams, fake.events) == (streams, events)
+    for _ in range(2):
+        eng.trace_frames_device(ctypes.addressof(arr), k, n, None, img.ctypes.data, None, None)
+        assert (fake.streams, fake.events) == (streams + 1, events + 2)
+    big = frame(512, 512)  # traced in pieces into host memory
+    eng.trace_frames([big])
+    many = fake.streams, fake.events
+    assert many[0] > streams + 1
+    eng.trace_frames([big])
+    eng.trace_frames_device(ctypes.addressof(arr), k, n, None, img.ctypes.data, None, None)
+    assert (fake.streams, fake.events) == many
