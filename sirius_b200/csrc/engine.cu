@@ -1301,6 +1301,7 @@ struct TrainState {
     train::StepState* st = nullptr;
     int* err = nullptr;  // [0] error flag, [2..3] the forward kernel's tile counter (which it leaves at zero)
     CUtensorMap wmap[4] = {};  // W2, W3, W4, W5 of wbf for the forward kernel
+    bool tma = false;          // whether the driver encoded them
     long long cap = 0;  // rows the activation buffers hold
     __nv_bfloat16* x0 = nullptr;
     __nv_bfloat16* h[4] = {};
@@ -1384,8 +1385,10 @@ void gemm_launch(const train::GemmArgs& g0, cudaStream_t s) {
 
 int train_set_attributes(Handle* H) {
     using namespace train;
-    CK(cudaFuncSetAttribute(surrogate::train_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            surrogate::kPairSmBytes));
+    CK(cudaFuncSetAttribute(surrogate::train_forward_kernel<surrogate::kTrainTma>,
+                            cudaFuncAttributeMaxDynamicSharedMemorySize, surrogate::kPairSmBytes));
+    CK(cudaFuncSetAttribute(surrogate::train_forward_kernel<surrogate::kTrainPlain>,
+                            cudaFuncAttributeMaxDynamicSharedMemorySize, surrogate::kPairSmBytes));
     CK(cudaFuncSetAttribute(gemm_kernel<256, kEpiDHidden, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             GemmSmem<256>::Bytes));
     CK(cudaFuncSetAttribute(gemm_kernel<256, kEpiDHidden, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1409,8 +1412,10 @@ EncodeTiledFn encode_tiled() {
         void* p = nullptr;
         cudaDriverEntryPointQueryResult q{};
         if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();  // (answered here, by the register path)
             return EncodeTiledFn(nullptr);
+        }
         return reinterpret_cast<EncodeTiledFn>(p);
     }();
     return fn;
@@ -1474,10 +1479,16 @@ void train_forward(const Handle* H, TrainState* T, int rows, cudaStream_t s) {
         f.z[l] = T->z[l];
         f.h[l] = T->h[l];
     }
-    for (int l = 0; l < 4; ++l) f.w[l] = T->wmap[l];
+    for (int l = 0; l < 4; ++l) {
+        f.w[l] = T->wmap[l];
+        f.wp[l] = T->wbf + (l < 3 ? kTrainBf[l + 1] : kBfW5);
+    }
     const int tiles = (rows + 2 * surrogate::kTileM - 1) / (2 * surrogate::kTileM);
     const int grid = 2 * std::min(tiles, std::max(H->num_sms / 2, 1));
-    surrogate::train_forward_kernel<<<grid, surrogate::kPairThreads, surrogate::kPairSmBytes, s>>>(
+    // (without tensor maps as the GEMMs do: operands through registers)
+    const auto kernel = T->tma ? surrogate::train_forward_kernel<surrogate::kTrainTma>
+                               : surrogate::train_forward_kernel<surrogate::kTrainPlain>;
+    kernel<<<grid, surrogate::kPairThreads, surrogate::kPairSmBytes, s>>>(
         f, rows, T->y, T->err, reinterpret_cast<unsigned long long*>(T->err + 2), train_wait_limit(H));
 }
 
@@ -2218,9 +2229,9 @@ int sirius_cuda_train_init(sirius_cuda_handle h, const float* params, const siri
     if (!T->wbf || !T->err || !T->side || !T->fork || !T->join)  // an earlier call ran out of resources here
         return fail(H, SIRIUS_ERR_CUDA, "training state is incomplete");
     const long long w[4] = {train::kBfW2, train::kBfW3, train::kBfW4, train::kBfW5};
+    T->tma = true;
     for (int l = 0; l < 4; ++l)
-        if (!kmajor_map(&T->wmap[l], T->wbf + w[l], l < 3 ? 256 : 16, 256, 256, l < 3 ? 128 : 8))
-            return fail(H, SIRIUS_ERR_CUDA, "no tensor map for the training weights");
+        T->tma = T->tma && kmajor_map(&T->wmap[l], T->wbf + w[l], l < 3 ? 256 : 16, 256, 256, l < 3 ? 128 : 8);
     train_drop_graph(T);  // the captured step embeds the configuration
     T->cfg = c;
     const int rc = train_rows(H, T, c.batch);

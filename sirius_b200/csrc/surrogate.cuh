@@ -104,15 +104,19 @@ __device__ __forceinline__ uint32_t act_column(int s) { return uint32_t(16 * s);
 
 // The training forward pass over the same network: input rows already packed (BF16, 16
 // wide), the weights the optimiser's row-major BF16 copies (layers 2..5 by TMA with the
-// 128-byte swizzle), and every layer's pre-activations (FP32) and activations (BF16) kept
-// for the backward pass.
+// 128-byte swizzle, or by plain loads into the core-matrix layout where the driver encodes no
+// tensor maps), and every layer's pre-activations (FP32) and activations (BF16) kept for the
+// backward pass.
+enum Forward : int { kInfer = 0, kTrainTma = 1, kTrainPlain = 2 };
+
 struct TrainForward {
     const __nv_bfloat16* x0;  // n x 16
     const __nv_bfloat16* w1;  // 256 x 16
     const float* bias[5];
     float* z[4];              // n x 256
     __nv_bfloat16* h[4];      // n x 256
-    CUtensorMap w[4];         // W2, W3, W4 in 128 x 64 boxes, W5 (16 x 256) in 8 x 64 boxes
+    CUtensorMap w[4];         // W2, W3, W4 in 128 x 64 boxes, W5 (16 x 256) in 8 x 64 boxes (kTrainTma)
+    const __nv_bfloat16* wp[4];  // the same weights, row-major (kTrainPlain)
 };
 
 // 32 bytes of global memory (32-byte aligned) in one instruction
@@ -122,11 +126,12 @@ __device__ __forceinline__ void st_global_32(void* p, const uint32_t r[8]) {
                  : "memory");
 }
 
-template <bool TRAIN>
+template <int MODE>
 __device__ __forceinline__ void mlp_pair_body(const unsigned char* __restrict__ wimg, const float* __restrict__ feat,
                                               long long n, float* __restrict__ out, volatile int* err,
                                               unsigned long long* tile_counter, unsigned long long wait_limit_ns,
                                               const unsigned* __restrict__ rows, const TrainForward* tf) {
+    constexpr bool TRAIN = MODE != kInfer;
     extern __shared__ __align__(1024) unsigned char sm[];
     float* bias = reinterpret_cast<float*>(sm + kSmBias);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + kSmSlot);
@@ -162,6 +167,15 @@ __device__ __forceinline__ void mlp_pair_body(const unsigned char* __restrict__ 
         for (int i = tid; i < kTileM * 2; i += kPairThreads)
             *reinterpret_cast<uint4*>(sm + kSmW1 + packed_offset(i >> 1, (i & 1) * 8, kInPad)) =
                 reinterpret_cast<const uint4*>(tf->w1 + size_t(rank) * kTileM * kInPad)[i];
+        if constexpr (MODE == kTrainPlain) {  // and of W2, W3, W4 (8 rows of W5)
+            constexpr int kPieces = kHid / 8;
+            for (int i = tid; i < (3 * kTileM + kOutPad / 2) * kPieces; i += kPairThreads) {
+                const int l = i / (kTileM * kPieces), r = i / kPieces - l * kTileM, k = 8 * (i % kPieces);
+                const int row = int(rank) * (l < 3 ? kTileM : kOutPad / 2) + r;
+                *reinterpret_cast<uint4*>(sm + (l < 3 ? kSmW + l * (kBigBytes / 2) : kSmW5) + packed_offset(r, k, kHid)) =
+                    *reinterpret_cast<const uint4*>(tf->wp[l] + size_t(row) * kHid + k);
+            }
+        }
         fence_async_smem();
     } else {
         for (int i = tid; i < kBiasBytes / 16; i += kPairThreads)
@@ -183,7 +197,9 @@ __device__ __forceinline__ void mlp_pair_body(const unsigned char* __restrict__ 
                     "l"(wimg + src + size_t(rank) * bytes), "r"(bytes), "r"(bar(b))
                     : "memory");
             };
-            if constexpr (TRAIN) {
+            if constexpr (MODE == kTrainPlain) {  // in place since the CTAs met
+                for (int i = 0; i < 4; ++i) mbar_expect_tx(bar(kBarW + i), 0);
+            } else if constexpr (TRAIN) {
                 mbar_expect_tx(bar(kBarW), kW5Bytes / 2);
                 for (int c = 0; c < 4; ++c)
                     tma_load_2d(sm0 + kSmW5 + c * 1024, &tf->w[3], 64 * c, 8 * int(rank), bar(kBarW));
@@ -212,8 +228,8 @@ __device__ __forceinline__ void mlp_pair_body(const unsigned char* __restrict__ 
                 const uint32_t sbo1 = (kInPad / 8) * 128, sbo = (kHid / 8) * 128;
                 // the descriptor of K step s of a layer's weights; chunk: bytes of 64 columns (swizzled)
                 auto wdesc = [&](uint32_t w, int s, uint32_t chunk) {
-                    return TRAIN ? smem_desc_sw128(w + uint32_t(s >> 2) * chunk + uint32_t(s & 3) * 32)
-                                 : smem_desc(w + uint32_t(s) * 256, sbo);
+                    return MODE == kTrainTma ? smem_desc_sw128(w + uint32_t(s >> 2) * chunk + uint32_t(s & 3) * 32)
+                                             : smem_desc(w + uint32_t(s) * 256, sbo);
                 };
                 uint32_t ph_x = 0, ph_a = 0, ph_out = 0, ph_tile = 0;
                 auto operand = [&](int c) {  // 64 columns of the operand are there
@@ -455,17 +471,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     mlp_pair_kernel(const unsigned char* __restrict__ wimg, const float* __restrict__ feat, long long n,
                     float* __restrict__ out, volatile int* err, unsigned long long* tile_counter,
                     unsigned long long wait_limit_ns, const unsigned* __restrict__ rows) {
-    mlp_pair_body<false>(wimg, feat, n, out, err, tile_counter, wait_limit_ns, rows, nullptr);
+    mlp_pair_body<kInfer>(wimg, feat, n, out, err, tile_counter, wait_limit_ns, rows, nullptr);
 }
 
 // n rows of the training set's batch; y: n x 4. Bound by what it keeps, 6 KB a row: 201 MB
 // for 32768 rows are 31 us at the measured copy bandwidth, and the stores, 32 bytes of a
 // row per lane, take the SMs' store path about twice that (67 us; five GEMM launches that
 // read every activation back took 95).
+template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     train_forward_kernel(const __grid_constant__ TrainForward tf, long long n, float* __restrict__ y, volatile int* err,
                          unsigned long long* tile_counter, unsigned long long wait_limit_ns) {
-    mlp_pair_body<true>(nullptr, nullptr, n, y, err, tile_counter, wait_limit_ns, nullptr, &tf);
+    mlp_pair_body<MODE>(nullptr, nullptr, n, y, err, tile_counter, wait_limit_ns, nullptr, &tf);
 }
 #endif  // __CUDACC__
 

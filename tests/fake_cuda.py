@@ -58,3 +58,18 @@ class Fake:
 
     def __getattr__(self, name):  # device_bytes, pinned, streams, events, pending, pending_own
         return getattr(self.lib, "fake_" + name)()
+
+
+def link_without_tensor_maps(folder):
+    """The library on the real runtime, but as on a driver that encodes no tensor maps; None where it cannot be linked."""
+    objs = [os.path.join(build.HERE, "_build", os.path.basename(s) + ".o") for s in build.sources()]
+    runtime = "/usr/local/cuda/lib64/libcudart_static.a"
+    if not all(os.path.exists(p) for p in objs + [runtime]):
+        return None
+    stub, lib = os.path.join(folder, "no_maps.cpp"), os.path.join(folder, "libsirius_no_maps.so")
+    with open(stub, "w") as f:
+        f.write('extern "C" int __wrap_cudaGetDriverEntryPoint(const char*, void**, unsigned long long, void*) '
+                "{ return %d; }\n" % NOT_SUPPORTED)
+    subprocess.run(["g++", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-Wl,--wrap=cudaGetDriverEntryPoint", stub, *objs,
+                    runtime, "-o", lib, "-lz", "-ldl", "-lrt", "-lpthread"], check=True)
+    return lib

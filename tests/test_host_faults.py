@@ -1,6 +1,7 @@
 """The library's host code on a CUDA runtime of the tests' own (fake_cuda.py): what a call allocates and keeps, and what it
 does when an allocation, a launch or a kernel's wait fails. No kernel runs: outputs are not looked at."""
 import os
+import shutil
 import sys
 
 import numpy as np
@@ -190,3 +191,29 @@ def test_a_batch_makes_the_streams_and_events_it_uses(eng, fake):
     eng.trace_frames([big])
     eng.trace_frames_device(ctypes.addressof(arr), k, n, None, img.ctypes.data, None, None)
     assert (fake.streams, fake.events) == many
+
+
+def training_set(n):
+    return np.zeros((n, 5), np.float32), np.zeros((n, 4), np.float32), np.ones(n, np.float32)
+
+
+def gradient(eng, n=256):
+    x, t, w = training_set(n)
+    return eng.train_gradient(x.ctypes.data, t.ctypes.data, w.ctypes.data, n)
+
+
+def test_training_without_tensor_maps(library, tmp_path):
+    """A driver that encodes no tensor maps: every operand goes through registers. (A copy of the library: it asks the
+    driver once.)"""
+    path = str(tmp_path / "libsirius_fake_no_maps.so")
+    shutil.copy(library, path)
+    fake = fake_cuda.Fake(path)
+    fake.fail("cudaGetDriverEntryPoint", 1, fake_cuda.NOT_SUPPORTED)
+    eng = Engine(0, lib=load_library(path))
+    try:
+        eng.train_init(weights(), abi.train_config(batch=256))
+        fake.reset()
+        gradient(eng)
+        assert fake.launches("train_forward_kernel") == 1 and fake.launches("gemm_kernel") == 9
+    finally:
+        eng.close()
