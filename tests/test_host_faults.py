@@ -217,3 +217,19 @@ def test_training_without_tensor_maps(library, tmp_path):
         assert fake.launches("train_forward_kernel") == 1 and fake.launches("gemm_kernel") == 9
     finally:
         eng.close()
+
+
+def test_training_rows_are_one_allocation(eng, fake):
+    """A batch's 15 buffers: one allocation, released with the next larger batch."""
+    fake.reset()
+    eng.train_init(weights(), abi.train_config(batch=256))
+    assert fake.calls("cudaMalloc") <= 8
+    small = fake.device_bytes
+    eng.train_init(weights(), abi.train_config(batch=512))
+    grown = fake.device_bytes
+    per_row = 2 * (16 + 16 + 8 * 256) + 4 * (4 * 256 + 4 + 1 + 4)
+    assert abs((grown - small) - 256 * per_row) <= 15 * 1024
+    fake.reset()
+    eng.train_init(weights(), abi.train_config(batch=256))
+    assert fake.calls("cudaMalloc") == 0 and fake.device_bytes == grown
+    gradient(eng)
