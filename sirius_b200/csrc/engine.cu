@@ -19,6 +19,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -1302,6 +1303,7 @@ struct TrainState {
     int* err = nullptr;  // [0] error flag, [2..3] the forward kernel's tile counter (which it leaves at zero)
     CUtensorMap wmap[4] = {};  // W2, W3, W4, W5 of wbf for the forward kernel
     bool tma = false;          // whether the driver encoded them
+    bool ready = false;        // an initialisation has succeeded: the parameters are there
     long long cap = 0;  // rows the activation buffers hold
     unsigned char* rows = nullptr;  // the allocation that holds them, x0 to y
     __nv_bfloat16* x0 = nullptr;
@@ -1373,6 +1375,10 @@ int train_rows(Handle* H, TrainState* T, long long rows) {
     T->cap = rows;
     return SIRIUS_OK;
 }
+
+// Whether a step can run: the parameters are there, and the buffers of the configured batch (an
+// initialisation for a larger one may have run out of memory).
+bool train_ready(const TrainState* T) { return T && T->ready && T->cap >= T->cfg.batch; }
 
 unsigned long long train_wait_limit(const Handle* H) {
     return (unsigned long long)(H->configured && H->cfg.watchdog_ms > 0 ? H->cfg.watchdog_ms : 30000) * 1000000ull;
@@ -2215,9 +2221,8 @@ int sirius_cuda_train_init(sirius_cuda_handle h, const float* params, const siri
         if (!std::isfinite(params[i])) return fail(H, SIRIUS_ERR_INVALID_ARGUMENT, "non-finite initial parameter");
     CK(cudaSetDevice(H->device));
     if (!H->train) {
-        TrainState* T = new (std::nothrow) TrainState;
+        std::unique_ptr<TrainState, void (*)(TrainState*)> T(new (std::nothrow) TrainState, train_free);
         if (!T) return fail(H, SIRIUS_ERR_OUT_OF_MEMORY, "training state");
-        H->train = T;
         const size_t pb = surrogate::kParams * sizeof(float);
         CK(cudaMalloc((void**)&T->params, pb));
         CK(cudaMalloc((void**)&T->grad, pb));
@@ -2231,10 +2236,9 @@ int sirius_cuda_train_init(sirius_cuda_handle h, const float* params, const siri
         CK(cudaEventCreateWithFlags(&T->join, cudaEventDisableTiming));
         const int rc = train_set_attributes(H);
         if (rc != SIRIUS_OK) return rc;
+        H->train = T.release();
     }
     TrainState* T = H->train;
-    if (!T->wbf || !T->err || !T->side || !T->fork || !T->join)  // an earlier call ran out of resources here
-        return fail(H, SIRIUS_ERR_CUDA, "training state is incomplete");
     const long long w[4] = {train::kBfW2, train::kBfW3, train::kBfW4, train::kBfW5};
     T->tma = true;
     for (int l = 0; l < 4; ++l)
@@ -2254,6 +2258,7 @@ int sirius_cuda_train_init(sirius_cuda_handle h, const float* params, const siri
     train::weights_to_bf16_kernel<<<H->num_sms, 256, 0, H->stream>>>(T->params, T->wbf);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(H->stream));
+    T->ready = true;
     return SIRIUS_OK;
 }
 
@@ -2262,7 +2267,7 @@ int sirius_cuda_train_steps(sirius_cuda_handle h, const float* d_features, const
     Handle* H = static_cast<Handle*>(h);
     if (!H || !d_features || !d_targets || !d_weights || n_steps < 0) return SIRIUS_ERR_INVALID_ARGUMENT;
     TrainState* T = H->train;
-    if (!T) return fail(H, SIRIUS_ERR_NOT_CONFIGURED, "sirius_cuda_train_init has not been called");
+    if (!train_ready(T)) return fail(H, SIRIUS_ERR_NOT_CONFIGURED, "sirius_cuda_train_init has not succeeded");
     if (n_rows < T->cfg.batch || n_rows > (1LL << 40))
         return fail(H, SIRIUS_ERR_INVALID_ARGUMENT, "n_rows must hold at least one batch");
     CK(cudaSetDevice(H->device));
@@ -2307,7 +2312,7 @@ int sirius_cuda_train_evaluate(sirius_cuda_handle h, const float* d_features, co
     if (!H || !d_features || !d_targets || !d_weights || !loss_parts || n_rows <= 0)
         return SIRIUS_ERR_INVALID_ARGUMENT;
     TrainState* T = H->train;
-    if (!T) return fail(H, SIRIUS_ERR_NOT_CONFIGURED, "sirius_cuda_train_init has not been called");
+    if (!train_ready(T)) return fail(H, SIRIUS_ERR_NOT_CONFIGURED, "sirius_cuda_train_init has not succeeded");
     CK(cudaSetDevice(H->device));
     double acc[4] = {0, 0, 0, 0};
     for (long long r0 = 0; r0 < n_rows; r0 += T->cfg.batch) {
@@ -2331,7 +2336,7 @@ int sirius_cuda_train_gradient(sirius_cuda_handle h, const float* d_features, co
     Handle* H = static_cast<Handle*>(h);
     if (!H || !d_features || !d_targets || !d_weights || !grad) return SIRIUS_ERR_INVALID_ARGUMENT;
     TrainState* T = H->train;
-    if (!T) return fail(H, SIRIUS_ERR_NOT_CONFIGURED, "sirius_cuda_train_init has not been called");
+    if (!train_ready(T)) return fail(H, SIRIUS_ERR_NOT_CONFIGURED, "sirius_cuda_train_init has not succeeded");
     if (n_rows <= 0 || n_rows % 128 != 0 || n_rows > T->cfg.batch)
         return fail(H, SIRIUS_ERR_INVALID_ARGUMENT, "n_rows must be a positive multiple of 128, at most the batch");
     CK(cudaSetDevice(H->device));
@@ -2357,7 +2362,7 @@ int sirius_cuda_train_params(sirius_cuda_handle h, float* params, int64_t* steps
     Handle* H = static_cast<Handle*>(h);
     if (!H || !params) return SIRIUS_ERR_INVALID_ARGUMENT;
     TrainState* T = H->train;
-    if (!T) return fail(H, SIRIUS_ERR_NOT_CONFIGURED, "sirius_cuda_train_init has not been called");
+    if (!T || !T->ready) return fail(H, SIRIUS_ERR_NOT_CONFIGURED, "sirius_cuda_train_init has not succeeded");
     CK(cudaSetDevice(H->device));
     long long st = 0;
     CK(cudaMemcpyAsync(params, T->params, surrogate::kParams * sizeof(float), cudaMemcpyDeviceToHost, H->stream));

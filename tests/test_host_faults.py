@@ -233,3 +233,38 @@ def test_training_rows_are_one_allocation(eng, fake):
     eng.train_init(weights(), abi.train_config(batch=256))
     assert fake.calls("cudaMalloc") == 0 and fake.device_bytes == grown
     gradient(eng)
+
+
+@pytest.mark.parametrize("first", [True, False])
+def test_training_whose_memory_ran_out_is_refused_until_it_is_made(eng, fake, first):
+    """An initialisation that ran out of memory leaves no state that a step, an evaluation or a gradient would run on."""
+    if not first:
+        eng.train_init(weights(), abi.train_config(batch=256))
+        gradient(eng)
+    nth = 0
+    while True:
+        nth += 1
+        fake.reset()
+        fake.fail("cudaMalloc", nth)
+        try:
+            eng.train_init(weights(), abi.train_config(batch=512 + 128 * nth))
+        except SiriusError as e:
+            assert e.code == abi.ERR_OUT_OF_MEMORY
+        else:
+            break
+        fake.reset()
+        x, t, w = (a.ctypes.data for a in training_set(2048))
+        calls = [lambda: gradient(eng), lambda: eng.train_steps(x, t, w, 2048, 1),
+                 lambda: eng.train_evaluate(x, t, w, 2048)]
+        if first:
+            calls.append(lambda: eng.train_params())
+        else:
+            eng.train_params()  # those of the initialisation before
+        for call in calls:
+            with pytest.raises(SiriusError) as r:
+                call()
+            assert r.value.code == abi.ERR_NOT_CONFIGURED
+        assert fake.launches("") == 0
+    assert nth == (9 if first else 2)
+    gradient(eng)
+    eng.train_params()
