@@ -610,6 +610,7 @@ struct HostOut {
 
 int fail(Handle* h, int code, const std::string& msg) {
     if (h) h->last_error = msg;
+    cudaGetLastError();  // reported here: the check of the next launch must not find it
     return code;
 }
 

@@ -268,3 +268,14 @@ def test_training_whose_memory_ran_out_is_refused_until_it_is_made(eng, fake, fi
     assert nth == (9 if first else 2)
     gradient(eng)
     eng.train_params()
+
+
+def test_an_error_is_reported_once(eng, fake):
+    """A call that ran out of memory is answered by that call, not by the next one's launch check."""
+    eng.surrogate_load(weights())
+    fake.fail("cudaMalloc", 1)
+    with pytest.raises(SiriusError) as r:
+        render(eng)
+    assert r.value.code == abi.ERR_OUT_OF_MEMORY
+    infer(eng)
+    render(eng)
