@@ -2092,26 +2092,37 @@ int sirius_cuda_surrogate_load(sirius_cuda_handle h, const float* params, int64_
     CK(cudaSetDevice(H->device));
     std::vector<unsigned char> img(surrogate::kImageBytes);
     surrogate::pack_weights(params, img.data());
-    if (!H->d_surrogate) {
-        if (cudaMalloc((void**)&H->d_surrogate, surrogate::kImageBytes) != cudaSuccess)
+    // (kept by the handle once all of it is there: a first load that failed leaves no weights)
+    using Buffer = std::unique_ptr<unsigned char, cudaError_t (*)(void*)>;
+    Buffer w(nullptr, cudaFree), e(nullptr, cudaFree);
+    unsigned char* d_w = H->d_surrogate;
+    if (!d_w) {
+        void* p = nullptr;
+        if (cudaMalloc(&p, surrogate::kImageBytes) != cudaSuccess)
             return fail(H, SIRIUS_ERR_OUT_OF_MEMORY, "cudaMalloc surrogate weights");
-        if (cudaMalloc((void**)&H->d_sur_err, 16 * sizeof(int)) != cudaSuccess)
+        w.reset(d_w = static_cast<unsigned char*>(p));
+        if (cudaMalloc(&p, 16 * sizeof(int)) != cudaSuccess)
             return fail(H, SIRIUS_ERR_OUT_OF_MEMORY, "cudaMalloc surrogate status");
-        CK(cudaMemsetAsync(H->d_sur_err, 0, 16 * sizeof(int), H->stream));
+        e.reset(static_cast<unsigned char*>(p));
+        CK(cudaMemsetAsync(p, 0, 16 * sizeof(int), H->stream));
         CK(cudaFuncSetAttribute(surrogate::mlp_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 surrogate::kPairSmBytes));
     }
-    CK(cudaMemcpyAsync(H->d_surrogate, img.data(), surrogate::kImageBytes, cudaMemcpyHostToDevice, H->stream));
+    CK(cudaMemcpyAsync(d_w, img.data(), surrogate::kImageBytes, cudaMemcpyHostToDevice, H->stream));
     CK(cudaStreamSynchronize(H->stream));
+    if (w) {
+        H->d_surrogate = w.release();
+        H->d_sur_err = reinterpret_cast<int*>(e.release());
+    }
     return SIRIUS_OK;
 }
 
-// launches the MLP on n feature rows (device buffers) on stream st
 // bound on any wait inside the MLP kernel: the configured watchdog (default 30 s)
 static unsigned long long surrogate_wait_ns(const Handle* H) {
     return (unsigned long long)(H->cfg.watchdog_ms > 0 ? H->cfg.watchdog_ms : 30000) * 1000000ull;
 }
 
+// launches the MLP on n feature rows (device buffers) on stream st
 static int surrogate_launch(Handle* H, const float* d_features, long long n, float* d_out, cudaStream_t st,
                             const unsigned* rows = nullptr) {
     if (!H->d_surrogate) return fail(H, SIRIUS_ERR_NOT_CONFIGURED, "no surrogate weights loaded");

@@ -279,3 +279,23 @@ def test_an_error_is_reported_once(eng, fake):
     assert r.value.code == abi.ERR_OUT_OF_MEMORY
     infer(eng)
     render(eng)
+
+
+@pytest.mark.parametrize("name,n", [("cudaMalloc", 1), ("cudaMalloc", 2), ("cudaMemsetAsync", 1),
+                                    ("cudaFuncSetAttribute", 1), ("cudaMemcpyAsync", 1), ("cudaStreamSynchronize", 1)])
+def test_weights_whose_load_failed_are_not_there(eng, fake, name, n):
+    """A first load that failed half-way leaves the network unloaded, and can be repeated."""
+    fake.reset()
+    fake.fail(name, n)
+    with pytest.raises(SiriusError):
+        eng.surrogate_load(weights())
+    for rows in (0, 300):
+        with pytest.raises(SiriusError) as r:
+            infer(eng, rows)
+        assert r.value.code == abi.ERR_NOT_CONFIGURED
+    features(eng)
+    assert fake.launches(MLP) == 0
+    eng.surrogate_load(weights())
+    infer(eng, 0)
+    infer(eng)
+    assert fake.launches(MLP) == 1
