@@ -634,6 +634,22 @@ int ensure(Handle* H, T*& ptr, size_t& cap, size_t count) {
     return SIRIUS_OK;
 }
 
+// The workspace of a call on host buffers (beams, metric, steps), kept for the next call while it
+// is at most kTmpKeep (a beam map of 1024^2 and less): a larger one is given back when the call ends.
+constexpr size_t kTmpKeep = size_t(64) << 20;
+struct TmpGuard {
+    Handle* H;
+    explicit TmpGuard(Handle* h) : H(h) {}
+    TmpGuard(const TmpGuard&) = delete;
+    TmpGuard& operator=(const TmpGuard&) = delete;
+    ~TmpGuard() {
+        if (H->tmp_cap <= kTmpKeep) return;
+        cudaFree(H->d_tmp);  // (waits for the device)
+        H->d_tmp = nullptr;
+        H->tmp_cap = 0;
+    }
+};
+
 double isco_host(double a_star) {
     const double a = std::min(std::fabs(a_star), 1.0);
     const double Z1 = 1 + std::cbrt(1 - a * a) * (std::cbrt(1 + a) + std::cbrt(1 - a));
@@ -1844,6 +1860,7 @@ int sirius_cuda_trace_beams(sirius_cuda_handle h, const sirius_frame* frames, in
     long long total = 0;
     int rc = upload_frames(H, frames, n_frames, &total);
     if (rc != SIRIUS_OK) return rc;
+    TmpGuard tmp(H);
     if ((rc = ensure(H, H->d_tmp, H->tmp_cap, size_t(total) * sizeof(sirius_beam_result))) != SIRIUS_OK) return rc;
     sirius_beam_result* d_out = reinterpret_cast<sirius_beam_result*>(H->d_tmp);
     BeamParams B{};
@@ -1967,6 +1984,7 @@ int sirius_cuda_metric_evaluate(sirius_cuda_handle h, const sirius_metric* metri
     int rc = validate_metric(H, *metric);
     if (rc != SIRIUS_OK) return rc;
     CK(cudaSetDevice(H->device));
+    TmpGuard tmp(H);
     if ((rc = ensure(H, H->d_tmp, H->tmp_cap, size_t(n) * 84 * sizeof(double))) != SIRIUS_OK) return rc;
     double* dp = reinterpret_cast<double*>(H->d_tmp);
     double *dgp = dp + 4 * size_t(n), *ddg = dgp + 16 * size_t(n);
@@ -1988,6 +2006,7 @@ int sirius_cuda_dp45_step(sirius_cuda_handle h, const sirius_metric* metric, dou
     int rc = validate_metric(H, *metric);
     if (rc != SIRIUS_OK) return rc;
     CK(cudaSetDevice(H->device));
+    TmpGuard tmp(H);
     if ((rc = ensure(H, H->d_tmp, H->tmp_cap, size_t(n) * (10 * sizeof(double) + sizeof(int)))) != SIRIUS_OK) return rc;
     double* ds = reinterpret_cast<double*>(H->d_tmp);
     double *dh = ds + 8 * size_t(n), *de = dh + n;

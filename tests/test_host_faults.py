@@ -299,3 +299,30 @@ def test_weights_whose_load_failed_are_not_there(eng, fake, name, n):
     infer(eng, 0)
     infer(eng)
     assert fake.launches(MLP) == 1
+
+
+def evaluate(eng, n):
+    eng.metric_evaluate(abi.make_metric(a=0.5), np.ones((n, 4)))
+
+
+def step(eng, n):
+    eng.dp45_step(abi.make_metric(a=0.5), np.ones((n, 8)), np.ones(n))
+
+
+def beams(eng, n):
+    eng.trace_beams([frame(n, 1)])
+
+
+@pytest.mark.parametrize("call,row", [(evaluate, 84 * 8), (step, 84), (beams, 32)])
+def test_a_large_calls_workspace_is_given_back(eng, fake, call, row):
+    """The calls on host buffers keep a small workspace from one call to the next, not a large one."""
+    call(eng, 1000)
+    before = fake.device_bytes
+    fake.reset()
+    call(eng, 1000)
+    assert fake.calls("cudaMalloc") == 0 and fake.device_bytes == before
+    large = (64 << 20) // row + 1000
+    call(eng, large)
+    assert fake.device_bytes <= before
+    call(eng, 1000)
+    assert fake.device_bytes <= before
