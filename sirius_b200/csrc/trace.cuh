@@ -13,6 +13,7 @@
 #include <stdint.h>
 
 #include "packed.cuh"
+#include "roots.cuh"
 #include "spacetime.cuh"
 
 #include <type_traits>
@@ -642,29 +643,6 @@ __device__ __forceinline__ float volume_step_cap_f(float r, float z, float vx, f
     const float H = hz * fminf(fmaxf(r, r_in), r_out);
     const float dist = fmaxf(fmaxf(r_in - r, r - r_out), fabsf(z) - float(kVolCutoff) * H);
     return fmaxf(0.5f * H, dist) * rsqrtf(fmaxf(vx * vx + vy * vy + vz * vz, 1e-6f));
-}
-
-// The zero in [0, 1] of the cubic Hermite interpolant of z over the accepted step
-// (z0 and z1 have opposite signs): Newton from the chord's zero, kept inside the
-// shrinking bracket (a step that leaves it bisects), to FP64 rounding. Four or five
-// iterations of nine dependent operations, where bisection to the same width takes 60.
-__device__ __forceinline__ double hermite_root(double z0, double z1, double dz0, double dz1, double h) {
-    const double m0 = h * dz0, m1 = h * dz1, d = z1 - z0;
-    const double c2 = 3.0 * d - 2.0 * m0 - m1, c3 = m0 + m1 - 2.0 * d;
-    double lo = 0.0, hi = 1.0, s = -z0 / d;
-#pragma unroll 1
-    for (int it = 0; it < 60; ++it) {
-        const double f = z0 + s * (m0 + s * (c2 + s * c3));
-        const double df = m0 + s * (2.0 * c2 + s * (3.0 * c3));
-        if ((f < 0.0) == (z0 < 0.0)) lo = s;
-        else hi = s;
-        double t = s - f / df;
-        if (!(t > lo && t < hi)) t = 0.5 * (lo + hi);
-        const double step = fabs(t - s);
-        s = t;
-        if (step < 1e-15) break;
-    }
-    return s;
 }
 
 // Keplerian emitter at BL radius rbl seen from the camera: g = (p.u_obs)/(p.u_em),
