@@ -828,7 +828,8 @@ FrameDev make_frame(const sirius_frame& f, const sirius_trace_config& c) {
 
 CfgDev make_cfg(const sirius_trace_config& c) {
     CfgDev d{};
-    d.atol = c.abs_tolerance; d.rtol = c.rel_tolerance; d.hmin = c.min_step; d.hmax = c.max_step;
+    // (a scale below 1e-300 has no reciprocal in the kernels' arithmetic)
+    d.atol = std::max(c.abs_tolerance, 1e-300); d.rtol = c.rel_tolerance; d.hmin = c.min_step; d.hmax = c.max_step;
     d.h0 = c.initial_step; d.safety = c.safety_factor; d.grow = c.step_grow_max; d.shrink = c.step_shrink_min;
     d.escape_r = c.escape_radius; d.decay = c.crossing_weight_decay;
     d.max_steps = c.max_steps; d.enable_disk = c.enable_disk; d.enable_vol = c.enable_volumetric;

@@ -4,6 +4,12 @@
 
 #include "dual.cuh"
 
+#ifdef __CUDACC__
+#define SIRIUS_DEVICE __device__
+#else
+#define SIRIUS_DEVICE
+#endif
+
 namespace sirius {
 
 // The zero in [0, 1] of the cubic Hermite interpolant of z over the accepted step
@@ -13,13 +19,13 @@ namespace sirius {
 // bracket: the iterate has just become one of the bracket's ends, and a correction that
 // rounds to zero would not lie inside. End slopes within 10 % of the chord's take 3.5 iterations in
 // the mean and at most 4, within a factor of 2 to 3 4.4 and at most 6.
-SIRIUS_HD __forceinline__ double hermite_root(double z0, double z1, double dz0, double dz1, double h,
+SIRIUS_DEVICE __forceinline__ double hermite_root(double z0, double z1, double dz0, double dz1, double h,
                                               int* iterations = nullptr) {
     const double m0 = h * dz0, m1 = h * dz1, d = z1 - z0;
     const double c2 = 3.0 * d - 2.0 * m0 - m1, c3 = m0 + m1 - 2.0 * d;
     double lo = 0.0, hi = 1.0, s = -z0 / d;
     int it = 0;
-#ifdef __CUDACC__
+#ifdef __CUDA_ARCH__
 #pragma unroll 1
 #endif
     while (it < 60) {
@@ -38,6 +44,33 @@ SIRIUS_HD __forceinline__ double hermite_root(double z0, double z1, double dz0, 
     }
     if (iterations) *iterations = it;
     return s;
+}
+
+// e^(-1/5) of e > 0: an FP32 estimate from the hardware logarithm and exponential
+// (1e-5 relative at worst), and two Newton steps of y -> y + y (1 - e y^5) / 5, whose
+// error goes from d to 3 d^2: FP64 rounding after the second (twelve FP64
+// operations, where pow takes more than a right-hand side). Above FLT_MAX, and at
+// infinity, the estimate is zero and stays so (the caller clamps the factor from below).
+SIRIUS_DEVICE __forceinline__ double inv_root5(double e) {
+#ifdef __CUDA_ARCH__
+    double y = double(exp2f(-0.2f * __log2f(float(e))));
+#else
+    double y = double(std::exp2(-0.2f * std::log2(float(e))));
+#endif
+    e = fmin(e, 1.7976931348623157e308);  // inf * 0 would be NaN
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+    for (int it = 0; it < 2; ++it) {
+        const double y2 = y * y;
+        y += 0.2 * y * (1.0 - e * y * (y2 * y2));
+    }
+    return y;
+}
+
+// The square root of a sum of squares, from rsqrt_: zero below 1e-280, infinity at infinity.
+SIRIUS_DEVICE __forceinline__ double root_of_sum(double s) {
+    return s * rsqrt_(fmin(fmax(s, 1e-280), 1.7976931348623157e308));
 }
 
 }  // namespace sirius

@@ -450,8 +450,7 @@ __device__ __forceinline__ double dp45_attempt_f64(const MetricDev& m, const Cfg
         const double s = h * (e[i] + D.E[6] * k7[i]) * rcp_(c.atol + c.rtol * fabs(xn[i]));
         en += s * s;
     }
-    en *= 0.25;
-    return en * rsqrt_(fmax(en, 1e-280));
+    return root_of_sum(0.25 * en);
 }
 
 template <class T, int FAM = kAnyFamily>
@@ -494,21 +493,6 @@ __device__ __forceinline__ void locate_equator_f32(const MetricDev& m, const Cfg
     const double dl = -xn[3] / double(k7[3]);
     xc1 = xn[1] + dl * double(k7[1]);
     xc2 = xn[2] + dl * double(k7[2]);
-}
-
-// e^(-1/5) of e > 0: an FP32 estimate from the hardware logarithm and exponential
-// (1e-5 relative at worst), and two Newton steps of y -> y + y (1 - e y^5) / 5, whose
-// error goes from d to 3 d^2: FP64 rounding after the second (twelve FP64
-// operations, where pow takes more than a right-hand side). An estimate that under-
-// or overflowed stays as it is (the caller clamps the factor).
-__device__ __forceinline__ double inv_root5(double e) {
-    double y = double(exp2f(-0.2f * __log2f(float(e))));
-#pragma unroll
-    for (int it = 0; it < 2; ++it) {
-        const double y2 = y * y;
-        y += 0.2 * y * (1.0 - e * y * (y2 * y2));
-    }
-    return y;
 }
 
 // Geodesic::computeOptimalStep (PHGD001A.cpp:471-483).

@@ -72,7 +72,33 @@ static void exact_crossings() {
     check(s >= 0 && s <= 1 && it <= 60, "crossing with steep ends", s, it);
 }
 
+// e^(-1/5) to a few ulps (two Newton steps leave 3 d^2 of an estimate good to d = 1e-5, then rounding of five products),
+// and a factor that never grows where the error is beyond FP32's range or infinite
+static void fifth_root() {
+    double off = 0;
+    for (int i = 0; i < 200000; ++i) {
+        const double e = std::exp(uniform(std::log(1e-15), std::log(1e38)));
+        off = std::fmax(off, std::fabs(double(inv_root5(e) * powl((long double)e, 0.2L) - 1)));
+    }
+    check(off <= 3e-10 * 3e-10 + 6 * 0x1p-53, "fifth root: relative error", off, 0);
+    for (double e : {1e39, 1e150, 1e300, 1.7976931348623157e308, HUGE_VAL}) {
+        const double y = inv_root5(e);
+        check(y >= 0 && y <= 1e-7, "fifth root of a huge error", y, e);
+        check(std::fmax(0.1, std::fmin(2.0, 0.9 * y)) == 0.1, "step factor of a huge error", y, e);
+    }
+    check(std::isnan(inv_root5(NAN)), "fifth root of NaN", inv_root5(NAN), 0);
+}
+
+static void root_of_sums() {
+    for (double s : {1e-279, 1e-30, 0.3, 2.0, 1e300, 1.7976931348623157e308})
+        check(std::fabs(root_of_sum(s) / std::sqrt(s) - 1) <= 3 * 0x1p-53, "root of a sum", root_of_sum(s), s);
+    check(root_of_sum(0.0) == 0 && root_of_sum(HUGE_VAL) == HUGE_VAL && std::isnan(root_of_sum(NAN)), "root of a sum",
+          root_of_sum(HUGE_VAL), root_of_sum(NAN));
+}
+
 int main() {
+    fifth_root();
+    root_of_sums();
     crossings(0.99, 1.01, 4, 3.5);
     crossings(0.9, 1.1, 5, 4.0);
     crossings(0.3, 2.0, 8, 5.0);
