@@ -36,13 +36,13 @@ namespace sirius {
 // third-order Householder step, e the seed's residual:
 //   1/x:        e = 1 - x y,    y <- y + y (e + e^2)
 //   1/sqrt(x):  e = 1 - x y^2,  y <- y + y e (1/2 + 3/8 e)
-// A seed good to 2^-20 leaves 2^-60, so the result is within an ulp or so, as the
-// CUDA functions' are; positive normal arguments only, so there is no
-// special-case branch beside each of the three per right-hand side (717 x 405 FP64
-// frame 5.78 -> 4.63 ms, 1024^2 mixed frame 20.3 -> 18.1 ms). Against 1/x and
-// 1/sqrt(x) in extended precision over e^-50..e^50 the largest relative errors are
-// 1.1e-16 and 1.4e-16 (the CUDA functions: 1.1e-16 both). A NaN or an infinite
-// argument gives NaN.
+// A seed good to 2^-20 leaves 2^-60, so a reciprocal is within 1.02 half-ulps and a reciprocal
+// root, whose x y is rounded too, within 1.5, with no special-case branch beside each of the
+// three per right-hand side (717 x 405 FP64 frame 5.78 -> 4.63 ms, 1024^2 mixed frame 20.3 ->
+// 18.1 ms). The largest relative errors over 1e-300..1e300 are 1.1e-16 and 1.4e-16 (the CUDA
+// functions': 1.1e-16 both). Arguments: normal numbers, for rcp_ of either sign, whose result is
+// normal too; zero, a subnormal or an infinite argument gives NaN, so callers clamp theirs
+// away from these where they can occur.
 __device__ __forceinline__ float rcp_(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
