@@ -422,7 +422,7 @@ __device__ __forceinline__ void inv_form(const MetricDev& m, const double x[4], 
     const double X = x[1], Y = x[2], Z = x[3];
     const double R2 = X * X + Y * Y + Z * Z;
     if (m.family == SIRIUS_METRIC_ALCUBIERRE) {
-        const double iR = rsqrt_(R2), Rr = R2 * iR;
+        const double iR = rsqrt_(fmax(R2, 1e-300)), Rr = R2 * iR;  // (the bubble's centre: r = 0, no direction)
         F.r = Rr;
         F.d[1] = X * iR; F.d[2] = Y * iR; F.d[3] = Z * iR;
         const D3<double> f = alc_f<double>(m, X, Y, Z);

@@ -24,9 +24,10 @@ def device(tmp_path_factory):
         pytest.skip("no nvcc to build the arrays' kernel with")
     lib = str(tmp_path_factory.mktemp("roots") / "device_roots.so")
     subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-shared", "-Xcompiler",
-                    "-fPIC", "-I", os.path.join(ROOT, "sirius_b200", "csrc"),
+                    "-fPIC", "-I", os.path.join(ROOT, "sirius_b200", "csrc"), "-I", os.path.join(ROOT, "include"),
                     os.path.join(ROOT, "tests", "cpp", "device_roots.cu"), "-o", lib], check=True)
     L = C.CDLL(lib)
+    L.device_warp_centre.argtypes = [C.c_double, C.c_void_p]
     L.device_apply.argtypes = [C.c_int, C.c_longlong, C.c_void_p, C.c_void_p]
 
     def apply(f, x):
@@ -34,6 +35,7 @@ def device(tmp_path_factory):
         y = np.empty_like(x)
         assert L.device_apply(f, x.size, x.ctypes.data, y.ctypes.data) == 0
         return y
+    apply.lib = L
     return apply
 
 
@@ -82,3 +84,19 @@ def test_root_of_a_sum(device):
     assert worst(device(5, x), np.sqrt(x.astype(np.longdouble))) <= 2.5 * U + 2.0 ** -57
     np.testing.assert_array_equal(device(5, [0.0, np.inf]), [0.0, np.inf])
     assert np.isnan(device(5, [np.nan])).all()
+
+
+@pytest.mark.parametrize("x", [0.0, 1e-160, 1e-100, -0.3, 1.0, 50.0])
+def test_warp_drive_at_its_centre(device, x):
+    """The radius and its direction at the bubble's centre and beside it: zero and none at the centre, where a projection
+    leaves the momentum as it is."""
+    y = np.full(10, np.nan)
+    assert device.lib.device_warp_centre(x, y.ctypes.data) == 0
+    assert np.isfinite(y).all()
+    np.testing.assert_allclose(y[0], abs(x) if abs(x) > 1e-150 else 0.0, rtol=4 * U, atol=1e-150)
+    if x == 0.0:
+        np.testing.assert_array_equal(y[1:5], 0)
+        np.testing.assert_array_equal(y[6:], [-1.0, 0.7, 0.3, -0.2])
+    elif abs(x) > 1e-150:
+        np.testing.assert_allclose(y[2], np.sign(x), rtol=4 * U)
+        np.testing.assert_array_equal(y[[1, 3, 4]], 0)
