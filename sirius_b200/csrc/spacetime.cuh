@@ -96,40 +96,9 @@ SIRIUS_HD __forceinline__ void ks_pieces(const MetricDev& m, T x, T y, T z, KSPi
     o.r = r;
 }
 
-template <class T>
-SIRIUS_HD __forceinline__ void ks_rhs(const MetricDev& m, const T x[4], const T p[4], T k[4], T f[4]) {
-    KSPieces<T> P;
-    ks_pieces(m, x[1], x[2], x[3], P);
-    const T H = P.H.v, l1 = P.l1.v, l2 = P.l2.v, l3 = P.l3.v;
-    // g^{-1} p = eta p - H l# (l# . p), l# = (-1, l1, l2, l3)
-    const T lp = -p[0] + l1 * p[1] + l2 * p[2] + l3 * p[3];
-    k[0] = -p[0] + H * lp;
-    k[1] = p[1] - H * l1 * lp;
-    k[2] = p[2] - H * l2 * lp;
-    k[3] = p[3] - H * l3 * lp;
-    if (m.has_lambda) {
-        const T c = T(m.lam3) * (x[1] * x[1] + x[2] * x[2] + x[3] * x[3]);
-        const T w0 = -T(1) - H, w1 = H * l1, w2 = H * l2, w3 = H * l3;
-        const T s = c * (w0 * p[0] + w1 * p[1] + w2 * p[2] + w3 * p[3]) * rcp_(T(1) + c * (T(1) + H));
-        k[0] += s * w0; k[1] += s * w1; k[2] += s * w2; k[3] += s * w3;
-    }
-    // dp_lambda = 1/2 dH (l.k)^2 + H (l.k)(dl.k) [- Lambda x_lambda (k^0)^2 / 3]
-    const T lk = k[0] + l1 * k[1] + l2 * k[2] + l3 * k[3];
-    f[0] = T(0);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const T dlk = P.l1.d[i] * k[1] + P.l2.d[i] * k[2] + P.l3.d[i] * k[3];
-        f[i + 1] = lk * (T(0.5) * P.H.d[i] * lk + H * dlk);
-    }
-    if (m.has_lambda) {
-        const T q = T(m.lam3) * k[0] * k[0];
-        f[1] -= q * x[1]; f[2] -= q * x[2]; f[3] -= q * x[3];
-    }
-}
-
-// The same right-hand side with the forward-mode tangents of ks_pieces
-// propagated term by term: the coordinate seeds dx = (1, 0, 0), ... have zero
-// components, and an IEEE product with a zero cannot be dropped at compile time
+// The Kerr-Schild right-hand side k = g^{-1} p, f = dp / dlambda with the forward-mode
+// tangents of ks_pieces propagated term by term: the coordinate seeds dx = (1, 0, 0), ... have
+// zero components, and an IEEE product with a zero cannot be dropped at compile time
 // (inf * 0 is NaN), so the generic dual arithmetic pays for every one of them.
 // Here only the non-zero terms are formed:
 //   dr  = (r x, r y, z (r^2 + a^2) / r) / sqrt(disc)

@@ -81,14 +81,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase, unsigned
     return true;
 }
 
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     dst),
-                 "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
-}
-
 // 2-D tiled tensor copy (TMA) from global to this CTA's shared memory, no
 // multicast; tmap is the address of a CUtensorMap in kernel-parameter or global
 // memory, (x, y) the box's first element (x the innermost, in elements). The
@@ -158,13 +150,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ float silu(float x) {
-    float t;
-    asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.5f * x));
-    return 0.5f * x * (1.f + t);
-}
-
-// silu of two values plus a bias each, packed FP32 arithmetic, the operations of silu()
+// SiLU x (1 + tanh(x / 2)) / 2 of two values plus a bias each, packed FP32 arithmetic, one MUFU op each
 __device__ __forceinline__ float2 silu_bias2(float2 v, float2 bias) {
     const float2 u = __fmul2_rn(__fadd2_rn(v, bias), make_float2(0.5f, 0.5f));
     float2 t;
