@@ -30,7 +30,7 @@ std::set<Stream*> streams;
 std::set<Event*> events;
 Stream legacy;
 std::string hook_kernel;
-int hook_arg = 0, hook_value = 0, sync_ms = 0;
+int hook_arg = 0, hook_value = 0, sync_ms = 0, major_version = 10;
 dim3 push_grid, push_block;
 size_t push_shmem = 0;
 cudaStream_t push_stream = nullptr;
@@ -70,6 +70,7 @@ void fake_reset() {
     failing.clear();
     hook_kernel.clear();
     sync_ms = 0;
+    major_version = 10;
     last = cudaSuccess;
 }
 void fake_fail(const char* name, long nth, int error) { failing[name] = {nth, cudaError_t(error)}; }
@@ -80,6 +81,7 @@ void fake_hook(const char* name, int arg, int value) {
     hook_value = value;
 }
 void fake_sync_ms(int ms) { sync_ms = ms; }  // how long a wait for a stream takes
+void fake_major(int v) { major_version = v; }
 long fake_calls(const char* name) { return calls.count(name) ? calls[name] : 0; }
 long fake_launches(const char* part) {
     long n = 0;
@@ -158,9 +160,15 @@ cudaError_t cudaSetDevice(int) {
     return cudaSuccess;
 }
 cudaError_t cudaGetDeviceProperties_v2(cudaDeviceProp* p, int) {
+    ENTER("cudaGetDeviceProperties");
     std::memset(p, 0, sizeof(*p));
-    p->major = 10;
+    p->major = major_version;
     p->multiProcessorCount = 148;
+    return cudaSuccess;
+}
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
+    ENTER("cudaDeviceGetAttribute");
+    *v = a == cudaDevAttrComputeCapabilityMajor ? major_version : a == cudaDevAttrMultiProcessorCount ? 148 : 0;
     return cudaSuccess;
 }
 cudaError_t cudaDeviceGetStreamPriorityRange(int* least, int* greatest) {

@@ -46,6 +46,10 @@ class Fake:
     def sync_ms(self, ms):
         self.lib.fake_sync_ms(ms)
 
+    def major(self, version):
+        """The device's compute capability, first number."""
+        self.lib.fake_major(version)
+
     def wait(self):
         """As a caller that waits for its own (the legacy default) stream."""
         self.lib.cudaStreamSynchronize(None)

@@ -326,3 +326,21 @@ def test_a_large_calls_workspace_is_given_back(eng, fake, call, row):
     assert fake.device_bytes <= before
     call(eng, 1000)
     assert fake.device_bytes <= before
+
+
+def test_a_handle_asks_for_the_attributes_it_needs(library, fake):
+    """A new handle does not query the whole property record; a device before compute capability 10 is refused."""
+    lib = load_library(library)
+    e = Engine(0, lib=lib)
+    assert fake.calls("cudaGetDeviceProperties") == 0
+    e.close()
+    fake.major(9)
+    with pytest.raises(SiriusError) as r:
+        Engine(0, lib=lib)
+    assert r.value.code == abi.ERR_UNSUPPORTED
+    fake.major(10)
+    for n in (1, 2):
+        fake.fail("cudaDeviceGetAttribute", n, fake_cuda.INVALID_VALUE)
+        with pytest.raises(SiriusError) as r:
+            Engine(0, lib=lib)
+        assert r.value.code == abi.ERR_CUDA
