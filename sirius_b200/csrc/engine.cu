@@ -913,6 +913,7 @@ struct PieceGuard {
         if (!armed) return;
         for (auto& q : H->piece_stream)
             if (q) cudaStreamSynchronize(q);
+        cudaGetLastError();  // (the call has its error)
     }
 };
 
@@ -2209,6 +2210,7 @@ struct SurrogateCall {
         cudaStreamSynchronize(st);
         for (auto& q : H->sur_stream)
             if (q) cudaStreamSynchronize(q);
+        cudaGetLastError();  // (the call has its error)
     }
 };
 

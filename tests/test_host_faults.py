@@ -344,3 +344,28 @@ def test_a_handle_asks_for_the_attributes_it_needs(library, fake):
         with pytest.raises(SiriusError) as r:
             Engine(0, lib=lib)
         assert r.value.code == abi.ERR_CUDA
+
+
+def test_waits_of_an_error_exit_leave_no_error_behind(eng, fake):
+    """Where the wait of an error exit fails as well, the call's own error is reported and the next call runs."""
+    import ctypes
+    eng.configure(abi.default_config(precision=abi.PRECISION_MIXED))
+    eng.surrogate_load(weights())
+    render(eng)
+    arr, k, n = batch()
+    img = np.zeros(n, np.float32)
+
+    def trace():
+        eng.trace_frames_device(ctypes.addressof(arr), k, n, None, img.ctypes.data, None, None)
+
+    trace()
+    for call, name, nth in ((render, "cudaStreamWaitEvent", 3), (lambda e: trace(), "cudaStreamWaitEvent", 2)):
+        fake.reset()
+        fake.fail(name, nth, fake_cuda.INVALID_VALUE)
+        fake.fail("cudaStreamSynchronize", 1, fake_cuda.NOT_SUPPORTED)
+        with pytest.raises(SiriusError):
+            call(eng)
+        assert fake.calls("cudaStreamSynchronize") >= 1
+        infer(eng)
+        render(eng)
+        trace()
