@@ -1013,9 +1013,12 @@ int launch_trace(Handle* H, int n_frames, long long total, sirius_ray_result* d_
                                 int(shmem_launch)));
     // a one-frame launch of camera rays traces 8 x 4 pixel tiles per warp (tile_ray:
     // blocks of 32, 64 and 128 threads cover 8 x 4, 16 x 4 and 16 x 8 pixels; tiles
-    // at the right and bottom edges are cut by the frame)
+    // at the right and bottom edges are cut by the frame). The one-frame forms of the
+    // kernels read the tile, and the pieces' first block, from the launch: the Kerr-Schild
+    // ones; a launch of another family takes consecutive rays in one piece.
     const int tile_x = block >= 64 ? 16 : 8, tile_y = block == 128 ? 8 : 4;
-    P.tiled = (n_frames == 1 && !d_list && !d_rays && !P.persistent && !pair && H->frame0.ray_offset == 0 &&
+    P.tiled = (n_frames == 1 && n_fams == 1 && fams[0] == SIRIUS_METRIC_KERR_SCHILD && !d_list && !d_rays &&
+               !P.persistent && !pair && H->frame0.ray_offset == 0 &&
                H->frame0.width > 0 && total == H->frame0.n_rays && total % H->frame0.width == 0)
                   ? 1 : 0;
     const long long tiled_blocks =
