@@ -62,8 +62,8 @@ __device__ __forceinline__ double rcp_(double x) {
 __device__ __forceinline__ double rsqrt_(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x * y, y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
+    const double e = fma(-__dmul_rn(x, y), y, 1.0);
+    return fma(__dmul_rn(y, e), fma(0.375, e, 0.5), y);
 }
 __device__ __forceinline__ float sqrt_(float x) { return sqrtf(x); }
 __device__ __forceinline__ double sqrt_(double x) { return sqrt(x); }
@@ -99,6 +99,21 @@ SIRIUS_HD __forceinline__ bool tanh_is_one(float x) { return x > 9.4f; }
 SIRIUS_HD __forceinline__ bool tanh_is_one(double x) { return x > 19.5; }
 template <class T>
 SIRIUS_HD __forceinline__ bool tanh_is_one(T) { return false; }  // (an operation count takes the general path)
+
+// a b + c in one rounding, and a product that no sum absorbs. Where a product meets a sum the
+// compiler may fuse either or neither, by what surrounds it, and the kernels of one-frame
+// launches and of batches (the same source, the metric in the parameter bank or in memory) then
+// differ in last bits. The arithmetic of the FP64 and symplectic paths leaves it no choice.
+template <class A, class B, class C>
+SIRIUS_HD __forceinline__ auto fma_(A a, B b, C c) { return a * b + c; }
+template <class A, class B>
+SIRIUS_HD __forceinline__ auto mul_(A a, B b) { return a * b; }
+#ifdef __CUDACC__
+__device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double mul_(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_(float a, float b) { return __fmul_rn(a, b); }
+#endif
 
 // The type of a function's constants when its variables are of type T.
 template <class T>

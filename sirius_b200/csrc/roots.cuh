@@ -21,8 +21,8 @@ namespace sirius {
 // the mean and at most 4, within a factor of 2 to 3 4.4 and at most 6.
 SIRIUS_DEVICE __forceinline__ double hermite_root(double z0, double z1, double dz0, double dz1, double h,
                                               int* iterations = nullptr) {
-    const double m0 = h * dz0, m1 = h * dz1, d = z1 - z0;
-    const double c2 = 3.0 * d - 2.0 * m0 - m1, c3 = m0 + m1 - 2.0 * d;
+    const double m0 = mul_(h, dz0), m1 = mul_(h, dz1), d = z1 - z0;
+    const double c2 = fma_(3.0, d, fma_(-2.0, m0, -m1)), c3 = fma_(-2.0, d, m0 + m1);
     double lo = 0.0, hi = 1.0, s = -z0 / d;
     int it = 0;
 #ifdef __CUDA_ARCH__
@@ -30,8 +30,8 @@ SIRIUS_DEVICE __forceinline__ double hermite_root(double z0, double z1, double d
 #endif
     while (it < 60) {
         ++it;
-        const double f = z0 + s * (m0 + s * (c2 + s * c3));
-        const double df = m0 + s * (2.0 * c2 + s * (3.0 * c3));
+        const double f = fma_(s, fma_(s, fma_(s, c3, c2), m0), z0);
+        const double df = fma_(s, fma_(s, mul_(3.0, c3), mul_(2.0, c2)), m0);
         const double t = s - f / df;
         if (fabs(t - s) < 1e-15) {
             s = t;
@@ -62,8 +62,8 @@ SIRIUS_DEVICE __forceinline__ double inv_root5(double e) {
 #pragma unroll
 #endif
     for (int it = 0; it < 2; ++it) {
-        const double y2 = y * y;
-        y += 0.2 * y * (1.0 - e * y * (y2 * y2));
+        const double y2 = mul_(y, y);
+        y = fma_(mul_(0.2, y), fma_(-mul_(e, y), mul_(y2, y2), 1.0), y);
     }
     return y;
 }
@@ -71,7 +71,7 @@ SIRIUS_DEVICE __forceinline__ double inv_root5(double e) {
 // The square root of a sum of squares, from rsqrt_ (2.2e-16): below 1e-280 at most 1e-140, infinity
 // at infinity.
 SIRIUS_DEVICE __forceinline__ double root_of_sum(double s) {
-    return s * rsqrt_(fmin(fmax(s, 1e-280), 1.7976931348623157e308));
+    return mul_(s, rsqrt_(fmin(fmax(s, 1e-280), 1.7976931348623157e308)));
 }
 
 }  // namespace sirius

@@ -197,43 +197,46 @@ template <class T>
 SIRIUS_HD __forceinline__ void ks_geom(const MetricDev& m, T X, T Y, T Z, KSGeom<T>& G) {
     using C = typename scalar_of<T>::type;
     const C a = cst<C>(m.a, m.fa), a2 = cst<C>(m.a2, m.fa2), M2 = cst<C>(2.0 * m.M, m.fM2);
-    const T zz = Z * Z;
-    const T R2 = X * X + Y * Y + zz;
+    const T zz = mul_(Z, Z);
+    const T R2 = fma_(X, X, fma_(Y, Y, zz));
     const T Rm2 = R2 - a2;
-    const T disc = tmax(Rm2 * Rm2 + C(4) * a2 * zz, C(1e-20));
+    const T a2zz = mul_(a2, zz);
+    const T disc = tmax(fma_(Rm2, Rm2, mul_(C(4), a2zz)), C(1e-20));
     const T isd = rsqrt_(disc);
-    const T r2 = tmax((Rm2 + disc * isd) * C(0.5), C(1e-10));
+    const T r2 = tmax(mul_(fma_(disc, isd, Rm2), C(0.5)), C(1e-10));
     const T ir = rsqrt_(r2);
-    const T r = r2 * ir;
+    const T r = mul_(r2, ir);
     const T den = r2 + a2;
     const T iden = rcp_(den);
-    const T q = M2 * r - cst<C>(m.Q2, m.fQ2);
+    const T q = fma_(M2, r, -cst<C>(m.Q2, m.fQ2));
     G.X = X; G.Y = Y; G.Z = Z; G.r = r; G.ir = ir; G.isd = isd; G.iden = iden; G.den = den;
-    G.l1 = (r * X + a * Y) * iden;
-    G.l2 = (r * Y - a * X) * iden;
-    G.l3 = Z * ir;
-    G.H = q * isd;
-    G.w = (M2 + C(2) * q * ir - C(4) * G.H * r) * isd;
-    G.hz = a2 * G.l3 * isd;
-    G.c = m.has_lambda ? cst<C>(m.lam3, m.flam3) * R2 : T(0);
+    G.l1 = mul_(fma_(r, X, mul_(a, Y)), iden);
+    G.l2 = mul_(fma_(r, Y, mul_(-a, X)), iden);
+    G.l3 = mul_(Z, ir);
+    G.H = mul_(q, isd);
+    G.w = mul_(fma_(mul_(C(2), q), ir, fma_(mul_(C(-4), G.H), r, M2)), isd);
+    G.hz = mul_(mul_(a2, G.l3), isd);
+    G.c = T(0);
+    if (m.has_lambda) G.c = mul_(cst<C>(m.lam3, m.flam3), R2);
 }
 
 // k = g^{-1} p = eta p - H l# (l# . p), l# = (-1, l1, l2, l3); lk = l . k
 template <class T>
 SIRIUS_HD __forceinline__ void ks_velocity(const MetricDev& m, const KSGeom<T>& G, const T p[4], T k[4], T& lk) {
     using C = typename scalar_of<T>::type;
-    const T lp = -p[0] + G.l1 * p[1] + G.l2 * p[2] + G.l3 * p[3];
-    const T Hlp = G.H * lp;
-    k[0] = -p[0] + Hlp;
-    k[1] = p[1] - G.l1 * Hlp;
-    k[2] = p[2] - G.l2 * Hlp;
-    k[3] = p[3] - G.l3 * Hlp;
+    const T lp = fma_(G.l3, p[3], fma_(G.l2, p[2], fma_(G.l1, p[1], -p[0])));
+    const T Hlp = mul_(G.H, lp);
+    k[0] = Hlp - p[0];
+    k[1] = fma_(-G.l1, Hlp, p[1]);
+    k[2] = fma_(-G.l2, Hlp, p[2]);
+    k[3] = fma_(-G.l3, Hlp, p[3]);
     lk = lp;
     if (m.has_lambda) {
-        const T w0 = -C(1) - G.H, w1 = G.H * G.l1, w2 = G.H * G.l2, w3 = G.H * G.l3;
-        const T s = G.c * (w0 * p[0] + w1 * p[1] + w2 * p[2] + w3 * p[3]) * rcp_(C(1) + G.c * (C(1) + G.H));
-        k[0] += s * w0; k[1] += s * w1; k[2] += s * w2; k[3] += s * w3;
-        lk = k[0] + G.l1 * k[1] + G.l2 * k[2] + G.l3 * k[3];
+        const T w0 = -C(1) - G.H, w1 = mul_(G.H, G.l1), w2 = mul_(G.H, G.l2), w3 = mul_(G.H, G.l3);
+        const T wp = fma_(w3, p[3], fma_(w2, p[2], fma_(w1, p[1], mul_(w0, p[0]))));
+        const T s = mul_(mul_(G.c, wp), rcp_(fma_(G.c, C(1) + G.H, C(1))));
+        k[0] = fma_(s, w0, k[0]); k[1] = fma_(s, w1, k[1]); k[2] = fma_(s, w2, k[2]); k[3] = fma_(s, w3, k[3]);
+        lk = fma_(G.l3, k[3], fma_(G.l2, k[2], fma_(G.l1, k[1], k[0])));
     }
 }
 
@@ -242,17 +245,18 @@ template <class T>
 SIRIUS_HD __forceinline__ void ks_force(const MetricDev& m, const KSGeom<T>& G, const T k[4], T lk, T f[4]) {
     using C = typename scalar_of<T>::type;
     const C a = cst<C>(m.a, m.fa);
-    const T S = (G.X * k[1] + G.Y * k[2] - C(2) * G.r * (G.l1 * k[1] + G.l2 * k[2])) * G.iden - k[3] * G.l3 * G.ir;
-    const T Hlk = G.H * lk, e = Hlk * G.iden;
-    const T g = lk * (C(0.5) * G.w * lk + G.H * S) * G.isd;
-    const T gr = g * G.r;
+    const T xk = fma_(G.X, k[1], mul_(G.Y, k[2])), l12 = fma_(G.l1, k[1], mul_(G.l2, k[2]));
+    const T S = fma_(fma_(mul_(C(-2), G.r), l12, xk), G.iden, mul_(mul_(-k[3], G.l3), G.ir));
+    const T Hlk = mul_(G.H, lk), e = mul_(Hlk, G.iden);
+    const T g = mul_(mul_(lk, fma_(mul_(C(0.5), G.w), lk, mul_(G.H, S))), G.isd);
+    const T gr = mul_(g, G.r);
     f[0] = T(0);
-    f[1] = gr * G.X + e * (G.r * k[1] - a * k[2]);
-    f[2] = gr * G.Y + e * (a * k[1] + G.r * k[2]);
-    f[3] = G.ir * (g * G.den * G.Z + Hlk * (k[3] - G.hz * lk));
+    f[1] = fma_(gr, G.X, mul_(e, fma_(G.r, k[1], mul_(-a, k[2]))));
+    f[2] = fma_(gr, G.Y, mul_(e, fma_(a, k[1], mul_(G.r, k[2]))));
+    f[3] = mul_(G.ir, fma_(mul_(g, G.den), G.Z, mul_(Hlk, fma_(-G.hz, lk, k[3]))));
     if (m.has_lambda) {  // - Lambda x_i (k^0)^2 / 3
-        const T qq = cst<C>(m.lam3, m.flam3) * k[0] * k[0];
-        f[1] -= qq * G.X; f[2] -= qq * G.Y; f[3] -= qq * G.Z;
+        const T qq = mul_(cst<C>(m.lam3, m.flam3), mul_(k[0], k[0]));
+        f[1] = fma_(-qq, G.X, f[1]); f[2] = fma_(-qq, G.Y, f[2]); f[3] = fma_(-qq, G.Z, f[3]);
     }
 }
 
@@ -384,57 +388,60 @@ __device__ __forceinline__ void inv_form(const MetricDev& m, const double x[4], 
         const D3<double> grr = mt_grr<double>(m, x[1]);
         F.r = x[1];
         F.d[1] = 1.0; F.d[2] = 0.0; F.d[3] = 0.0;
-        const double ir2 = rcp_(r * r);
-        F.diag[0] = rcp_(m.gtt_mt); F.diag[1] = rcp_(grr.v); F.diag[2] = ir2; F.diag[3] = ir2 * rcp_(s2);
+        const double ir2 = rcp_(mul_(r, r));
+        F.diag[0] = rcp_(m.gtt_mt); F.diag[1] = rcp_(grr.v); F.diag[2] = ir2; F.diag[3] = mul_(ir2, rcp_(s2));
         return;
     }
     const double X = x[1], Y = x[2], Z = x[3];
-    const double R2 = X * X + Y * Y + Z * Z;
+    const double zz = mul_(Z, Z), R2 = fma_(X, X, fma_(Y, Y, zz));
     if (m.family == SIRIUS_METRIC_ALCUBIERRE) {
-        const double iR = rsqrt_(fmax(R2, 1e-300)), Rr = R2 * iR;  // (the bubble's centre: r = 0, no direction)
+        const double iR = rsqrt_(fmax(R2, 1e-300)), Rr = mul_(R2, iR);  // (the bubble's centre: r = 0, no direction)
         F.r = Rr;
-        F.d[1] = X * iR; F.d[2] = Y * iR; F.d[3] = Z * iR;
+        F.d[1] = mul_(X, iR); F.d[2] = mul_(Y, iR); F.d[3] = mul_(Z, iR);
         const D3<double> f = alc_f<double>(m, X, Y, Z);
-        F.vf = m.vs * f.v;
+        F.vf = mul_(m.vs, f.v);
         return;
     }
     // (roots and reciprocals as in ks_rhs_closed: H = (2 M r - Q^2) / sd)
-    const double a2 = m.a2, Rm2 = R2 - a2;
-    const double disc = fmax(Rm2 * Rm2 + 4.0 * a2 * Z * Z, 1e-20);
+    const double a2 = m.a2, Rm2 = R2 - a2, a2zz = mul_(a2, zz);
+    const double disc = fmax(fma_(Rm2, Rm2, mul_(4.0, a2zz)), 1e-20);
     const double isd = rsqrt_(disc);
-    const double r2 = fmax(0.5 * (Rm2 + disc * isd), 1e-10);
-    const double ir = rsqrt_(r2), r = r2 * ir;
+    const double r2 = fmax(mul_(0.5, fma_(disc, isd, Rm2)), 1e-10);
+    const double ir = rsqrt_(r2), r = mul_(r2, ir);
     const double den = r2 + a2, iden = rcp_(den);
+    const double q = fma_(2.0 * m.M, r, -m.Q2);
     F.r = r;
-    F.d[1] = r * X * isd; F.d[2] = r * Y * isd; F.d[3] = Z * den * ir * isd;
+    F.d[1] = mul_(mul_(r, X), isd); F.d[2] = mul_(mul_(r, Y), isd); F.d[3] = mul_(mul_(Z, den), mul_(ir, isd));
     F.l[0] = -1.0;  // l# = eta l
-    F.l[1] = (r * X + m.a * Y) * iden;
-    F.l[2] = (r * Y - m.a * X) * iden;
-    F.l[3] = Z * ir;
-    F.H = (2.0 * m.M * r - m.Q2) * isd;
-    F.w[0] = -1.0 - F.H; F.w[1] = F.H * F.l[1]; F.w[2] = F.H * F.l[2]; F.w[3] = F.H * F.l[3];
+    F.l[1] = mul_(fma_(r, X, mul_(m.a, Y)), iden);
+    F.l[2] = mul_(fma_(r, Y, mul_(-m.a, X)), iden);
+    F.l[3] = mul_(Z, ir);
+    F.H = mul_(q, isd);
+    F.w[0] = -1.0 - F.H; F.w[1] = mul_(F.H, F.l[1]); F.w[2] = mul_(F.H, F.l[2]); F.w[3] = mul_(F.H, F.l[3]);
     F.c = 0.0;
     F.sm = 0.0;
     if (m.has_lambda) {
-        F.c = m.lam3 * R2;
-        F.sm = F.c / (1.0 + F.c * (1.0 + F.H));
+        F.c = mul_(m.lam3, R2);
+        F.sm = F.c / fma_(F.c, 1.0 + F.H, 1.0);
     }
 }
 
 __device__ __forceinline__ double inv_apply(const MetricDev& m, const InvForm& F, const double u[4], const double v[4]) {
     if (m.family == SIRIUS_METRIC_MORRIS_THORNE)
-        return F.diag[0] * u[0] * v[0] + F.diag[1] * u[1] * v[1] + F.diag[2] * u[2] * v[2] + F.diag[3] * u[3] * v[3];
-    if (m.family == SIRIUS_METRIC_ALCUBIERRE)
-        return -u[0] * v[0] - F.vf * (u[0] * v[1] + u[1] * v[0]) + (1.0 - F.vf * F.vf) * u[1] * v[1] + u[2] * v[2] +
-               u[3] * v[3];
-    const double eta = -u[0] * v[0] + u[1] * v[1] + u[2] * v[2] + u[3] * v[3];
-    const double lu = F.l[0] * u[0] + F.l[1] * u[1] + F.l[2] * u[2] + F.l[3] * u[3];
-    const double lv = F.l[0] * v[0] + F.l[1] * v[1] + F.l[2] * v[2] + F.l[3] * v[3];
-    double s = eta - F.H * lu * lv;
+        return fma_(mul_(F.diag[3], u[3]), v[3],
+                    fma_(mul_(F.diag[2], u[2]), v[2], fma_(mul_(F.diag[1], u[1]), v[1], mul_(mul_(F.diag[0], u[0]), v[0]))));
+    if (m.family == SIRIUS_METRIC_ALCUBIERRE) {
+        const double cross = fma_(u[0], v[1], mul_(u[1], v[0])), g11 = fma_(-F.vf, F.vf, 1.0);
+        return fma_(u[3], v[3], fma_(u[2], v[2], fma_(mul_(g11, u[1]), v[1], fma_(-F.vf, cross, mul_(-u[0], v[0])))));
+    }
+    const double eta = fma_(u[3], v[3], fma_(u[2], v[2], fma_(u[1], v[1], mul_(-u[0], v[0]))));
+    const double lu = fma_(F.l[3], u[3], fma_(F.l[2], u[2], fma_(F.l[1], u[1], mul_(F.l[0], u[0]))));
+    const double lv = fma_(F.l[3], v[3], fma_(F.l[2], v[2], fma_(F.l[1], v[1], mul_(F.l[0], v[0]))));
+    double s = fma_(mul_(-F.H, lu), lv, eta);
     if (m.has_lambda) {
-        const double wu = F.w[0] * u[0] + F.w[1] * u[1] + F.w[2] * u[2] + F.w[3] * u[3];
-        const double wv = F.w[0] * v[0] + F.w[1] * v[1] + F.w[2] * v[2] + F.w[3] * v[3];
-        s += F.sm * wu * wv;
+        const double wu = fma_(F.w[3], u[3], fma_(F.w[2], u[2], fma_(F.w[1], u[1], mul_(F.w[0], u[0]))));
+        const double wv = fma_(F.w[3], v[3], fma_(F.w[2], v[2], fma_(F.w[1], v[1], mul_(F.w[0], v[0]))));
+        s = fma_(mul_(F.sm, wu), wv, s);
     }
     return s;
 }
@@ -447,14 +454,14 @@ __device__ __forceinline__ double project_null(const MetricDev& m, const InvForm
     const double A = inv_apply(m, F, F.d, F.d);
     const double B = 2.0 * inv_apply(m, F, p, F.d);
     const double C = inv_apply(m, F, p, p);
-    const double disc = B * B - 4.0 * A * C;
+    const double disc = fma_(B, B, mul_(mul_(-4.0, A), C));
     if (disc < 0.0 || fabs(A) < 1e-15) return C;
-    const double sq = disc * rsqrt_(fmax(disc, 1e-280));
-    const double q = -0.5 * (B + (B >= 0.0 ? sq : -sq));
+    const double sq = mul_(disc, rsqrt_(fmax(disc, 1e-280)));
+    const double q = mul_(-0.5, B + (B >= 0.0 ? sq : -sq));
     if (q == 0.0) return C;
-    const double alpha = C * rcp_(q);
+    const double alpha = mul_(C, rcp_(q));
 #pragma unroll
-    for (int i = 0; i < 4; ++i) p[i] += alpha * F.d[i];
+    for (int i = 0; i < 4; ++i) p[i] = fma_(alpha, F.d[i], p[i]);
     return C;
 }
 
@@ -475,37 +482,39 @@ __device__ __forceinline__ double project_null_ks(const MetricDev& m, const doub
     moved = false;
     const double X = x[1], Y = x[2], Z = x[3];
     const double a = m.a, a2 = m.a2;
-    const double R2 = X * X + Y * Y + Z * Z, Rm2 = R2 - a2;
-    const double disc2 = fmax(Rm2 * Rm2 + 4.0 * a2 * Z * Z, 1e-20);
+    const double zz = mul_(Z, Z), R2 = fma_(X, X, fma_(Y, Y, zz)), Rm2 = R2 - a2, a2zz = mul_(a2, zz);
+    const double disc2 = fmax(fma_(Rm2, Rm2, mul_(4.0, a2zz)), 1e-20);
     const double isd = rsqrt_(disc2);
-    const double r2 = fmax(0.5 * (Rm2 + disc2 * isd), 1e-10);
-    const double ir = rsqrt_(r2), r = r2 * ir;
+    const double r2 = fmax(mul_(0.5, fma_(disc2, isd, Rm2)), 1e-10);
+    const double ir = rsqrt_(r2), r = mul_(r2, ir);
     r_out = r;
     const double den = r2 + a2, iden = rcp_(den);
-    const double l1 = (r * X + a * Y) * iden, l2 = (r * Y - a * X) * iden, l3 = Z * ir;
-    const double H = (2.0 * m.M * r - m.Q2) * isd;
-    const double lp = -p[0] + l1 * p[1] + l2 * p[2] + l3 * p[3];
-    const double C = -p[0] * p[0] + p[1] * p[1] + p[2] * p[2] + p[3] * p[3] - H * lp * lp;
-    const T isdt = T(isd), rs = T(r) * isdt, dt = T(den) * isdt;
-    const T d1 = rs * T(X), d2 = rs * T(Y), d3 = T(Z) * dt * T(ir);
+    const double l1 = mul_(fma_(r, X, mul_(a, Y)), iden), l2 = mul_(fma_(r, Y, mul_(-a, X)), iden), l3 = mul_(Z, ir);
+    const double H = mul_(fma_(2.0 * m.M, r, -m.Q2), isd);
+    const double lp = fma_(l3, p[3], fma_(l2, p[2], fma_(l1, p[1], -p[0])));
+    const double pp = fma_(p[3], p[3], fma_(p[2], p[2], fma_(p[1], p[1], mul_(-p[0], p[0]))));
+    const double C = fma_(mul_(-H, lp), lp, pp);
+    const T isdt = T(isd), rs = mul_(T(r), isdt), dt = mul_(T(den), isdt);
+    const T d1 = mul_(rs, T(X)), d2 = mul_(rs, T(Y)), d3 = mul_(mul_(T(Z), dt), T(ir));
     const T p1 = T(p[1]), p2 = T(p[2]), p3 = T(p[3]);
     const T Ht = T(H);
     const T A = dt - Ht;
-    const T B = T(2) * (p1 * d1 + p2 * d2 + p3 * d3 - Ht * T(lp));
+    const T pd = fma_(p3, d3, fma_(p2, d2, mul_(p1, d1)));
+    const T B = mul_(T(2), fma_(-Ht, T(lp), pd));
     const T Ct = T(C);
-    const T disc = B * B - T(4) * A * Ct;
+    const T disc = fma_(B, B, mul_(mul_(T(-4), A), Ct));
     // (at the horizon A = 0, exactly so in FP32 for some rays: C / q needs no division by A)
     if (!(disc >= T(0)) || (sizeof(T) == sizeof(double) && fabs(A) < T(1e-15))) return C;
     T sq;
-    if constexpr (sizeof(T) == sizeof(double)) sq = disc * rsqrt_(fmax(disc, 1e-280));
+    if constexpr (sizeof(T) == sizeof(double)) sq = mul_(disc, rsqrt_(fmax(disc, 1e-280)));
     else sq = sqrtf(disc);
-    const T q = T(-0.5) * (B + (B >= T(0) ? sq : -sq));
+    const T q = mul_(T(-0.5), B + (B >= T(0) ? sq : -sq));
     if (q == T(0)) return C;
-    const T al = Ct * rcp_(q);
+    const T al = mul_(Ct, rcp_(q));
     const double alpha = double(al);
-    p[1] += alpha * double(d1);
-    p[2] += alpha * double(d2);
-    p[3] += alpha * double(d3);
+    p[1] = fma_(alpha, double(d1), p[1]);
+    p[2] = fma_(alpha, double(d2), p[2]);
+    p[3] = fma_(alpha, double(d3), p[3]);
     const float pm = fmaxf(fmaxf(fabsf(float(p[0])), fabsf(float(p1))), fmaxf(fabsf(float(p2)), fabsf(float(p3))));
     const float dm = fmaxf(fmaxf(fabsf(float(d1)), fabsf(float(d2))), fabsf(float(d3)));
     moved = fabsf(float(al)) * dm > (sizeof(T) == sizeof(double) ? 1e-10f : 1e-6f) * pm;

@@ -403,54 +403,54 @@ __device__ __forceinline__ double dp45_attempt_f64(const MetricDev& m, const Cfg
         double xs[4], ps[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            xs[i] = x[i] + h * sx[i];
-            ps[i] = i == 0 ? p[0] : p[i] + h * sx[4 + i];
+            xs[i] = fma_(h, sx[i], x[i]);
+            ps[i] = i == 0 ? p[0] : fma_(h, sx[4 + i], p[i]);
         }
         rhs<double, FAM>(m, xs, ps, kk, kk + 4);
     };
 #pragma unroll
-    for (int q = 0; q < 7; ++q) sx[C[q]] = D.A[0][0] * k1[C[q]];
+    for (int q = 0; q < 7; ++q) sx[C[q]] = mul_(D.A[0][0], k1[C[q]]);
     stage(k2);
 #pragma unroll
-    for (int q = 0; q < 7; ++q) sx[C[q]] = D.A[0][1] * k1[C[q]] + D.A[1][0] * k2[C[q]];
+    for (int q = 0; q < 7; ++q) sx[C[q]] = fma_(D.A[1][0], k2[C[q]], mul_(D.A[0][1], k1[C[q]]));
     stage(k3);
 #pragma unroll
     for (int q = 0; q < 7; ++q)
-        sx[C[q]] = D.A[0][2] * k1[C[q]] + D.A[1][1] * k2[C[q]] + D.A[2][0] * k3[C[q]];
+        sx[C[q]] = fma_(D.A[2][0], k3[C[q]], fma_(D.A[1][1], k2[C[q]], mul_(D.A[0][2], k1[C[q]])));
     stage(k4);
 #pragma unroll
     for (int q = 0; q < 7; ++q) {
         const int i = C[q];
-        sx[i] = D.A[0][3] * k1[i] + D.A[1][2] * k2[i] + D.A[2][1] * k3[i] + D.A[3][0] * k4[i];
-        a6[q] = D.A[0][4] * k1[i] + D.A[1][3] * k2[i] + D.A[2][2] * k3[i] + D.A[3][1] * k4[i];
-        b[q] = D.A[0][5] * k1[i] + D.A[2][3] * k3[i] + D.A[3][2] * k4[i];
-        if (i < 4) e[i] = D.E[0] * k1[i] + D.E[2] * k3[i] + D.E[3] * k4[i];
+        sx[i] = fma_(D.A[3][0], k4[i], fma_(D.A[2][1], k3[i], fma_(D.A[1][2], k2[i], mul_(D.A[0][3], k1[i]))));
+        a6[q] = fma_(D.A[3][1], k4[i], fma_(D.A[2][2], k3[i], fma_(D.A[1][3], k2[i], mul_(D.A[0][4], k1[i]))));
+        b[q] = fma_(D.A[3][2], k4[i], fma_(D.A[2][3], k3[i], mul_(D.A[0][5], k1[i])));
+        if (i < 4) e[i] = fma_(D.E[3], k4[i], fma_(D.E[2], k3[i], mul_(D.E[0], k1[i])));
     }
     stage(k2);  // k_5
 #pragma unroll
     for (int q = 0; q < 7; ++q) {
         const int i = C[q];
-        sx[i] = a6[q] + D.A[4][0] * k2[i];
-        b[q] += D.A[4][1] * k2[i];
-        if (i < 4) e[i] += D.E[4] * k2[i];
+        sx[i] = fma_(D.A[4][0], k2[i], a6[q]);
+        b[q] = fma_(D.A[4][1], k2[i], b[q]);
+        if (i < 4) e[i] = fma_(D.E[4], k2[i], e[i]);
     }
     stage(k3);  // k_6
 #pragma unroll
     for (int q = 0; q < 7; ++q) {
         const int i = C[q];
-        b[q] += D.A[5][0] * k3[i];
-        if (i < 4) e[i] += D.E[5] * k3[i];
-        (i < 4 ? xn[i] : pn[i - 4]) = (i < 4 ? x[i] : p[i - 4]) + h * b[q];
+        b[q] = fma_(D.A[5][0], k3[i], b[q]);
+        if (i < 4) e[i] = fma_(D.E[5], k3[i], e[i]);
+        (i < 4 ? xn[i] : pn[i - 4]) = fma_(h, b[q], i < 4 ? x[i] : p[i - 4]);
     }
     pn[0] = p[0];
     rhs<double, FAM>(m, xn, pn, k7, k7 + 4);
     double en = 0.0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const double s = h * (e[i] + D.E[6] * k7[i]) * rcp_(c.atol + c.rtol * fabs(xn[i]));
-        en += s * s;
+        const double s = mul_(mul_(h, fma_(D.E[6], k7[i], e[i])), rcp_(fma_(c.rtol, fabs(xn[i]), c.atol)));
+        en = fma_(s, s, en);
     }
-    return root_of_sum(0.25 * en);
+    return root_of_sum(mul_(0.25, en));
 }
 
 template <class T, int FAM = kAnyFamily>
@@ -498,9 +498,9 @@ __device__ __forceinline__ void locate_equator_f32(const MetricDev& m, const Cfg
 // Geodesic::computeOptimalStep (PHGD001A.cpp:471-483).
 __device__ __forceinline__ double optimal_step(double h, double err, const CfgDev& c) {
     if (err < 1e-15) return fmin(h * c.grow, c.hmax);
-    double fac = c.safety * inv_root5(err);
+    double fac = mul_(c.safety, inv_root5(err));
     fac = fmax(c.shrink, fmin(c.grow, fac));
-    return fmax(c.hmin, fmin(c.hmax, h * fac));
+    return fmax(c.hmin, fmin(c.hmax, mul_(h, fac)));
 }
 
 // ---------------------------------------------------------------------------
@@ -538,7 +538,7 @@ __device__ __forceinline__ void symplectic_step(const MetricDev& m, int order, d
             ks_force(m, G, k, lk, f);
 #pragma unroll
             for (int i = 1; i < 4; ++i) {
-                p[i] += hk * double(f[i]);
+                p[i] = fma_(hk, double(f[i]), p[i]);
                 P[i] = T(p[i]);
             }
         };
@@ -547,13 +547,13 @@ __device__ __forceinline__ void symplectic_step(const MetricDev& m, int order, d
         ks_geom(m, T(x[1]), T(x[2]), T(x[3]), G);
 #pragma unroll 1
         for (int s = 0; s < n; ++s) {
-            const double hs = kYoshida[row][s] * h;
-            kick(0.5 * hs);
+            const double hs = mul_(kYoshida[row][s], h), hk = mul_(0.5, hs);
+            kick(hk);
             ks_velocity(m, G, P, k, lk);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) x[i] += hs * double(k[i]);
+            for (int i = 0; i < 4; ++i) x[i] = fma_(hs, double(k[i]), x[i]);
             ks_geom(m, T(x[1]), T(x[2]), T(x[3]), G);
-            kick(0.5 * hs);
+            kick(hk);
         }
         return;
     }
@@ -579,10 +579,10 @@ __device__ __forceinline__ void symplectic_step(const MetricDev& m, int order, d
 
 // The Kerr-Schild radius r(x, y, z) (r^4 - (R^2 - a^2) r^2 - a^2 z^2 = 0), FP64.
 __device__ __forceinline__ double ks_radius(const MetricDev& m, const double x[4]) {
-    const double R2 = x[1] * x[1] + x[2] * x[2] + x[3] * x[3], Rm2 = R2 - m.a2;
-    const double disc = fmax(Rm2 * Rm2 + 4.0 * m.a2 * x[3] * x[3], 1e-20);
-    const double r2 = fmax(0.5 * (Rm2 + disc * rsqrt_(disc)), 1e-10);
-    return r2 * rsqrt_(r2);
+    const double zz = mul_(x[3], x[3]), Rm2 = fma_(x[1], x[1], fma_(x[2], x[2], zz)) - m.a2;
+    const double disc = fmax(fma_(Rm2, Rm2, mul_(4.0, mul_(m.a2, zz))), 1e-20);
+    const double r2 = fmax(mul_(0.5, fma_(disc, rsqrt_(disc), Rm2)), 1e-10);
+    return mul_(r2, rsqrt_(r2));
 }
 
 // Step control in FP32 for the mixed path (the factor needs a few digits only).
@@ -616,9 +616,9 @@ constexpr double kVolCutoff = 6.0;
 // distance to that region, so that no step jumps into its interior.
 __device__ __forceinline__ double volume_step_cap(double r, double z, double vx, double vy, double vz, double hz,
                                                   double r_in, double r_out) {
-    const double H = hz * fmin(fmax(r, r_in), r_out);
-    const double dist = fmax(fmax(r_in - r, r - r_out), fabs(z) - kVolCutoff * H);
-    return fmax(0.5 * H, dist) * rsqrt_(fmax(vx * vx + vy * vy + vz * vz, 1e-6));
+    const double H = mul_(hz, fmin(fmax(r, r_in), r_out));
+    const double dist = fmax(fmax(r_in - r, r - r_out), fma_(-kVolCutoff, H, fabs(z)));
+    return mul_(fmax(mul_(0.5, H), dist), rsqrt_(fmax(fma_(vx, vx, fma_(vy, vy, mul_(vz, vz))), 1e-6)));
 }
 
 // The same cap in FP32 for the mixed path (a step-size bound needs a few digits).
@@ -636,18 +636,19 @@ __device__ __forceinline__ float volume_step_cap_f(float r, float z, float vx, f
 template <class T>
 __device__ __forceinline__ T kepler_g(const MetricDev& m, T x, T y, T z, T rbl, T E, T Lz, T sqrt_m_gtt_cam) {
     const T a = cst<T>(m.a, m.fa), a2 = cst<T>(m.a2, m.fa2), sqrtM = cst<T>(m.sqrtM, m.fsqrtM);
-    const T r2 = rbl * rbl, iden = rcp_(r2 + a2);
-    const T l1 = (rbl * x + a * y) * iden, l2 = (rbl * y - a * x) * iden;
-    const T H = (cst<T>(2.0 * m.M, m.fM2) * rbl - cst<T>(m.Q2, m.fQ2)) * r2 * rcp_(r2 * r2 + a2 * z * z);
-    const T lxi = -y * l1 + x * l2;
-    T gtt = -T(1) + H;
-    if (m.has_lambda) gtt -= cst<T>(m.lam3, m.flam3) * (x * x + y * y + z * z);
-    const T gtp = H * lxi, gpp = x * x + y * y + H * lxi * lxi;
-    const T Om = sqrtM * rcp_(rbl * sqrtp_(rbl) + a * sqrtM);
-    const T n = -(gtt + T(2) * Om * gtp + Om * Om * gpp);
+    const T r2 = mul_(rbl, rbl), iden = rcp_(r2 + a2);
+    const T l1 = mul_(fma_(rbl, x, mul_(a, y)), iden), l2 = mul_(fma_(rbl, y, mul_(-a, x)), iden);
+    const T num = mul_(fma_(cst<T>(2.0 * m.M, m.fM2), rbl, -cst<T>(m.Q2, m.fQ2)), r2);
+    const T H = mul_(num, rcp_(fma_(r2, r2, mul_(mul_(a2, z), z))));
+    const T lxi = fma_(x, l2, mul_(-y, l1));
+    T gtt = H - T(1);
+    if (m.has_lambda) gtt = fma_(-cst<T>(m.lam3, m.flam3), fma_(x, x, fma_(y, y, mul_(z, z))), gtt);
+    const T gtp = mul_(H, lxi), gpp = fma_(gtp, lxi, fma_(x, x, mul_(y, y)));
+    const T Om = mul_(sqrtM, rcp_(fma_(rbl, sqrtp_(rbl), mul_(a, sqrtM))));
+    const T n = -fma_(mul_(Om, Om), gpp, fma_(mul_(T(2), Om), gtp, gtt));
     if (!(n > T(0))) return T(0);
     const T ut = rsqrt_(n);
-    const T den = sqrt_m_gtt_cam * ut * (T(1) - Om * Lz * rcp_(E));
+    const T den = mul_(mul_(sqrt_m_gtt_cam, ut), fma_(-Om, mul_(Lz, rcp_(E)), T(1)));
     return den > T(0) ? rcp_(den) : T(0);
 }
 

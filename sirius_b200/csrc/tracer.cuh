@@ -246,9 +246,9 @@ __device__ __forceinline__ void end_ray(const Params& P, const Ray<MIXED>& s, in
 }
 
 __device__ __forceinline__ float ks_r(const MetricDev& m, float x, float y, float z) {
-    const float a2 = m.fa2, R2 = x * x + y * y + z * z, Rm2 = R2 - a2;
-    const float sd = sqrtp_(fmaxf(Rm2 * Rm2 + 4.f * a2 * z * z, 1e-20f));
-    return sqrtp_(fmaxf(0.5f * (Rm2 + sd), 1e-10f));
+    const float a2 = m.fa2, zz = mul_(z, z), Rm2 = fma_(x, x, fma_(y, y, zz)) - a2;
+    const float disc = fmaxf(fma_(Rm2, Rm2, mul_(4.f, mul_(a2, zz))), 1e-20f);
+    return sqrtp_(fmaxf(mul_(0.5f, fma_(disc, rsqrt_(disc), Rm2)), 1e-10f));
 }
 
 // The step's cubic Hermite interpolant in powers of q in [0, 1] relative to the step's
@@ -263,17 +263,17 @@ struct StepCubic {
                                          double h) {
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            const T d = T(b[i + 1] - a[i + 1]), m1 = T(h) * T(k1[i + 1]);
+            const T d = T(b[i + 1] - a[i + 1]), m1 = mul_(T(h), T(k1[i + 1]));
             x0[i] = T(a[i + 1]);
-            m0[i] = T(h) * T(k0[i + 1]);
-            c2[i] = T(3) * d - T(2) * m0[i] - m1;
-            c3[i] = m0[i] + m1 - T(2) * d;
+            m0[i] = mul_(T(h), T(k0[i + 1]));
+            c2[i] = fma_(T(3), d, fma_(T(-2), m0[i], -m1));
+            c3[i] = fma_(T(-2), d, m0[i] + m1);
         }
     }
     __device__ __forceinline__ void at(T q, float& xs, float& ys, float& zs) const {
-        xs = float(x0[0] + q * (m0[0] + q * (c2[0] + q * c3[0])));
-        ys = float(x0[1] + q * (m0[1] + q * (c2[1] + q * c3[1])));
-        zs = float(x0[2] + q * (m0[2] + q * (c2[2] + q * c3[2])));
+        xs = float(fma_(q, fma_(q, fma_(q, c3[0], c2[0]), m0[0]), x0[0]));
+        ys = float(fma_(q, fma_(q, fma_(q, c3[1], c2[1]), m0[1]), x0[1]));
+        zs = float(fma_(q, fma_(q, fma_(q, c3[2], c2[2]), m0[2]), x0[2]));
     }
 };
 
@@ -299,7 +299,7 @@ __device__ __forceinline__ void volumetric_segment(const Params& P, const FrameD
     const CfgDev& c = P.c;
     const int nq = c.vol_sub < 1 ? 1 : (c.vol_sub > 4 ? 4 : c.vol_sub);
     const float E = float(-p[0]);
-    const float Lz = float(x1[1] * p[2] - x1[2] * p[1]);
+    const float Lz = float(fma_(x1[1], p[2], -mul_(x1[2], p[1])));
     const float nu_cam = E * rcp_(observer_factor<float>(F, E));
     const float iaoj = rcp_(c.fvol_aoj);
     const float rin = F.fdisk_in, rout = F.fdisk_out;
@@ -315,7 +315,7 @@ __device__ __forceinline__ void volumetric_segment(const Params& P, const FrameD
         double qa = 0.0, qb = 1.0, ga = double(r0) - edge, gb = double(r1) - edge;
         int side = 0;
         for (int it = 0; it < 3; ++it) {
-            const double q = (qa * gb - qb * ga) / (gb - ga);
+            const double q = fma_(qa, gb, -mul_(qb, ga)) / (gb - ga);
             float xs, ys, zs;
             point(q, xs, ys, zs);
             const double g = double(ks_r(F.m, xs, ys, zs)) - edge;
@@ -329,7 +329,7 @@ __device__ __forceinline__ void volumetric_segment(const Params& P, const FrameD
                 side = 1;
             }
         }
-        const double qe = (qa * gb - qb * ga) / (gb - ga);
+        const double qe = fma_(qa, gb, -mul_(qb, ga)) / (gb - ga);
         if (in0) fb = qe;
         else fa = qe;
     }
@@ -356,7 +356,7 @@ __device__ __forceinline__ void volumetric_segment(const Params& P, const FrameD
         dts = 0.f;
         Ss = 0.f;
         float xs, ys, zs;
-        point(fa + span * double(kGLx[nq - 1][s]), xs, ys, zs);
+        point(fma_(span, double(kGLx[nq - 1][s]), fa), xs, ys, zs);
         const float r = ks_r(F.m, xs, ys, zs);
         if (r < rin || r > rout) return;
         const float zr = zs * rcp_(c.fvol_hz * r);
@@ -594,8 +594,8 @@ __device__ __forceinline__ int advance(const Params& P, Ray<MIXED>& s, float& ma
         // does (h0 min(1, ((r - r_+)/r_+)^2), PHSI001A.h:260-263); always accepted
         double hs = c.symp_step;
         if (F.has_horizon) {
-            const double q = (s.r - F.r_plus) * rcp_(F.r_plus);
-            hs = fmax(c.hmin, hs * fmin(1.0, q * q));
+            const double q = mul_(s.r - F.r_plus, rcp_(F.r_plus));
+            hs = fmax(c.hmin, mul_(hs, fmin(1.0, mul_(q, q))));
         }
         s.h = hs;
 #pragma unroll
