@@ -74,6 +74,7 @@ struct BeamParams {
 };
 
 // f of a state and of its tangent: y = (x, p) and V in, k and dk out (8 components)
+template <bool RING>
 __device__ __forceinline__ void beam_rhs(const MetricDev& m, const double y[8], const double V[8], double f[8],
                                          double fV[8]) {
     D1<double> x[4], p[4], k[4], g[4];
@@ -82,7 +83,7 @@ __device__ __forceinline__ void beam_rhs(const MetricDev& m, const double y[8], 
         x[i] = D1<double>(y[i], V[i]);
         p[i] = D1<double>(y[4 + i], V[4 + i]);
     }
-    ks_rhs_closed(m, x, p, k, g);
+    ks_rhs_closed<RING>(m, x, p, k, g);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         f[i] = k[i].v; fV[i] = k[i].d;
@@ -100,7 +101,8 @@ __device__ __forceinline__ void beam_rhs(const MetricDev& m, const double y[8], 
 // seven stage derivatives of 24 components in local memory (120 x 68 beams to
 // R = 1000 M: 22.3 -> 3.1 ms; magnifications against the same steps with exact
 // tangents in 64 bits: both within the rounding of a float). The sums of the stages
-// are those of dp45_attempt_f64.
+// are those of dp45_attempt_f64. RING: the beams of the frames of class kClassRing, without it the others'.
+template <bool RING>
 __global__ void __launch_bounds__(64) beam_kernel(const __grid_constant__ BeamParams B) {
     const long long thread = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long idx = thread >> 1;
@@ -109,6 +111,7 @@ __global__ void __launch_bounds__(64) beam_kernel(const __grid_constant__ BeamPa
     const unsigned pair = 3u << (threadIdx.x & 30);
     const int fi = B.n_frames > 1 ? find_frame(B.frames, B.n_frames, idx) : 0;
     const FrameDev& F = B.frames[fi];
+    if ((F.cls == kClassRing) != RING) return;
     const CfgDev& c = B.c;
     const MetricDev m = F.m;
     const long long pix = idx - F.ray_offset;
@@ -132,7 +135,7 @@ __global__ void __launch_bounds__(64) beam_kernel(const __grid_constant__ BeamPa
     const DPTable& D = kDPd;
     double h = c.h0;
     double k1[8], j1[8];  // f of the ray and of its tangent at the current state
-    beam_rhs(m, y, V, k1, j1);
+    beam_rhs<RING>(m, y, V, k1, j1);
     int outcome = SIRIUS_MAX_STEPS, steps = 0;
     const unsigned long long t0 = globaltimer();
     double r_prev = ks_radius(m, y);
@@ -156,7 +159,7 @@ __global__ void __launch_bounds__(64) beam_kernel(const __grid_constant__ BeamPa
                 yn[C[q]] = y[C[q]] + h * sy[q];
                 Vn[C[q]] = V[C[q]] + h * sV[q];
             }
-            beam_rhs(m, yn, Vn, kk, jj);
+            beam_rhs<RING>(m, yn, Vn, kk, jj);
         };
 #pragma unroll
         for (int q = 0; q < 7; ++q) {

@@ -88,7 +88,7 @@ constexpr long long kPieceMinBlocks = 2048;
 TraceFn pick_kernel(bool mixed, int minb, int fam, bool symp, bool uni = false) {
     if (fam == SIRIUS_METRIC_KERR_SCHILD)
         return mixed ? pick_ks_mixed(minb, uni, symp) : pick_ks_fp64(minb, uni, symp);
-    return pick_family(mixed, fam);
+    return pick_family(mixed, fam, symp);
 }
 
 // ---------------------------------------------------------------------------
@@ -536,7 +536,7 @@ struct Handle {
     bool pending = false;
     cudaStream_t pending_stream = nullptr;
     long long pending_total = 0;
-    int family_mask = 0;  // bit f: a frame of the last upload is of metric family f
+    int family_mask = 0;  // bit f: a frame of the last upload is of class f (FrameDev::cls)
     FrameDev frame0{};    // the first frame of the last upload (a one-frame launch's parameter copy)
     std::vector<FrameDev> frames_host;  // the last upload's descriptors (multi-sample passes)
     std::vector<FrameDev> pass_frames_host;  // ... with each pass's sub-pixel offset
@@ -787,6 +787,9 @@ FrameDev make_frame(const sirius_frame& f, const sirius_trace_config& c) {
     const double rp = F.has_horizon ? m.M + std::sqrt(d) : -1.0;
     F.r_hor = F.has_horizon ? rp * c.horizon_factor : -1.0;
     F.r_plus = rp;
+    // (r is held at 1e-5; without mass and charge the metric is flat and both forms are zero there)
+    const bool ring = m.family == SIRIUS_METRIC_KERR_SCHILD && (m.M != 0.0 || m.Q != 0.0) && !(F.r_hor > 1e-3);
+    F.cls = ring ? kClassRing : m.family;
     // the radial-potential gate applies to Kerr-Newman frames (separable: no Lambda term)
     F.gate = (F.has_horizon && std::fabs(m.Lambda) <= 1e-15) ? 1 : 0;
     const double aM = std::clamp(a_star, -0.998, 0.998);
@@ -883,9 +886,6 @@ int validate_config(Handle* H, const sirius_trace_config& c) {
     return SIRIUS_OK;
 }
 
-// Launch the tracer over [0, total) of already-uploaded frames.
-
-
 // The streams of launches 1..n-1 and the events of n launches (copies: and of their copies to the
 // host); those a handle has not yet, so that a batch's first call makes one or two streams, where
 // a frame in pieces needs 7 and 17 events (about 0.7 ms).
@@ -917,6 +917,7 @@ struct PieceGuard {
     }
 };
 
+// Launch the tracer over [0, total) of already-uploaded frames.
 int launch_trace(Handle* H, int n_frames, long long total, sirius_ray_result* d_results, float* d_image,
                  float* d_spectra, const sirius_camera_ray* d_rays, cudaStream_t st, bool timed,
                  const LaunchScratch* scratch = nullptr, const unsigned* d_list = nullptr, bool flux_ready = false,
@@ -972,16 +973,16 @@ int launch_trace(Handle* H, int n_frames, long long total, sirius_ray_result* d_
                      : mixed_dp45             ? kDefaultMinBlocksMixed
                      : !mixed && !symp        ? kDefaultMinBlocksFp64
                                               : kDefaultMinBlocks;
-    // the families present: one family -> its specialised kernel; several ->
-    // one launch per family (each thread skips the rays of other families), so
-    // a ray's result never depends on what else shares the batch; the
-    // persistent queue serves every family from one generic kernel
-    int fams[3], n_fams = 0;
-    for (int f = 0; f < 3; ++f)
+    // the classes present: one -> its specialised kernel; several -> one launch per
+    // class (each thread skips the rays of others), so a ray's result never
+    // depends on what else shares the batch; the persistent queue serves every
+    // class from one generic kernel
+    int fams[4], n_fams = 0;
+    for (int f = 0; f < 4; ++f)
         if (H->family_mask & (1 << f)) fams[n_fams++] = f;
     P.family = -1;
-    TraceFn launch_fn[3];
-    int launch_family[3], n_launches = 0;
+    TraceFn launch_fn[4];
+    int launch_family[4], n_launches = 0;
     if (n_fams == 1) {
         launch_fn[0] = pick_kernel(mixed, minb, fams[0], symp, n_frames == 1);
         launch_family[0] = -1;
@@ -1013,12 +1014,9 @@ int launch_trace(Handle* H, int n_frames, long long total, sirius_ray_result* d_
                                 int(shmem_launch)));
     // a one-frame launch of camera rays traces 8 x 4 pixel tiles per warp (tile_ray:
     // blocks of 32, 64 and 128 threads cover 8 x 4, 16 x 4 and 16 x 8 pixels; tiles
-    // at the right and bottom edges are cut by the frame). The one-frame forms of the
-    // kernels read the tile, and the pieces' first block, from the launch: the Kerr-Schild
-    // ones; a launch of another family takes consecutive rays in one piece.
+    // at the right and bottom edges are cut by the frame)
     const int tile_x = block >= 64 ? 16 : 8, tile_y = block == 128 ? 8 : 4;
-    P.tiled = (n_frames == 1 && n_fams == 1 && fams[0] == SIRIUS_METRIC_KERR_SCHILD && !d_list && !d_rays &&
-               !P.persistent && !pair && H->frame0.ray_offset == 0 &&
+    P.tiled = (n_frames == 1 && !d_list && !d_rays && !P.persistent && !pair && H->frame0.ray_offset == 0 &&
                H->frame0.width > 0 && total == H->frame0.n_rays && total % H->frame0.width == 0)
                   ? 1 : 0;
     const long long tiled_blocks =
@@ -1042,7 +1040,7 @@ int launch_trace(Handle* H, int n_frames, long long total, sirius_ray_result* d_
     // covers only that family's frames. Per launch i: frame entries [tab_off[i], tab_off[i+1])
     // of the table (x: first block, y: frame), grid tab_grid[i].
     std::vector<int2> tab;
-    int tab_off[4] = {0, 0, 0, 0}, tab_grid[3] = {grid, grid, grid};
+    int tab_off[5] = {0, 0, 0, 0, 0}, tab_grid[4] = {grid, grid, grid, grid};
     const bool use_table = n_frames > 1 && !P.persistent && !d_list && !d_rays && !pair && !scratch &&
                            int(H->frames_host.size()) == n_frames;
     if (use_table) {
@@ -1051,7 +1049,7 @@ int launch_trace(Handle* H, int n_frames, long long total, sirius_ray_result* d_
             int b0 = 0;
             for (int f = 0; f < n_frames; ++f) {
                 const FrameDev& F = H->frames_host[size_t(f)];
-                if (launch_family[i] >= 0 && F.m.family != launch_family[i]) continue;
+                if (launch_family[i] >= 0 && F.cls != launch_family[i]) continue;
                 tab.push_back(make_int2(b0, f));
                 const long long rows = F.n_rays / F.width;
                 b0 += int(((F.width + tile_x - 1) / tile_x) * ((rows + tile_y - 1) / tile_y));
@@ -1072,7 +1070,7 @@ int launch_trace(Handle* H, int n_frames, long long total, sirius_ray_result* d_
     // the mixed path reads the disk flux from per-frame tables
     P.flux = nullptr;
     int extra_launches = 0;
-    if (mixed && c.enable_disk && (H->family_mask & (1 << SIRIUS_METRIC_KERR_SCHILD)) && S.flux) {
+    if (mixed && c.enable_disk && (H->family_mask & ((1 << SIRIUS_METRIC_KERR_SCHILD) | (1 << kClassRing))) && S.flux) {
         if (!flux_ready) {  // else the caller built this upload's tables ahead of this stream
             flux_table_kernel<<<n_frames, kFluxN, 0, st>>>(S.frames, S.flux);
             CK(cudaGetLastError());
@@ -1731,7 +1729,7 @@ static int upload_frames(Handle* H, const sirius_frame* frames, int n, long long
         total += fd[i].n_rays;
     }
     H->family_mask = 0;
-    for (int i = 0; i < n; ++i) H->family_mask |= 1 << frames[i].metric.family;
+    for (int i = 0; i < n; ++i) H->family_mask |= 1 << fd[i].cls;
     H->frame0 = fd[0];
     H->frames_host = fd;
     int rc = ensure(H, H->d_frames, H->frames_cap, size_t(n));
@@ -1881,7 +1879,9 @@ int sirius_cuda_trace_beams(sirius_cuda_handle h, const sirius_frame* frames, in
     B.status = H->d_status;
     cudaError_t e = cudaMemsetAsync(H->d_status, 0, sizeof(int), H->stream);
     if (e == cudaSuccess) {
-        beam_kernel<<<int((total + 31) / 32), 64, 0, H->stream>>>(B);  // two lanes per beam
+        const int grid = int((total + 31) / 32);  // two lanes per beam
+        if (H->family_mask & (1 << SIRIUS_METRIC_KERR_SCHILD)) beam_kernel<false><<<grid, 64, 0, H->stream>>>(B);
+        if (H->family_mask & (1 << kClassRing)) beam_kernel<true><<<grid, 64, 0, H->stream>>>(B);
         e = cudaGetLastError();
     }
     int status = 0;
@@ -1927,7 +1927,7 @@ int sirius_cuda_trace_frames_static(sirius_cuda_handle h, const sirius_frame* d_
         fd[i] = make_frame(f, H->cfg);
         fd[i].flux_slot = i;
         total += fd[i].n_rays;
-        mask |= 1 << f.metric.family;
+        mask |= 1 << fd[i].cls;
     }
     if (total != total_rays) return fail(H, SIRIUS_ERR_INVALID_ARGUMENT, "total_rays does not match the frames");
     // a pageable source: the copy has been staged when cudaMemcpyAsync returns

@@ -60,6 +60,10 @@ template <class T>
 SIRIUS_HD __forceinline__ T tmax(T a, T b) { return a > b ? a : b; }
 template <class T>
 SIRIUS_HD __forceinline__ D1<T> tmax(D1<T> a, T b) { return a.v > b ? a : D1<T>(b); }
+template <class T>
+SIRIUS_HD __forceinline__ T value_of(T a) { return a; }
+template <class T>
+SIRIUS_HD __forceinline__ T value_of(D1<T> a) { return a.v; }
 
 // ---------------------------------------------------------------------------
 // Kerr-Schild family (PHMT100A.h:198-396): H and l_i as dual numbers.
@@ -188,12 +192,19 @@ SIRIUS_HD __forceinline__ void ks_rhs_terms(const MetricDev& m, const T x[4], co
 // In three parts: what depends on the position alone (KSGeom), the velocity and the
 // force at a momentum, so that the symplectic integrator, which takes two kicks and
 // a drift at each position, evaluates the geometry once.
+//
+// All of it rests on r solving its equation. Where r is held at 1e-5 (inside the ring, next
+// to its disc) r^2 sd is not r^4 + a^2 z^2 and l is not null: there 1 / sd gives way to
+// r^2 / (r^4 + a^2 z^2) wherever it stands for that, and l.k is formed from k, which makes this
+// the terms' right-hand side again. RING compiles that in; only rays that no horizon stops
+// need it (FrameDev::cls). It cost the others 6 % in FP64 and 3 % in symplectic steps.
 template <class T>
 struct KSGeom {
     T X, Y, Z, r, ir, isd, iden, den, l1, l2, l3, H, w, c, hz;  // c = Lambda R^2 / 3, hz = a^2 z / (r sd)
+    bool held;  // r is the least one
 };
 
-template <class T>
+template <bool RING, class T>
 SIRIUS_HD __forceinline__ void ks_geom(const MetricDev& m, T X, T Y, T Z, KSGeom<T>& G) {
     using C = typename scalar_of<T>::type;
     const C a = cst<C>(m.a, m.fa), a2 = cst<C>(m.a2, m.fa2), M2 = cst<C>(2.0 * m.M, m.fM2);
@@ -208,14 +219,17 @@ SIRIUS_HD __forceinline__ void ks_geom(const MetricDev& m, T X, T Y, T Z, KSGeom
     const T r = mul_(r2, ir);
     const T den = r2 + a2;
     const T iden = rcp_(den);
+    T ih = isd;  // r^2 / (r^4 + a^2 z^2)
+    G.held = RING && !(value_of(r2) > C(1e-10));
+    if (G.held) ih = mul_(r2, rcp_(fma_(r2, r2, a2zz)));
     const T q = fma_(M2, r, -cst<C>(m.Q2, m.fQ2));
     G.X = X; G.Y = Y; G.Z = Z; G.r = r; G.ir = ir; G.isd = isd; G.iden = iden; G.den = den;
     G.l1 = mul_(fma_(r, X, mul_(a, Y)), iden);
     G.l2 = mul_(fma_(r, Y, mul_(-a, X)), iden);
     G.l3 = mul_(Z, ir);
-    G.H = mul_(q, isd);
-    G.w = mul_(fma_(mul_(C(2), q), ir, fma_(mul_(C(-4), G.H), r, M2)), isd);
-    G.hz = mul_(mul_(a2, G.l3), isd);
+    G.H = mul_(q, ih);
+    G.w = mul_(fma_(mul_(C(2), q), ir, fma_(mul_(C(-4), G.H), r, M2)), ih);
+    G.hz = mul_(mul_(a2, G.l3), ih);
     G.c = T(0);
     if (m.has_lambda) G.c = mul_(cst<C>(m.lam3, m.flam3), R2);
 }
@@ -236,8 +250,8 @@ SIRIUS_HD __forceinline__ void ks_velocity(const MetricDev& m, const KSGeom<T>& 
         const T wp = fma_(w3, p[3], fma_(w2, p[2], fma_(w1, p[1], mul_(w0, p[0]))));
         const T s = mul_(mul_(G.c, wp), rcp_(fma_(G.c, C(1) + G.H, C(1))));
         k[0] = fma_(s, w0, k[0]); k[1] = fma_(s, w1, k[1]); k[2] = fma_(s, w2, k[2]); k[3] = fma_(s, w3, k[3]);
-        lk = fma_(G.l3, k[3], fma_(G.l2, k[2], fma_(G.l1, k[1], k[0])));
     }
+    if (m.has_lambda || G.held) lk = fma_(G.l3, k[3], fma_(G.l2, k[2], fma_(G.l1, k[1], k[0])));
 }
 
 // f_i = dp_i / dl, i = 1..3 (f_0 = 0: the metric is static), from the velocity
@@ -260,20 +274,20 @@ SIRIUS_HD __forceinline__ void ks_force(const MetricDev& m, const KSGeom<T>& G, 
     }
 }
 
-template <class T>
+template <bool RING, class T>
 SIRIUS_HD __forceinline__ void ks_rhs_closed(const MetricDev& m, const T x[4], const T p[4], T k[4], T f[4]) {
     KSGeom<T> G;
     T lk;
-    ks_geom(m, x[1], x[2], x[3], G);
+    ks_geom<RING>(m, x[1], x[2], x[3], G);
     ks_velocity(m, G, p, k, lk);
     ks_force(m, G, k, lk, f);
 }
 
 // The Kerr-Schild right-hand side of precision T: the closed form in FP64, the
 // terms otherwise (and for the operation count, which is the FP32 kernel's).
-template <class T>
+template <bool RING, class T>
 SIRIUS_HD __forceinline__ void ks_rhs_fast(const MetricDev& m, const T x[4], const T p[4], T k[4], T f[4]) {
-    if constexpr (std::is_same<T, double>::value) ks_rhs_closed(m, x, p, k, f);
+    if constexpr (std::is_same<T, double>::value) ks_rhs_closed<RING>(m, x, p, k, f);
     else ks_rhs_terms(m, x, p, k, f);
 }
 
@@ -348,13 +362,20 @@ SIRIUS_HD __forceinline__ void alc_rhs(const MetricDev& m, const T x[4], const T
 // FAM selects the metric family at compile time (a kernel specialised for one
 // family carries one right-hand side); kAnyFamily dispatches on m.family.
 constexpr int kAnyFamily = -1;
+// Kerr-Schild frames whose rays may come to where r is held (KSGeom): no horizon stops them before.
+// They have kernels of their own, and no one-frame forms (Q = 1.3, 512^2: FP64 6.0 -> 3.2 ms).
+constexpr int kClassRing = 3;
+// Whether a kernel of family FAM carries the forms of that region.
+template <int FAM>
+constexpr bool kRing = FAM == kAnyFamily || FAM == kClassRing;
 
 template <class T, int FAM = kAnyFamily>
 SIRIUS_HD __forceinline__ void rhs(const MetricDev& m, const T x[4], const T p[4], T k[4], T f[4]) {
-    if constexpr (FAM == SIRIUS_METRIC_KERR_SCHILD) ks_rhs_fast(m, x, p, k, f);
+    if constexpr (FAM == SIRIUS_METRIC_KERR_SCHILD) ks_rhs_fast<false>(m, x, p, k, f);
+    else if constexpr (FAM == kClassRing) ks_rhs_fast<true>(m, x, p, k, f);
     else if constexpr (FAM == SIRIUS_METRIC_MORRIS_THORNE) mt_rhs(m, x, p, k, f);
     else if constexpr (FAM == SIRIUS_METRIC_ALCUBIERRE) alc_rhs(m, x, p, k, f);
-    else if (m.family == SIRIUS_METRIC_KERR_SCHILD) ks_rhs_fast(m, x, p, k, f);
+    else if (m.family == SIRIUS_METRIC_KERR_SCHILD) ks_rhs_fast<true>(m, x, p, k, f);
     else if (m.family == SIRIUS_METRIC_MORRIS_THORNE) mt_rhs(m, x, p, k, f);
     else alc_rhs(m, x, p, k, f);
 }
@@ -363,6 +384,7 @@ SIRIUS_HD __forceinline__ void rhs(const MetricDev& m, const T x[4], const T p[4
 template <int FAM>
 SIRIUS_HD __forceinline__ bool is_family(const MetricDev& m, int F) {
     if constexpr (FAM == kAnyFamily) return m.family == F;
+    else if constexpr (FAM == kClassRing) return F == SIRIUS_METRIC_KERR_SCHILD;
     else return FAM == F;
 }
 
@@ -379,6 +401,7 @@ struct InvForm {
     double vf;                    // Alcubierre
 };
 
+template <bool RING = true>
 __device__ __forceinline__ void inv_form(const MetricDev& m, const double x[4], InvForm& F) {
     F.d[0] = 0.0;
     if (m.family == SIRIUS_METRIC_MORRIS_THORNE) {
@@ -417,6 +440,13 @@ __device__ __forceinline__ void inv_form(const MetricDev& m, const double x[4], 
     F.l[2] = mul_(fma_(r, Y, mul_(-m.a, X)), iden);
     F.l[3] = mul_(Z, ir);
     F.H = mul_(q, isd);
+    if (RING && !(r2 > 1e-10)) {  // r is held (KSGeom): H as in the terms, and for a = 0 the radial direction
+        F.H = mul_(mul_(q, r2), rcp_(fma_(r2, r2, a2zz)));
+        if (m.a == 0.0) {
+            const double iR = rsqrt_(fmax(R2, 1e-300));
+            F.d[1] = mul_(X, iR); F.d[2] = mul_(Y, iR); F.d[3] = mul_(Z, iR);
+        }
+    }
     F.w[0] = -1.0 - F.H; F.w[1] = mul_(F.H, F.l[1]); F.w[2] = mul_(F.H, F.l[2]); F.w[3] = mul_(F.H, F.l[3]);
     F.c = 0.0;
     F.sm = 0.0;
@@ -476,7 +506,7 @@ __device__ __forceinline__ double project_null(const MetricDev& m, const InvForm
 // ~1e-7 C; the FP64 path (T = double) keeps everything in FP64. Returns C; r_out = r;
 // moved: the update is beyond what the stored f(x, p) resolves (1e-6 of p with FP32
 // storage, 1e-10 in FP64).
-template <class T>
+template <class T, bool RING>
 __device__ __forceinline__ double project_null_ks(const MetricDev& m, const double x[4], double p[4], double& r_out,
                                                   bool& moved) {
     moved = false;
@@ -490,15 +520,27 @@ __device__ __forceinline__ double project_null_ks(const MetricDev& m, const doub
     r_out = r;
     const double den = r2 + a2, iden = rcp_(den);
     const double l1 = mul_(fma_(r, X, mul_(a, Y)), iden), l2 = mul_(fma_(r, Y, mul_(-a, X)), iden), l3 = mul_(Z, ir);
-    const double H = mul_(fma_(2.0 * m.M, r, -m.Q2), isd);
+    const bool held = RING && !(r2 > 1e-10);  // r does not solve its equation there (KSGeom)
+    const double q2 = fma_(2.0 * m.M, r, -m.Q2);
+    double H = mul_(q2, isd);
+    if (held) H = mul_(mul_(q2, r2), rcp_(fma_(r2, r2, a2zz)));
     const double lp = fma_(l3, p[3], fma_(l2, p[2], fma_(l1, p[1], -p[0])));
     const double pp = fma_(p[3], p[3], fma_(p[2], p[2], fma_(p[1], p[1], mul_(-p[0], p[0]))));
     const double C = fma_(mul_(-H, lp), lp, pp);
     const T isdt = T(isd), rs = mul_(T(r), isdt), dt = mul_(T(den), isdt);
-    const T d1 = mul_(rs, T(X)), d2 = mul_(rs, T(Y)), d3 = mul_(mul_(T(Z), dt), T(ir));
+    T d1 = mul_(rs, T(X)), d2 = mul_(rs, T(Y)), d3 = mul_(mul_(T(Z), dt), T(ir));
+    T ld = T(1), dd = dt;  // l . dr, |dr|^2
+    if (held) {
+        if (sizeof(T) == sizeof(double) && m.a == 0.0) {
+            const double iR = rsqrt_(fmax(R2, 1e-300));
+            d1 = T(mul_(X, iR)); d2 = T(mul_(Y, iR)); d3 = T(mul_(Z, iR));
+        }
+        ld = fma_(T(l3), d3, fma_(T(l2), d2, mul_(T(l1), d1)));
+        dd = fma_(d3, d3, fma_(d2, d2, mul_(d1, d1)));
+    }
     const T p1 = T(p[1]), p2 = T(p[2]), p3 = T(p[3]);
-    const T Ht = T(H);
-    const T A = dt - Ht;
+    const T Ht = mul_(T(H), ld);
+    const T A = fma_(-Ht, ld, dd);
     const T pd = fma_(p3, d3, fma_(p2, d2, mul_(p1, d1)));
     const T B = mul_(T(2), fma_(-Ht, T(lp), pd));
     const T Ct = T(C);

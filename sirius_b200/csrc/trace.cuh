@@ -27,6 +27,7 @@ struct FrameDev {
     MetricDev m;
     long long ray_offset, n_rays;
     int width, height, projection, has_horizon, gate;
+    int cls;        // which kernel traces its rays: the metric family, or kClassRing
     int flux_slot;  // index of this frame's disk flux table (its position in the launch)
     int row0;       // first camera row of the frame's row window (pixel row of its ray 0)
     // camera
@@ -544,7 +545,7 @@ __device__ __forceinline__ void symplectic_step(const MetricDev& m, int order, d
         };
 #pragma unroll
         for (int i = 1; i < 4; ++i) P[i] = T(p[i]);
-        ks_geom(m, T(x[1]), T(x[2]), T(x[3]), G);
+        ks_geom<kRing<FAM>>(m, T(x[1]), T(x[2]), T(x[3]), G);
 #pragma unroll 1
         for (int s = 0; s < n; ++s) {
             const double hs = mul_(kYoshida[row][s], h), hk = mul_(0.5, hs);
@@ -552,7 +553,7 @@ __device__ __forceinline__ void symplectic_step(const MetricDev& m, int order, d
             ks_velocity(m, G, P, k, lk);
 #pragma unroll
             for (int i = 0; i < 4; ++i) x[i] = fma_(hs, double(k[i]), x[i]);
-            ks_geom(m, T(x[1]), T(x[2]), T(x[3]), G);
+            ks_geom<kRing<FAM>>(m, T(x[1]), T(x[2]), T(x[3]), G);
             kick(hk);
         }
         return;

@@ -39,7 +39,7 @@ struct Params {
     int* status;                          // [0] watchdog flag
     int persistent;
     int refill_threshold;
-    int family;                           // >= 0: trace only the rays of frames of this family
+    int family;                           // >= 0: trace only the rays of frames of this class (FrameDev::cls)
     const int2* blocks;                   // multi-frame launch: per frame of the launch, x: its first block,
     int n_block_frames;                   // y: its index; a block traces one pixel tile of one frame
                                           // (tile_ray's layout, edge tiles cut by the frame)
@@ -720,13 +720,13 @@ __device__ __forceinline__ int advance_post(const Params& P, Ray<MIXED>& s, bool
         double before;
         bool stale;  // the projection moved p beyond what the stored f(x, p) resolves: recompute it
         if (ks_fast) {
-            before = project_null_ks<K>(m, s.x, s.p, rr, stale);
+            before = project_null_ks<K, kRing<FAM>>(m, s.x, s.p, rr, stale);
         } else {
             double pb[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) pb[i] = s.p[i];
             InvForm IF;
-            inv_form(m, s.x, IF);
+            inv_form<kRing<FAM>>(m, s.x, IF);
             rr = IF.r;
             before = project_null(m, IF, s.p);
             // 1e-10 relative in FP64, 1e-6 with FP32 storage
@@ -744,7 +744,7 @@ __device__ __forceinline__ int advance_post(const Params& P, Ray<MIXED>& s, bool
         rr = ks_radius(m, s.x);
     } else {
         InvForm IF;
-        inv_form(m, s.x, IF);
+        inv_form<kRing<FAM>>(m, s.x, IF);
         rr = IF.r;
     }
     s.r = rr;
@@ -884,18 +884,18 @@ __device__ __forceinline__ void trace_body(const Params& P) {
             const int frame = P.blocks[lo].y, lb = int(blockIdx.x) - P.blocks[lo].x;
             const FrameDev& F = P.frames[frame];
             const long long pix = tile_ray(F.width, int(F.n_rays / F.width), lb);
-            if (pix >= 0 && (P.family < 0 || F.m.family == P.family)) {
+            if (pix >= 0 && (P.family < 0 || F.cls == P.family)) {
                 begin_ray<MIXED, FAM, UNI>(P, s, F.ray_offset + pix, frame, vol);
                 alive = true;
             }
         } else {
-            const long long gid = UNI && P.tiled ? tile_ray(P.f0.width, int(P.f0.n_rays / P.f0.width), int(blockIdx.x) + P.block0)
-                                                 : (long long)blockIdx.x * blockDim.x + threadIdx.x;
+            const long long gid = P.tiled ? tile_ray(P.f0.width, int(P.f0.n_rays / P.f0.width), int(blockIdx.x) + P.block0)
+                                          : (long long)blockIdx.x * blockDim.x + threadIdx.x;
             const unsigned entry = (P.list && gid >= 0 && gid < P.total) ? P.list[gid] : 0u;
             if (gid >= 0 && gid < P.total && entry != kListSkip) {
                 const long long idx = P.list ? (long long)entry : gid;
                 const int frame = P.n_frames > 1 ? find_frame(P.frames, P.n_frames, idx) : 0;
-                if (P.family < 0 || P.frames[frame].m.family == P.family) {
+                if (P.family < 0 || P.frames[frame].cls == P.family) {
                     begin_ray<MIXED, FAM, UNI>(P, s, idx, frame, vol);
                     alive = true;
                 }
@@ -982,7 +982,8 @@ using TraceFn = void (*)(Params);
 // Kerr-Schild family, mixed precision / FP64; symp: the symplectic integrator (else DP45)
 TraceFn pick_ks_mixed(int minb, bool uni, bool symp);
 TraceFn pick_ks_fp64(int minb, bool uni, bool symp);
-TraceFn pick_family(bool mixed, int fam);   // Morris-Thorne, Alcubierre, or any family (kAnyFamily)
+// Morris-Thorne, Alcubierre, kClassRing, or any family (kAnyFamily)
+TraceFn pick_family(bool mixed, int fam, bool symp);
 // Kerr-Schild family, mixed precision, two rays per thread (minb 2: 255 registers, 3: 168)
 TraceFn pick_ks_mixed_pair(int minb, bool uni);
 

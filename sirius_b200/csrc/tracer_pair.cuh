@@ -263,7 +263,7 @@ __device__ __forceinline__ void trace_pair_body(const Params& P) {
         if (li < P.total && entry != kListSkip) {
             const long long idx = P.list ? (long long)entry : li;
             const int frame = P.n_frames > 1 ? find_frame(P.frames, P.n_frames, idx) : 0;
-            if (P.family < 0 || P.frames[frame].m.family == P.family) {
+            if (P.family < 0 || P.frames[frame].cls == P.family) {
                 begin_ray<true, KS, UNI>(P, s[q], idx, frame, volq[q]);
                 alive[q] = true;
             }

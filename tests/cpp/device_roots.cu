@@ -1,5 +1,6 @@
-// The device's scalar reciprocals and roots (csrc/dual.cuh, csrc/roots.cuh) on arrays, and the warp drive's projection
-// form at a radius, for tests/test_gpu_roots.py.
+// The device's scalar reciprocals and roots (csrc/dual.cuh, csrc/roots.cuh) on arrays, the warp drive's projection form
+// at a radius, and the two forms of the Kerr-Schild projection, for tests/test_gpu_roots.py and
+// tests/test_gpu_naked_ring.py.
 #include <cuda_runtime.h>
 
 #include "roots.cuh"
@@ -25,7 +26,7 @@ __global__ void warp_centre(sirius::MetricDev m, double x, double* y) {
     const double pos[4] = {0.0, x, 0.0, 0.0};
     double p[4] = {-1.0, 0.7, 0.3, -0.2};
     InvForm F;
-    inv_form(m, pos, F);
+    inv_form<true>(m, pos, F);
     y[0] = F.r;
     for (int i = 0; i < 4; ++i) y[1 + i] = i == 0 ? 0.0 : F.d[i];
     y[5] = project_null(m, F, p);
@@ -42,6 +43,42 @@ extern "C" int device_warp_centre(double x, double* y) {
     warp_centre<<<1, 1>>>(sirius::metric_dev(s), x, d);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpy(y, d, 10 * sizeof(double), cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return int(e);
+}
+
+// state (x, p) -> 8 numbers: the momentum after the short projection, the null value before it, r; and the general one's
+__global__ void ks_projections(sirius::MetricDev m, long long n, const double* state, double* fast, double* general) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    using namespace sirius;
+    const double *x = state + 8 * i, *p = x + 4;
+    double a[4], b[4], r;
+    bool moved;
+    for (int j = 0; j < 4; ++j) a[j] = b[j] = p[j];
+    fast[8 * i + 4] = project_null_ks<double, true>(m, x, a, r, moved);
+    InvForm F;
+    inv_form<true>(m, x, F);
+    general[8 * i + 4] = project_null(m, F, b);
+    for (int j = 0; j < 4; ++j) {
+        fast[8 * i + j] = a[j];
+        general[8 * i + j] = b[j];
+    }
+    fast[8 * i + 5] = r;
+    general[8 * i + 5] = F.r;
+    for (int j = 6; j < 8; ++j) fast[8 * i + j] = general[8 * i + j] = 0.0;
+}
+
+extern "C" int device_ks_projections(const sirius_metric* s, long long n, const double* state, double* out) {
+    double* d = nullptr;
+    cudaError_t e = cudaMalloc((void**)&d, 3 * 8 * n * sizeof(double));
+    if (e != cudaSuccess) return int(e);
+    e = cudaMemcpy(d, state, 8 * n * sizeof(double), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        ks_projections<<<unsigned((n + 127) / 128), 128>>>(sirius::metric_dev(*s), n, d, d + 8 * n, d + 16 * n);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(out, d + 8 * n, 16 * n * sizeof(double), cudaMemcpyDeviceToHost);
     cudaFree(d);
     return int(e);
 }
