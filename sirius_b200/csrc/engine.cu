@@ -959,8 +959,8 @@ int launch_trace(Handle* H, int n_frames, long long total, sirius_ray_result* d_
     // blocks per SM (persistent), or for max_registers (one thread per ray);
     // fewer registers, possibly spills. The default was measured on the 1024^2
     // bench frame in the tiled layout: mixed DP45 runs fastest at 128 registers
-    // (16 warps per SM; 16.7 ms against 18.5 at 168 and 19.0 at 255), FP64 DP45 at
-    // 168 (19.7 ms against 20.2 at 128 and 21.2 at 255); the symplectic
+    // (16 warps per SM; 16.7 ms against 18.1 at 168 and 18.4 at 255), FP64 DP45 at
+    // 168 (19.8 ms against 20.2 at 128 and 21.0 at 255); the symplectic
     // integrator keeps 255. The choice depends on the configuration
     // only, never on the launch's size or contents: the budgets' FP32 roundings
     // differ, and a ray's result must not depend on what else shares its launch.

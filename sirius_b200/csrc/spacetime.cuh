@@ -363,7 +363,8 @@ SIRIUS_HD __forceinline__ void alc_rhs(const MetricDev& m, const T x[4], const T
 // family carries one right-hand side); kAnyFamily dispatches on m.family.
 constexpr int kAnyFamily = -1;
 // Kerr-Schild frames whose rays may come to where r is held (KSGeom): no horizon stops them before.
-// They have kernels of their own, and no one-frame forms (Q = 1.3, 512^2: FP64 6.0 -> 3.2 ms).
+// They have kernels of their own, without one-frame forms (charged, Q = 1.3, 512^2: FP64 2.9 ms, 2.5
+// without the test for held r and 6.0 with the general forms throughout).
 constexpr int kClassRing = 3;
 // Whether a kernel of family FAM carries the forms of that region.
 template <int FAM>
