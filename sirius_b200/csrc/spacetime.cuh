@@ -187,8 +187,9 @@ SIRIUS_HD __forceinline__ void ks_rhs_terms(const MetricDev& m, const T x[4], co
 // and an FP64 root or reciprocal is a sequence of about ten: this form takes two
 // reciprocal square roots and one reciprocal where the terms take two square
 // roots and four reciprocals, and 94 operations instead of 143 (717 x 405 FP64
-// frame 8.73 -> 7.45 ms from this alone). The FP32 arithmetic keeps the terms: the two forms round
-// differently, and near the critical curve FP32 roundings reach the image.
+// frame 8.73 -> 7.45 ms from this alone). The FP32 stages of the mixed DP45 path keep the terms:
+// the two forms round differently, near the critical curve FP32 roundings reach the image, and which
+// of the two images is nearer to FP64 has not been measured.
 // In three parts: what depends on the position alone (KSGeom), the velocity and the
 // force at a momentum, so that the symplectic integrator, which takes two kicks and
 // a drift at each position, evaluates the geometry once.
